@@ -220,7 +220,7 @@ size_t slot_bytes(int nt, size_t rf, int K, int segcap, int stepcap) {
     size_t b = 0;
     b += 2 * D2 + 2 * D2;               // u[2], lam[2]
     b += 7 * C + 7 * D2;                // kf (RF), ka (FP64)
-    b += 2 * D2 + D2 + 8 * (size_t)nt;  // scr[2], esv, skv
+    b += 2 * D2 + D2;                   // scr[2], esv
     b += (size_t)K * (D2 + C);          // checkpoints
     b += 16 * (size_t)stepcap;          // step log
     b += (size_t)segcap * 5 * C;        // recompute segment
@@ -310,7 +310,6 @@ int work_create(fl_problem* pr, int B, int nsave, int mode, Work** out,
         d.scr[0] = carve(p, D2);
         d.scr[1] = carve(p, D2);
         d.esv = (double*)carve(p, D2);
-        d.skv = (double*)carve(p, 8 * (size_t)nt);
         d.ck_u = (double*)carve(p, D2 * w->K);
         d.ck_k1 = carve(p, C * w->K);
         d.steplog = (double*)carve(p, 16 * (size_t)w->stepcap);
@@ -331,6 +330,36 @@ int work_create(fl_problem* pr, int B, int nsave, int mode, Work** out,
     return FL_OK;
 }
 
+// CTAs per slot for a launch of this many slots: the size whose waves take
+// the least time.  A C-CTA solve takes a fraction of a one-CTA solve (column
+// rel), and the clusters in flight are bounded by the SMs of a GPC: 74 of two
+// CTAs, 32 of four, 14 of eight on 148 SMs.  Measured per gradient batch
+// (ms, 0.3 m; 1 / 2 / 4 / 8 CTAs): Nt = 2^13, 8 slots 8.9 / 5.9 / 4.7 / 4.5,
+// 24 slots 9.0 / 6.0 / 4.8 / 8.7, 60 slots 9.6 / 6.5 / 9.5 / 17.7, 148 slots
+// 11.6 / 13.7 / 23 / 44; 2^12, 8 slots 4.9 / 4.2 / 4.0, 36 slots 5.4 / 4.6 /
+// 7.9; 2^14, 8 slots 23.8 / - / 9.1 / 8.1, 40 slots 26.6 / - / 18.5 / 24.1.
+int sm_cluster(const fl_ctx* ctx, int logn, int slots) {
+    static const struct {
+        int c, per148;
+        double rel[3];  // 2^12, 2^13, 2^14
+    } size[] = {{1, 148, {1.0, 1.0, 1.0}},
+                {2, 74, {0.86, 0.66, 1.0}},
+                {4, 32, {0.82, 0.54, 0.38}},
+                {8, 14, {1.0, 0.50, 0.34}}};
+    int best = 1;
+    double least = 1e300;
+    for (const auto& z : size) {
+        if (z.c > 1 && !sm_cluster_built(logn, z.c)) continue;
+        const int cap = std::max(1, z.per148 * ctx->sm_count / 148);
+        const double t = ((slots + cap - 1) / cap) * (z.c == 1 ? 1.0 : z.rel[logn - 12]);
+        if (t < least) {
+            least = t;
+            best = z.c;
+        }
+    }
+    return best;
+}
+
 int launch_slots(fl_ctx* ctx, fl_problem* pr, Work* w, int nactive, int max_evals) {
     const int logn = ilog2i(pr->nt);
     const int fp64 = pr->precision == FL_PRECISION_FP64;
@@ -339,6 +368,7 @@ int launch_slots(fl_ctx* ctx, fl_problem* pr, Work* w, int nactive, int max_eval
         return set_err(ctx, FL_EUNSUPPORTED, "Nt = 2^%d is not built for %s", logn,
                        fp64 ? "FP64" : "FP32");
     LaunchArgs a{w->d_desc, w->d_state, w->d_active, nactive, max_evals, ctx->stream};
+    a.cluster = sm_cluster(ctx, logn, nactive);
     CU(fn(a));
     ctx->launches++;
     return FL_OK;
@@ -1457,9 +1487,21 @@ int srv_launch(fl_server* sv, SrvBucket* b, SrvChunk* c) {
         CU(cudaGraphLaunch(c->graph, c->stream));
         sv->launches += 1 + (long)sv->opts.evals_per_launch * (a.fp64 ? 7 : 10);
     } else {
+        // only the occupied slots, each over as many CTAs as the slots in
+        // flight on the single-mode stepper leave it
         LaunchFn fn = sm_launcher(b->precision == FL_PRECISION_FP64, logn);
-        LaunchArgs a{c->w->d_desc, c->w->d_state, c->w->d_active, c->B,
+        std::vector<int> act;
+        for (int i = 0; i < c->B; i++)
+            if (c->slot[i]) act.push_back(i);
+        int all = 0;
+        for (const auto* ob : sv->buckets)
+            for (const auto* oc : ob->chunks)
+                for (const auto* r : oc->slot) all += r && !oc->mm;
+        CU(cudaMemcpyAsync(c->w->d_active, act.data(), sizeof(int) * act.size(),
+                           cudaMemcpyHostToDevice, c->stream));
+        LaunchArgs a{c->w->d_desc, c->w->d_state, c->w->d_active, (int)act.size(),
                      sv->opts.evals_per_launch, c->stream};
+        a.cluster = sm_cluster(ctx, logn, all);
         CU(fn(a));
         sv->launches++;
     }
@@ -1859,13 +1901,13 @@ int fl_forward_gain(fl_problem* pr, const fl_gain* gain, double pump_power, cons
     }
     if (!(nrm > 0)) return set_err(ctx, FL_EINVAL, "input spectrum must be nonzero");
     if (cudaSetDevice(ctx->device) != cudaSuccess) return set_err(ctx, FL_ENODEV, "cudaSetDevice");
-    // one device area: launch, two states, seven FP32 stages, two scratch
-    // fields, error partial and weights, output, gain tables, descriptor, result
+    // one device area: launch, two states, seven FP32 stages, the stage
+    // field and its gain term, two scratch fields, error partial and weights, output, gain tables, descriptor, result
     // (the size is the sum of the regions taken below, each rounded up to the
     // 256-byte alignment that take() gives it)
     const size_t F = 16 * (size_t)nt, H = 8 * (size_t)nt;
     auto al = [](size_t n) { return (n + 255) & ~size_t(255); };
-    const size_t bytes = 4 * al(F) + 7 * al(H) + 2 * al(F) + al(F) + al(H) + al(4 * H) +
+    const size_t bytes = 4 * al(F) + 9 * al(H) + 2 * al(F) + al(F) + al(H) + al(4 * H) +
                          al(8 * (size_t)nsave) + al(F * (size_t)nsave) + al(8 * (size_t)nsave) +
                          al(sizeof(GainDesc)) + al(sizeof(GainOut));
     char* pool = nullptr;
@@ -1892,6 +1934,8 @@ int fl_forward_gain(fl_problem* pr, const fl_gain* gain, double pump_power, cons
     d.u[1] = (double*)take(F);
     d.uL_out = (double*)take(F);
     for (int i = 0; i < 7; i++) d.kf[i] = take(H);
+    d.ka[0] = take(H);  // the stage field and its derivative
+    d.ka[1] = take(H);  // the stage's gain term
     d.scr[0] = take(F);
     d.scr[1] = take(F);
     d.esv = (double*)take(F);

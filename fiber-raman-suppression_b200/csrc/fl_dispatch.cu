@@ -38,10 +38,4 @@ RhsFn rhs_launcher(int fp64, int logn) {
     return fp64 ? f64[logn] : f32[logn];
 }
 
-int sm_threads(int fp64, int logn) {
-    if (!sm_launcher(fp64, logn)) return 0;
-    const int loge = logn <= 8 ? logn - 5 : (logn == 14 ? 5 : 4);
-    return 1 << (logn - loge);
-}
-
 }  // namespace fl

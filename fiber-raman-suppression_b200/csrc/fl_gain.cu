@@ -21,22 +21,27 @@
 
 namespace fl {
 
-template <int LOGN, int LOGE>
-__global__ void __launch_bounds__(FftShape<LOGN, LOGE>::T, 1)
+template <int LOGN>
+__global__ void __launch_bounds__(XShape<LOGN, 1>::T, 1)
     gain_forward_kernel(const GainDesc* __restrict__ gdp, GainOut* __restrict__ out) {
-    using Sol = SmSolver<float, LOGN, LOGE>;
+    using Sol = SmSolver<float, float, LOGN, 1>;
     using CF = cx<float>;
-    using IO = FieldIO<CF, LOGN, LOGE>;
-    static_assert(IO::SMEM, "the stage field is handed over in shared memory");
-    constexpr int N = Sol::N, E = Sol::E, T = Sol::T;
+    constexpr int N = Sol::N, E = Sol::E, T = Sol::XF::T;
     extern __shared__ __align__(16) unsigned char smraw[];
-    double* red = reinterpret_cast<double*>(smraw + SmemPlan<double, LOGN>::BYTES);
+    double* red = reinterpret_cast<double*>(smraw + SmShared<float, LOGN, 1>::RED);
     const GainDesc& g = *gdp;
     const SlotDesc& d = g.s;
-    load_twiddles<LOGN>(d, red);
-    Sol S(d, smraw, red);
-    const IO io{reinterpret_cast<CF*>(smraw)};
-    CF* gb = static_cast<CF*>(d.scr[1]);  // g_b ũ_b / 2 of the current stage
+    load_tables<float, LOGN, 1>(d, smraw, 0);
+    Sol S(d, smraw, 0);
+    int flip = 0;
+    auto sum = [&](double v) { return x_reduce<T, 1, false>(v, red, flip, 0); };
+    // the stage field, then its derivative (the thread's own bins)
+    struct {
+        CF* p;
+        const Sol& S;
+        __device__ CF& operator[](int s) const { return p[S.own(s)]; }
+    } const io{static_cast<CF*>(d.ka[0]), S};
+    CF* gb = static_cast<CF*>(d.ka[1]);  // g_b ũ_b / 2 of the current stage
     CF* k[7];
 #pragma unroll
     for (int i = 0; i < 7; i++) k[i] = static_cast<CF*>(d.kf[i]);
@@ -48,43 +53,46 @@ __global__ void __launch_bounds__(FftShape<LOGN, LOGE>::T, 1)
     auto gain_of_stage = [&](double pp) -> double {
         if (g.kind == 0) {
 #pragma unroll
-            for (int s = 0; s < E; s++) gb[Sol::bin(s)] = scale(io[s], (float)(0.5 * g.g_const));
+            for (int s = 0; s < E; s++) gb[S.own(s)] = scale(io[s], (float)(0.5 * g.g_const));
             return -1.0;
         }
         double w12 = 0.0, w21 = 0.0;
 #pragma unroll
         for (int s = 0; s < E; s++) {
-            const int b = Sol::bin(s);
+            const int b = S.bin(s);
             const double e = abs2(up(io[s]));
             w12 += g.wa[b] * e;
             w21 += g.we[b] * e;
         }
-        w12 = block_sum<T>(w12, red);
-        w21 = block_sum<T>(w21, red);
+        w12 = sum(w12);
+        w21 = sum(w21);
         const double r12 = g.r12c * pp, r21 = g.r21c * pp;
         const double n2 = (r12 + w12) / (r12 + r21 + w12 + w21 + g.inv_tau), n1 = 1.0 - n2;
 #pragma unroll
         for (int s = 0; s < E; s++) {
-            const int b = Sol::bin(s);
-            gb[b] = scale(io[s], (float)(0.5 * (g.sE[b] * n2 - g.sA[b] * n1)));
+            const int b = S.bin(s);
+            gb[S.own(s)] = scale(io[s], (float)(0.5 * (g.sE[b] * n2 - g.sA[b] * n1)));
         }
         return g.gpe * n2 - g.gpa * n1;
     };
     // derivative of the stage (field in io, pump pp) at z: io <- dũ, returns dP
     auto deriv = [&](double z, double pp) -> double {
         const double gP = gain_of_stage(pp);
-        rhs_fwd_call<float, LOGN, LOGE>(&d, smraw, red, z, io);
+        StageRun in{};
+        in.k1 = io.p;
+        in.out = io.p;
+        in.z = z;
+        rhs_fwd_call<float, float, LOGN, 1>(&d, smraw, 0, &in);
 #pragma unroll
-        for (int s = 0; s < E; s++) io[s] = io[s] + gb[Sol::bin(s)];
+        for (int s = 0; s < E; s++) io[s] = io[s] + gb[S.own(s)];
         return gP * pp;
     };
 
     // ---- launch and f0
 #pragma unroll
     for (int s = 0; s < E; s++) {
-        const int b = Sol::bin(s);
-        const cx<double> x = ld2(d.u0, b);
-        st2(u, b, x);
+        const cx<double> x = ld2(d.u0, S.bin(s));
+        st2(u, S.own(s), x);
         io[s] = down<float>(x);
     }
     double pp = g.pump0;
@@ -93,7 +101,7 @@ __global__ void __launch_bounds__(FftShape<LOGN, LOGE>::T, 1)
     while (save_idx < d.nsave && d.zsave[save_idx] == 0.0) {
         double* o = d.save_out + (size_t)save_idx * 2 * N;
 #pragma unroll
-        for (int s = 0; s < E; s++) st2(o, Sol::bin(s), ld2(d.u0, Sol::bin(s)));
+        for (int s = 0; s < E; s++) st2(o, S.bin(s), ld2(d.u0, S.bin(s)));
         if (threadIdx.x == 0) g.pump_save[save_idx] = pp;
         save_idx++;
     }
@@ -103,7 +111,7 @@ __global__ void __launch_bounds__(FftShape<LOGN, LOGE>::T, 1)
     kp[0] = deriv(0.0, pp);
     nf++;
 #pragma unroll
-    for (int s = 0; s < E; s++) k[0][Sol::bin(s)] = io[s];
+    for (int s = 0; s < E; s++) k[0][S.own(s)] = io[s];
 
     // ---- initial step (OrdinaryDiffEqCore ode_determine_initdt), P one more
     // component of the norms; weights from the launch
@@ -111,15 +119,14 @@ __global__ void __launch_bounds__(FftShape<LOGN, LOGE>::T, 1)
     double s0 = 0.0, s1 = 0.0;
 #pragma unroll
     for (int s = 0; s < E; s++) {
-        const int b = Sol::bin(s);
-        const cx<double> x = ld2(u, b);
+        const cx<double> x = ld2(u, S.own(s));
         const double ax = sqrt(x.re * x.re + x.im * x.im), sk = at + ax * rt;
         const double af = sqrt(abs2(up(io[s])));
         s0 += (ax / sk) * (ax / sk);
         s1 += (af / sk) * (af / sk);
     }
-    s0 = block_sum<T>(s0, red) + (pp / skp) * (pp / skp);
-    s1 = block_sum<T>(s1, red) + (kp[0] / skp) * (kp[0] / skp);
+    s0 = sum(s0) + (pp / skp) * (pp / skp);
+    s1 = sum(s1) + (kp[0] / skp) * (kp[0] / skp);
     const double d0 = sqrt(s0 / (N + 1)), d1 = sqrt(s1 / (N + 1));
     double dt;
     if (isnan(d1)) {
@@ -131,7 +138,7 @@ __global__ void __launch_bounds__(FftShape<LOGN, LOGE>::T, 1)
         } else {
 #pragma unroll
             for (int s = 0; s < E; s++) {
-                const int b = Sol::bin(s);
+                const int b = S.own(s);
                 const cx<double> x = ld2(u, b);
                 const CF f0 = k[0][b];
                 io[s] = mk((float)(x.re + dt0 * (double)f0.re), (float)(x.im + dt0 * (double)f0.im));
@@ -141,7 +148,7 @@ __global__ void __launch_bounds__(FftShape<LOGN, LOGE>::T, 1)
             double s2 = 0.0, nd = 0.0;
 #pragma unroll
             for (int s = 0; s < E; s++) {
-                const int b = Sol::bin(s);
+                const int b = S.own(s);
                 const cx<double> x = ld2(u, b);
                 const double sk = at + sqrt(x.re * x.re + x.im * x.im) * rt;
                 const CF f0 = k[0][b];
@@ -151,8 +158,8 @@ __global__ void __launch_bounds__(FftShape<LOGN, LOGE>::T, 1)
                 nd += (dr != 0.0 || di != 0.0) ? 1.0 : 0.0;
             }
             const double dp = kp1 - kp[0];
-            s2 = block_sum<T>(s2, red) + (dp / skp) * (dp / skp);
-            nd = block_sum<T>(nd, red) + (dp != 0.0 ? 1.0 : 0.0);
+            s2 = sum(s2) + (dp / skp) * (dp / skp);
+            nd = sum(nd) + (dp != 0.0 ? 1.0 : 0.0);
             const double d2 = sqrt(s2 / (N + 1)) / dt0;
             dt = initdt_final(dt0, d1, d2, nd, dtmin, L);
         }
@@ -180,29 +187,48 @@ __global__ void __launch_bounds__(FftShape<LOGN, LOGE>::T, 1)
             double acc = 0.0;
             for (int j = 0; j < st; j++) acc += kT5a[st][j] * kp[j];
             const double pps = pp + dt * acc;
-            if (st < 6) {
-                S.stage_input(st, u, d.kf, 0, dt, io);
-            } else {
-                S.stage7_input(u, un, d.kf, 0, dt, at, rt, io, true);
-                pnew = pps;
+            // stage input (FP64 accumulation) and, for stage 7, the new state,
+            // the partial error and the weights
+#pragma unroll 4
+            for (int s = 0; s < E; s++) {
+                const int b = S.own(s);
+                double ar = 0.0, ai = 0.0, er = 0.0, ei = 0.0;
+                for (int j = 0; j < st; j++) {
+                    const CF x = k[j][b];
+                    ar += kT5a[st][j] * (double)x.re;
+                    ai += kT5a[st][j] * (double)x.im;
+                    er += kT5bt[j] * (double)x.re;
+                    ei += kT5bt[j] * (double)x.im;
+                }
+                const cx<double> x0 = ld2(u, b);
+                const cx<double> u1 = mk(x0.re + dt * ar, x0.im + dt * ai);
+                io[s] = down<float>(u1);
+                if (st == 6) {
+                    st2(un, b, u1);
+                    st2(d.esv, b, mk(dt * er, dt * ei));
+                    const double m0 = x0.re * x0.re + x0.im * x0.im;
+                    const double m1 = u1.re * u1.re + u1.im * u1.im;
+                    d.skv[b] = at + sqrt_nb(fmax(m0, m1)) * rt;
+                }
             }
+            if (st == 6) pnew = pps;
             kp[st] = deriv(z + kT5c[st] * dt, pps);
             nf++;
 #pragma unroll
-            for (int s = 0; s < E; s++) k[st][Sol::bin(s)] = io[s];
+            for (int s = 0; s < E; s++) k[st][S.own(s)] = io[s];
         }
         // error dt Σ b̃_j k_j over the Nt + 1 components
         double acc = 0.0;
 #pragma unroll
         for (int s = 0; s < E; s++) {
-            const int b = Sol::bin(s);
+            const int b = S.own(s);
             const cx<double> e6 = ld2(d.esv, b);
             const double er = e6.re + dt * kT5bt[6] * (double)io[s].re;
             const double ei = e6.im + dt * kT5bt[6] * (double)io[s].im;
             const double w = d.skv[b];
             acc += (er * er + ei * ei) / (w * w);
         }
-        acc = block_sum<T>(acc, red);
+        acc = sum(acc);
         double ep = 0.0;
         for (int j = 0; j < 7; j++) ep += kT5bt[j] * kp[j];
         ep *= dt;
@@ -240,7 +266,7 @@ __global__ void __launch_bounds__(FftShape<LOGN, LOGE>::T, 1)
             double* o = d.save_out + (size_t)save_idx * 2 * N;
 #pragma unroll
             for (int s = 0; s < E; s++) {
-                const int b = Sol::bin(s);
+                const int b = S.own(s), f = S.bin(s);
                 double xr = 0.0, xi = 0.0;
                 for (int i = 0; i < 7; i++) {
                     const CF ki = k[i][b];
@@ -249,8 +275,8 @@ __global__ void __launch_bounds__(FftShape<LOGN, LOGE>::T, 1)
                 }
                 const cx<double> un0 = ld2(u, b);
                 const cx<double> x = mk(un0.re + dt * xr, un0.im + dt * xi);
-                const cx<double> p = phasor<double>(d.Dturns[b], zs);
-                st2(o, b, mk(x.re * p.re - x.im * p.im, x.re * p.im + x.im * p.re));
+                const cx<double> p = phasor<double>(d.Dturns[f], zs);
+                st2(o, f, mk(x.re * p.re - x.im * p.im, x.re * p.im + x.im * p.re));
             }
             if (threadIdx.x == 0) {
                 double pk = 0.0;
@@ -262,7 +288,7 @@ __global__ void __launch_bounds__(FftShape<LOGN, LOGE>::T, 1)
         z = znew;
 #pragma unroll
         for (int s = 0; s < E; s++) {
-            const int b = Sol::bin(s);
+            const int b = S.own(s);
             st2(u, b, ld2(un, b));
             k[0][b] = io[s];
         }
@@ -276,8 +302,8 @@ __global__ void __launch_bounds__(FftShape<LOGN, LOGE>::T, 1)
     // power and counters
 #pragma unroll
     for (int s = 0; s < E; s++) {
-        const int b = Sol::bin(s);
-        const cx<double> x = ld2(u, b);
+        const int b = S.bin(s);
+        const cx<double> x = ld2(u, S.own(s));
         const cx<double> p = phasor<double>(d.Dturns[b], z);
         const cx<double> y = mk(x.re * p.re - x.im * p.im, x.re * p.im + x.im * p.re);
         st2(d.uL_out, b, y);
@@ -296,29 +322,29 @@ __global__ void __launch_bounds__(FftShape<LOGN, LOGE>::T, 1)
     }
 }
 
-template <int LOGN, int LOGE>
+template <int LOGN>
 cudaError_t launch_gain_t(const GainDesc* desc, GainOut* out, cudaStream_t stream) {
-    auto kern = gain_forward_kernel<LOGN, LOGE>;
-    const size_t smem = smem_bytes<double, LOGN>();
+    auto kern = gain_forward_kernel<LOGN>;
+    const size_t smem = SmShared<float, LOGN, 1>::BYTES;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem);
     if (e != cudaSuccess) return e;
-    kern<<<1, FftShape<LOGN, LOGE>::T, smem, stream>>>(desc, out);
+    kern<<<1, XShape<LOGN, 1>::T, smem, stream>>>(desc, out);
     return cudaGetLastError();
 }
 
 bool gain_built(int logn) { return logn >= 6 && logn <= 13; }
 
 cudaError_t launch_gain(int logn, const GainDesc* desc, GainOut* out, cudaStream_t stream) {
-    switch (logn) {  // the single-mode stepper's shapes: E = 2^(logn-5) up to 2^8, then 16
-        case 6: return launch_gain_t<6, 1>(desc, out, stream);
-        case 7: return launch_gain_t<7, 2>(desc, out, stream);
-        case 8: return launch_gain_t<8, 3>(desc, out, stream);
-        case 9: return launch_gain_t<9, 4>(desc, out, stream);
-        case 10: return launch_gain_t<10, 4>(desc, out, stream);
-        case 11: return launch_gain_t<11, 4>(desc, out, stream);
-        case 12: return launch_gain_t<12, 4>(desc, out, stream);
-        case 13: return launch_gain_t<13, 4>(desc, out, stream);
+    switch (logn) {
+        case 6: return launch_gain_t<6>(desc, out, stream);
+        case 7: return launch_gain_t<7>(desc, out, stream);
+        case 8: return launch_gain_t<8>(desc, out, stream);
+        case 9: return launch_gain_t<9>(desc, out, stream);
+        case 10: return launch_gain_t<10>(desc, out, stream);
+        case 11: return launch_gain_t<11>(desc, out, stream);
+        case 12: return launch_gain_t<12>(desc, out, stream);
+        case 13: return launch_gain_t<13>(desc, out, stream);
         default: return cudaErrorInvalidValue;
     }
 }

@@ -14,7 +14,15 @@ struct LaunchArgs {
     int nactive;
     int max_evals;         // RHS evaluations per slot in this launch
     cudaStream_t stream;
+    int cluster = 1;       // CTAs per slot (a size of sm_cluster_built, else 1)
 };
+
+// cluster sizes built for a grid
+constexpr bool sm_cluster_built(int logn, int c) {
+    return logn == 12 ? c == 2 || c == 4
+         : logn == 13 ? c == 2 || c == 4 || c == 8
+         : logn == 14 ? c == 4 || c == 8 : false;
+}
 
 using LaunchFn = cudaError_t (*)(const LaunchArgs&);
 
@@ -32,8 +40,6 @@ RhsFn rhs_launcher(int fp64, int logn);
 
 // returns nullptr when (precision, log2 Nt) is not built
 LaunchFn sm_launcher(int fp64, int logn);
-// threads per CTA of a built launcher (0 when not built)
-int sm_threads(int fp64, int logn);
 
 // pump-gain forward solve of one single-mode problem (FP32 right-hand side,
 // FP64 state and error norm), run to completion in one launch; false / an

@@ -38,7 +38,7 @@ size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
 // Offsets of every region inside the scratch array for nt points.
 struct Layout {
-    size_t desc, state, active, dturns, heff, ss, tw, u0b, u1b, kf[7], scr0, scr1, esv, skv, end;
+    size_t desc, state, active, dturns, heff, ss, tw, u0b, u1b, kf[7], scr0, scr1, esv, end;
     explicit Layout(int nt) {
         size_t p = 0;
         auto take = [&](size_t bytes) {
@@ -59,7 +59,6 @@ struct Layout {
         scr0 = take(16 * (size_t)nt);
         scr1 = take(16 * (size_t)nt);
         esv = take(16 * (size_t)nt);
-        skv = take(8 * (size_t)nt);
         end = p;
     }
 };
@@ -175,7 +174,6 @@ extern "C" int fl_forward_noalloc(int device, int nt, const double* d_D, double 
     d.scr[0] = base + lay.scr0;
     d.scr[1] = base + lay.scr1;
     d.esv = reinterpret_cast<double*>(base + lay.esv);
-    d.skv = reinterpret_cast<double*>(base + lay.skv);
 
     noalloc_prepare<<<(nt + 255) / 256, 256, 0, s>>>(d, base, lay, nt, d_D, d_hR, d_selfsteep);
     if (cudaGetLastError() != cudaSuccess) return FL_ECUDA;  // this launch's own error

@@ -1,4 +1,5 @@
-// fl_sm.cuh -- single-mode GMMNLSE stepper: one CTA owns one problem (slot)
+// fl_sm.cuh -- single-mode GMMNLSE stepper: one CTA, or a cluster of CTAs
+// when few problems run at once, owns one problem (slot)
 // and runs its whole adaptive Tsit5 solve, the checkpoint-replay recompute
 // and the adjoint solve as a state machine whose state lives in global
 // memory, so a launch can advance a slot by a bounded number of attempted
@@ -30,8 +31,11 @@
 // anomalous-dispersion fiber and misses 1e-3 gradient accuracy (measured
 // 2e-3..7e-3 on the Nt = 2^13 band-objective problem; 4e-6 in FP64).
 #pragma once
+#include <type_traits>
+
 #include "fl_fft.cuh"
 #include "fl_types.h"
+#include "fl_xfft.cuh"
 
 namespace fl {
 
@@ -66,25 +70,84 @@ constexpr double kBeta1 = 7.0 / 50.0, kBeta2 = 2.0 / 25.0, kGamma = 0.9;
 constexpr double kQmin = 0.2, kQmax = 10.0, kQoldInit = 1e-4;
 constexpr double kEps = 2.220446049250313e-16;
 
-// exp(+i D z) from the FP64 phase in turns reduced to [-1/2, 1/2] before the
-// sincos of the working precision.
+// Square root and reciprocal without the library's branches (sixteen of
+// each per step sit on one warp's critical path, and a call in the slow path
+// keeps the compiler from interleaving them): the hardware's approximation
+// (about 2^-20) and two Newton steps each, error at most an ulp or two.
+// Subnormal arguments of the root count as zero.
+__device__ __forceinline__ double sqrt_nb(double m) {
+    double r;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(m));
+    double g = m * r, h = 0.5 * r;
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        const double e = fma(-g, h, 0.5);
+        g = fma(g, e, g);
+        h = fma(h, e, h);
+    }
+    return m < 2.3e-308 ? 0.0 : g;
+}
+__device__ __forceinline__ double rcp_nb(double w) {
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(w));
+#pragma unroll
+    for (int i = 0; i < 2; i++) r = fma(r, fma(-w, r, 1.0), r);
+    return r;
+}
+
+// exp(+i D z) from the FP64 phase in turns, reduced mod 1 by adding and
+// subtracting 1.5 2^52 (the nearest integer for |D z| < 2^51 turns).
+// The turns split into a quadrant q and a rest |r| <= 1/8; cos and sin of
+// 2 pi r by their Taylor series (to x^16 and x^15 in FP64: the first term
+// left out is 5e-17 at pi/4; to x^10 and x^9 in FP32: 2e-9), then a quarter
+// turn per q.  Straight-line, so the values of a chunk interleave: the
+// library's FP64 sincospi took 330 cycles per value on one warp.
+template <typename R>
+__device__ __forceinline__ cx<R> quarter_turns(R c, R s, int q) {
+    const bool odd = q & 1;
+    const R a = odd ? s : c, b = odd ? c : s;
+    return mk((q + 1) & 2 ? -a : a, q & 2 ? -b : b);
+}
 template <typename R>
 __device__ __forceinline__ cx<R> phasor(double dturn, double z);
+__device__ __forceinline__ double turn_split(double dturn, double z, int& q) {
+    const double big = 6755399441055744.0;
+    const double t = __dmul_rn(dturn, z), f = t - ((t + big) - big);  // [-1/2, 1/2]
+    const double k = fma(f, 4.0, big);                                // nearest quarter
+    q = __double2loint(k);
+    return fma(k - big, -0.25, f);
+}
 template <>
 __device__ __forceinline__ cx<float> phasor<float>(double dturn, double z) {
-    double ph = dturn * z;
-    ph -= rint(ph);
-    float s, c;
-    sincospif(2.0f * (float)ph, &s, &c);
-    return mk(c, s);
+    int q;
+    const float x = 6.2831853071795864769f * (float)turn_split(dturn, z, q), y = x * x;
+    const float s = fmaf(x * y, fmaf(y, fmaf(y, fmaf(y, 1.0f / 362880.0f, -1.0f / 5040.0f),
+                                             1.0f / 120.0f), -1.0f / 6.0f), x);
+    const float c = fmaf(y, fmaf(y, fmaf(y, fmaf(y, fmaf(y, -1.0f / 3628800.0f, 1.0f / 40320.0f),
+                                                 -1.0f / 720.0f), 1.0f / 24.0f), -0.5f), 1.0f);
+    return quarter_turns(c, s, q);
 }
 template <>
 __device__ __forceinline__ cx<double> phasor<double>(double dturn, double z) {
-    double ph = dturn * z;
-    ph -= rint(ph);
-    double s, c;
-    sincospi(2.0 * ph, &s, &c);
-    return mk(c, s);
+    int q;
+    const double x = 6.2831853071795864769 * turn_split(dturn, z, q), y = x * x;
+    double s = -1.0 / 1307674368000.0, c = 1.0 / 20922789888000.0;
+    s = fma(s, y, 1.0 / 6227020800.0);
+    c = fma(c, y, -1.0 / 87178291200.0);
+    s = fma(s, y, -1.0 / 39916800.0);
+    c = fma(c, y, 1.0 / 479001600.0);
+    s = fma(s, y, 1.0 / 362880.0);
+    c = fma(c, y, -1.0 / 3628800.0);
+    s = fma(s, y, -1.0 / 5040.0);
+    c = fma(c, y, 1.0 / 40320.0);
+    s = fma(s, y, 1.0 / 120.0);
+    c = fma(c, y, -1.0 / 720.0);
+    s = fma(s, y, -1.0 / 6.0);
+    c = fma(c, y, 1.0 / 24.0);
+    s = fma(x * y, s, x);
+    c = fma(c, y, -0.5);
+    c = fma(c, y, 1.0);
+    return quarter_turns(c, s, q);
 }
 
 __device__ __forceinline__ cx<double> ld2(const double* p, int b) {
@@ -136,76 +199,75 @@ __device__ __forceinline__ double block_max(double v, double* red) {
     return s;
 }
 
-// Shared-memory layout of the stepper: [transform buffer][32 reduction
-// doubles][FP32 twiddles][FP64 twiddles].  red points at the reduction area.
-template <typename R, int LOGN>
-__device__ __forceinline__ const cx<R>* smem_twiddles(double* red) {
-    unsigned char* p = reinterpret_cast<unsigned char*>(red) + 32 * sizeof(double);
-    if constexpr (sizeof(R) == 8)
-        p += sizeof(cx<float>) * Twiddles<float, LOGN>::SIZE;
-    return reinterpret_cast<const cx<R>*>(p);
-}
-
-// Copy both precisions' twiddle tables into shared memory (the FP64 table is
-// absent when no adjoint will run) and wait for the block.
-template <int LOGN>
-__device__ __forceinline__ void load_twiddles(const SlotDesc& d, double* red) {
-    Twiddles<float, LOGN>::fill(const_cast<cx<float>*>(smem_twiddles<float, LOGN>(red)),
-                                (const cx<float>*)d.tw[0]);
-    if (d.tw[1])
-        Twiddles<double, LOGN>::fill(const_cast<cx<double>*>(smem_twiddles<double, LOGN>(red)),
-                                     (const cx<double>*)d.tw[1]);
-    __syncthreads();
-}
-
-// The field handed between the state machine and the out-of-line RHS, as
-// element s = bin t + T s of thread t: in the transform buffer in shared
-// memory where that buffer holds a complex FP64 field (Nt <= 2^13), else in
-// a per-thread array in local memory.  Each thread only touches its own
-// bins, so handing over needs no barrier; the RHS synchronises once after
-// reading its input, before its first transform exchange overwrites the
-// buffer.
-template <typename C, int LOGN, int LOGE>
-struct FieldIO {
-    static constexpr bool SMEM = !SmemPlan<double, LOGN>::SPLIT;
-    static constexpr int T = FftShape<LOGN, LOGE>::T;
-    C* p;
-    __device__ __forceinline__ C& operator[](int s) const {
-        if constexpr (SMEM) return p[pad(threadIdx.x + T * s)];
-        else return p[s];
-    }
+// Shared-memory layout of the stepper: [transform buffers][64 reduction
+// doubles][FP32 tables][FP64 tables][tensor-memory slot].
+template <typename RMAX, int LOGN, int C>
+struct SmShared {
+    static constexpr size_t RED = XPlan<RMAX, RMAX, LOGN, C>::BYTES;
+    static constexpr size_t TAB32 = RED + 64 * sizeof(double);
+    static constexpr size_t TAB64 =
+        (TAB32 + sizeof(cx<float>) * XTables<float, LOGN, C>::SIZE + 15) & ~size_t(15);
+    static constexpr size_t SLOT = TAB64 + sizeof(cx<double>) * XTables<double, LOGN, C>::SIZE;
+    // a cluster's CTAs hold tensor memory until their siblings finish: at
+    // most one such CTA fits an SM, so that no two clusters wait for each
+    // other's columns
+    static constexpr size_t BYTES = C > 1 && SLOT + 16 < 116 * 1024 ? 116 * 1024 : SLOT + 16;
+    static_assert(BYTES <= 227 * 1024, "shared memory of one CTA");
 };
+template <typename R, typename RMAX, int LOGN, int C>
+__device__ __forceinline__ cx<R>* smem_tables(unsigned char* smraw) {
+    using M = SmShared<RMAX, LOGN, C>;
+    return reinterpret_cast<cx<R>*>(smraw + (sizeof(R) == 8 ? M::TAB64 : M::TAB32));
+}
+
+// Fill both precisions' tables (the FP64 table is absent when no adjoint
+// will run) and wait for the group.
+template <typename RMAX, int LOGN, int C>
+__device__ __forceinline__ void load_tables(const SlotDesc& d, unsigned char* smraw, int rank) {
+    x_fill<float, LOGN, C>(smem_tables<float, RMAX, LOGN, C>(smraw), (const cx<float>*)d.tw[0], rank);
+    if (d.tw[1])
+        x_fill<double, LOGN, C>(smem_tables<double, RMAX, LOGN, C>(smraw), (const cx<double>*)d.tw[1],
+                                rank);
+    XForm<float, RMAX, LOGN, C>::sync();
+}
 
 // ---------------------------------------------------------------------------
 // Tensor memory as the right-hand side's per-thread scratch (sm_100a).
 //
 // Each RHS evaluation parks two fields between its transforms -- u_t in the
-// forward, λ_t and u_t in the adjoint -- and every thread only ever reads
-// back the bins it wrote.  At Nt = 2^12..2^13 those fields fit the SM's
-// 256 KB of tensor memory, which this kernel's FFT leaves unused: the CTA
-// allocates it once (tcgen05.alloc) and threads move their own values with
-// tcgen05.st / tcgen05.ld (32x32b shape: a warp addresses the 32 lanes of
-// its lane quarter, warp % 4, and each thread its own lane's columns), in
-// place of two per-slot fields in global memory (five 128 KB round trips
-// per FP64 adjoint evaluation).  Layout: lane 32 (w % 4) + (t % 32), columns
-// (w / 4) * 8E + f * 4E + [0, 4E) for field f of warp w: room for two FP64
-// fields, which also holds the FP32 forward's one.
+// forward, λ_t and u_t in the adjoint -- and, where there is room, its
+// phasors, and every thread only ever reads back the bins it wrote.  The
+// transforms leave the SM's 256 KB of tensor memory unused: the CTA
+// allocates columns once (tcgen05.alloc) and threads move their own values
+// with tcgen05.st / tcgen05.ld (32x32b shape: a warp addresses the 32 lanes
+// of its lane quarter, warp % 4, and each thread its own lane's columns), in
+// place of per-slot fields in global memory (five 128 KB round trips per FP64
+// adjoint evaluation at Nt = 2^13).  Layout: lane 32 (w % 4) + (t % 32),
+// columns (w / 4) COLS_WARP + f 4E + [0, 4E) for field f of warp w.
 constexpr uint32_t kNoTmem = 0xFFFFFFFFu;
 
-template <int LOGN, int LOGE>
+template <int LOGN, int C>
 struct TmLayout {
-    using S = FftShape<LOGN, LOGE>;
-    static constexpr int E = S::E, T = S::T;
+    using S = XShape<LOGN, C>;
+    static constexpr int E = S::E, T = S::TC;
     static constexpr int WARPS = T / 32;
     static constexpr int PER_Q = (WARPS + 3) / 4;      // warps sharing a lane quarter
-    static constexpr int COLS_WARP = 8 * E;            // two FP64 fields (4 words per value)
+    // FP64 fields (4 words per value); the third holds the evaluation's
+    // phasors where the columns of the CTAs that fit an SM allow it.
+    static constexpr int FIELDS = C > 1 || LOGN <= 11 ? 3 : 2;
+    static constexpr int COLS_WARP = FIELDS * 4 * E;
     static constexpr int NEED = COLS_WARP * PER_Q;
     // allocation: a power of two >= 32 columns
     static constexpr int COLS = NEED <= 32 ? 32 : NEED <= 64 ? 64 : NEED <= 128 ? 128
                               : NEED <= 256 ? 256 : 512;
-    // only for the grids whose CTAs are few per SM (their allocations then
-    // never wait on one another): 2^12 (2 CTAs, 256 columns each) and 2^13
-    static constexpr bool ENABLED = (LOGN == 12 || LOGN == 13) && NEED <= 512 && T >= 256;
+    // one CTA per problem: the grids whose registers admit no more CTAs per
+    // SM than the columns do (2^8: 8 of 64, 2^10: 4 of 128 columns, 2^11 and
+    // 2^12: 2 of 256, 2^13: 1), so an allocation never waits; clusters:
+    // always (one CTA per SM, SmShared)
+    static constexpr bool ENABLED = NEED <= 512 && E >= 4 && (C > 1 || LOGN <= 13);
+    static_assert(C == 1 || ENABLED, "clusters keep their scratch in tensor memory");
+    template <typename R>
+    static constexpr bool phasors() { return ENABLED && (FIELDS == 3 || sizeof(R) == 4); }
 };
 
 __device__ __forceinline__ void tm_st16(uint32_t a, const uint32_t (&r)[16]) {
@@ -227,6 +289,24 @@ __device__ __forceinline__ void tm_ld16(uint32_t a, uint32_t (&r)[16]) {
         : "r"(a)
         : "memory");
 }
+__device__ __forceinline__ void tm_st8(uint32_t a, const uint32_t (&r)[8]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(a),
+        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+        : "memory");
+}
+__device__ __forceinline__ void tm_ld8(uint32_t a, uint32_t (&r)[8]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+          "=r"(r[7])
+        : "r"(a)
+        : "memory");
+}
+__device__ __forceinline__ void tm_st(uint32_t a, const uint32_t (&r)[16]) { tm_st16(a, r); }
+__device__ __forceinline__ void tm_st(uint32_t a, const uint32_t (&r)[8]) { tm_st8(a, r); }
+__device__ __forceinline__ void tm_ld(uint32_t a, uint32_t (&r)[16]) { tm_ld16(a, r); }
+__device__ __forceinline__ void tm_ld(uint32_t a, uint32_t (&r)[8]) { tm_ld8(a, r); }
 __device__ __forceinline__ void tm_wait_st() {
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
@@ -252,44 +332,44 @@ __device__ __forceinline__ void unpack_words(const uint32_t* w, cx<double>& v) {
     v.im = __hiloint2double((int)w[3], (int)w[2]);
 }
 
-// This thread's two scratch fields (its own E bins) in precision R.
-template <typename R, int LOGN, int LOGE>
+// This thread's scratch fields (its own E bins) in precision R, in chunks of
+// VPC values.
+template <typename R, int LOGN, int C>
 struct TmScratch {
-    using L = TmLayout<LOGN, LOGE>;
+    using L = TmLayout<LOGN, C>;
     static constexpr int E = L::E;
     static constexpr int WPV = (int)(2 * sizeof(R) / 4);  // words per complex value
-    static constexpr int VPC = 16 / WPV;                  // values per 16-word chunk
+    // values per chunk: the loads of a chunk have to fit the registers
+    // (FP64 with 512 threads: half as many)
+    static constexpr int VPC = E < 4 ? E : sizeof(R) == 8 && E < 16 ? 2 : 4;
     static constexpr int CH = E / VPC;                    // chunks per field
-    static_assert(!L::ENABLED || E % VPC == 0, "a field is whole chunks");
+    static constexpr int W = VPC * WPV < 8 ? 8 : VPC * WPV;  // words per chunk
+    static_assert(!L::ENABLED || W == VPC * WPV, "a field is whole chunks");
     uint32_t a0;  // this warp's field 0, column 0
     __device__ explicit TmScratch(uint32_t tm) {
         const int w = threadIdx.x >> 5;
         a0 = tm + ((uint32_t)(32 * (w & 3)) << 16) + (uint32_t)((w >> 2) * L::COLS_WARP);
     }
     __device__ __forceinline__ uint32_t addr(int f, int c) const {
-        return a0 + (uint32_t)(f * 4 * E + c * 16);
+        return a0 + (uint32_t)(f * 4 * E + c * W);
     }
-    __device__ __forceinline__ void put(int f, const cx<R> (&v)[E]) const {
+    __device__ __forceinline__ void put_chunk(int f, int c, const cx<R> (&v)[VPC]) const {
+        uint32_t w[W];
 #pragma unroll
-        for (int c = 0; c < CH; c++) {
-            uint32_t w[16];
-#pragma unroll
-            for (int j = 0; j < VPC; j++) pack_words(v[c * VPC + j], w + j * WPV);
-            tm_st16(addr(f, c), w);
-        }
-        tm_wait_st();
+        for (int j = 0; j < VPC; j++) pack_words(v[j], w + j * WPV);
+        tm_st(addr(f, c), w);
     }
     __device__ __forceinline__ void get(int f, int c, cx<R> (&o)[VPC]) const {
-        uint32_t w[16];
-        tm_ld16(addr(f, c), w);
+        uint32_t w[W];
+        tm_ld(addr(f, c), w);
         tm_wait_ld();
 #pragma unroll
         for (int j = 0; j < VPC; j++) unpack_words(w + j * WPV, o[j]);
     }
     __device__ __forceinline__ void get2(int c, cx<R> (&o0)[VPC], cx<R> (&o1)[VPC]) const {
-        uint32_t w0[16], w1[16];
-        tm_ld16(addr(0, c), w0);
-        tm_ld16(addr(1, c), w1);
+        uint32_t w0[W], w1[W];
+        tm_ld(addr(0, c), w0);
+        tm_ld(addr(1, c), w1);
         tm_wait_ld();
 #pragma unroll
         for (int j = 0; j < VPC; j++) {
@@ -302,9 +382,9 @@ struct TmScratch {
 // Allocate the CTA's scratch columns (warp 0) and publish the address through
 // the shared-memory slot; every thread of the CTA calls it.  The caller frees
 // them with tm_free before the CTA exits.
-template <int LOGN, int LOGE>
+template <int LOGN, int C>
 __device__ __forceinline__ uint32_t tm_alloc(uint32_t* slot) {
-    using L = TmLayout<LOGN, LOGE>;
+    using L = TmLayout<LOGN, C>;
     if constexpr (!L::ENABLED) {
         return kNoTmem;
     } else {
@@ -320,9 +400,9 @@ __device__ __forceinline__ uint32_t tm_alloc(uint32_t* slot) {
         return *slot;
     }
 }
-template <int LOGN, int LOGE>
+template <int LOGN, int C>
 __device__ __forceinline__ void tm_free(uint32_t tm) {
-    using L = TmLayout<LOGN, LOGE>;
+    using L = TmLayout<LOGN, C>;
     if constexpr (L::ENABLED) {
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncthreads();
@@ -332,312 +412,580 @@ __device__ __forceinline__ void tm_free(uint32_t tm) {
     }
 }
 
-// Block-level pieces of one problem's solve in RHS precision R.
-template <typename R, int LOGN, int LOGE>
+struct NoLoad {  // the forward reads no stored field
+    struct Raw {};
+};
+
+// What a run of right-hand-side evaluations starts from: the stages
+// [stage, stage + count) of one attempt, or (stage 0) one evaluation of a
+// given field.  Each stage's input is built in the registers its first
+// transform starts from; the derivative of the stage before it is still there.
+struct StageRun {
+    int stage, count;
+    const double* x;     // FP64 state (workspace order; stage 0 with xbin: bin order)
+    int xbin;
+    const void* k1;      // stage 0: x + c k1 (null: x); with x null: the field itself
+    double c;
+    double* copy;        // stage 0: x also goes here (nullable)
+    void* out;           // stage 0: where the derivative goes
+    double z, zload;     // stage 0: position, and that of the forward field (adjoint)
+    char* kb;            // stage vectors, ks bytes apart, and their FSAL permutation
+    size_t ks;
+    int perm;
+    // logical stage i: the permutation swaps stages 0 and 6 (an index, not a
+    // table of pointers: a pointer load in front of every stage's data loads
+    // cost as much as the data, 1.7 k of 5.4 k cycles per chunk at 2^10)
+    __device__ __forceinline__ char* stage_vec(int i) const {
+        const int p = perm && (i == 0 || i == 6) ? 6 - i : i;
+        return kb + (size_t)p * ks;
+    }
+    double cz, dt;       // stage i is evaluated at cz + c_i dt
+    double* xnew;        // stage 7: the new state
+    int want_err;        // stage 7: also the error partial, weights and norm
+    double at, rt;
+    // adjoint: the stored steps [seg_lo, seg_hi) of the forward, or a field
+    int seg_lo, seg_hi;
+    const double* ufwd;
+    int pre;             // the first exchange waits for the group
+};
+
+// Pieces of one problem's solve in RHS precision R over a group of C CTAs.
+// Workspace fields (states, stages, scratch, checkpoints, interpolants) are
+// private to the thread that owns their bins and lie in thread order
+// (own(s)), tables and caller arrays in bin order (bin(s)).
+//
+// Code size is a first-order cost here: with one to four warps per scheduler
+// nothing hides an instruction-cache miss, and every evaluation runs the
+// whole body once.  So only the transforms and the pointwise terms between
+// them are unrolled over the thread's values; the stage input and the
+// derivative's way out are rolled loops over chunks of VPC values that pass
+// through the scratch slots (tensor memory).  Unrolling those as well made
+// the forward evaluation 147 KB of code instead of 44 KB and every part of
+// it slower (Nt = 2^10: radix-16 pass with twiddles 711 against 474 cycles).
+template <typename R, typename RMAX, int LOGN, int CL>
 struct SmSolver {
-    using S = FftShape<LOGN, LOGE>;
-    static constexpr int N = S::N, E = S::E, T = S::T;
+    using XF = XForm<R, RMAX, LOGN, CL>;
+    static constexpr int N = XF::N, E = XF::E;
     static constexpr int P = sizeof(R) == 8 ? 1 : 0;  // table precision index
     using C = cx<R>;
-    using IO = FieldIO<C, LOGN, LOGE>;
+    using TM = TmLayout<LOGN, CL>;
+    using TMS = TmScratch<R, LOGN, CL>;
+    static constexpr int VPC = TMS::VPC, CH = TMS::CH;
+    static constexpr bool PHC = TM::template phasors<R>();  // phasors kept in tensor memory
+    static constexpr int PHF = sizeof(R) == 8 ? 2 : 1;       // ... in this slot
 
     const SlotDesc& d;
-    void* sm;       // padded transform buffer
-    double* red;    // 32 doubles
-    Twiddles<R, LOGN> tw;  // two-level table in shared memory
+    XF xf;
     const C* __restrict__ Heff;
     const R* __restrict__ ss;
     const double* __restrict__ Dturns;
     C* scr0;
     C* scr1;
     uint32_t tm;  // tensor-memory scratch of the CTA, or kNoTmem: scr0 / scr1 in global memory
-    using TMS = TmScratch<R, LOGN, LOGE>;
-    static constexpr int VPC = TMS::VPC;
 
-    __device__ SmSolver(const SlotDesc& dd, void* smem, double* r, uint32_t tmaddr = kNoTmem)
-        : d(dd), sm(smem), red(r), tw(Twiddles<R, LOGN>::at(smem_twiddles<R, LOGN>(r))),
+    __device__ SmSolver(const SlotDesc& dd, unsigned char* smem, int rank, uint32_t tmaddr = kNoTmem)
+        : d(dd), xf(smem, smem_tables<R, RMAX, LOGN, CL>(smem), rank),
           Heff((const C*)dd.Heff[P]), ss((const R*)dd.ss[P]), Dturns(dd.Dturns),
           scr0((C*)dd.scr[0]), scr1((C*)dd.scr[1]), tm(tmaddr) {}
 
-    __device__ __forceinline__ static int bin(int s) { return threadIdx.x + T * s; }
+    __device__ __forceinline__ int bin(int s) const { return xf.bin(s); }
+    __device__ __forceinline__ int own(int s) const { return xf.own(s); }
+    __device__ __forceinline__ bool tmem() const { return TM::ENABLED && tm != kNoTmem; }
 
-    // One right-hand-side evaluation, forward (adj = false) or adjoint, as a
-    // runtime loop over its transforms so the kernel holds one copy of the
-    // FFT code (inverse transforms run as conj∘F∘conj):
-    //   forward  f0: ũ e^{iDz} -F-> u_t       f1: (γ|u_t|², 0) -F->
+    // ---- scratch slots: chunk c (values c VPC ..) of slot f ----
+    __device__ __forceinline__ void put(int f, int c, const C (&v)[VPC]) const {
+        if (tmem()) {
+            TMS(tm).put_chunk(f, c, v);
+        } else {
+            C* s = f ? scr1 : scr0;
+#pragma unroll
+            for (int j = 0; j < VPC; j++) s[own(c * VPC + j)] = v[j];
+        }
+    }
+    __device__ __forceinline__ void get(int f, int c, C (&v)[VPC]) const {
+        if (tmem()) {
+            TMS(tm).get(f, c, v);
+        } else {
+            const C* s = f ? scr1 : scr0;
+#pragma unroll
+            for (int j = 0; j < VPC; j++) v[j] = s[own(c * VPC + j)];
+        }
+    }
+    __device__ __forceinline__ void wait_put() const {
+        if (tmem()) tm_wait_st();
+    }
+    __device__ __forceinline__ void put_all(int f, const C (&v)[E]) const {
+#pragma unroll
+        for (int c = 0; c < CH; c++) {
+            C t[VPC];
+#pragma unroll
+            for (int j = 0; j < VPC; j++) t[j] = v[c * VPC + j];
+            put(f, c, t);
+        }
+        wait_put();
+    }
+    __device__ __forceinline__ void get_all(int f, C (&v)[E]) const {
+#pragma unroll
+        for (int c = 0; c < CH; c++) {
+            C t[VPC];
+            get(f, c, t);
+#pragma unroll
+            for (int j = 0; j < VPC; j++) v[c * VPC + j] = t[j];
+        }
+    }
+
+    // The transforms of one right-hand side, forward (adj = false) or
+    // adjoint, from the input in v (ũ e^{iDz}, or λ̃ e^{iDz} τ with
+    // ũ(z) e^{iDz} in slot 1) to the nonlinear term back in frequency, as a
+    // runtime loop over the transforms so the kernel holds one
+    // copy of each direction (inverse transforms run as conj∘F∘conj):
+    //   forward  f0: -F-> u_t                 f1: (γ|u_t|², 0) -F->
     //            f2: ·Heff -F⁻¹-> N h∗I       f3: ((1-fR)I + h∗I) u_t -F⁻¹->
-    //            post: dũ = i e^{-iDz} τ (·)/N
-    //   adjoint  f0: λ̃ e^{iDz} τ -F-> λ_t     f1: ũ(z) e^{iDz} -F-> u_t
+    //   adjoint  f0: -F-> λ_t                 f1: -F-> u_t
     //            f2: (I, Y) -F-> X            f3: split X into Î, Ŷ;
     //                Heff Î + i conj(Heff) Ŷ -F⁻¹-> N (h∗I + i h̃⋆Y)
-    //            f4: η -F⁻¹->                post: dλ̃ = i e^{-iDz} (·)/N
-    // load_u(v) fills v with the forward field ũ(z) for the adjoint.
-    template <class LoadU>
-    __device__ void rhs(const bool adj, const double z, C (&v)[E], LoadU&& load_u) {
+    //            f4: η -F⁻¹->
+    __device__ __forceinline__ void transforms(const bool adj, C (&v)[E], const bool pre) const {
         const R g = (R)d.gamma, ofr = (R)d.one_m_fR, invn = R(1) / R(N);
         const int nfft = adj ? 5 : 4;
 #pragma unroll 1
         for (int f = 0; f < nfft; f++) {
-            bool inv = false;
+            bool inv = false, to_a = false, presync = false;
             const int op = adj ? 8 + f : f;
-            if (op == 0) {
-#pragma unroll
-                for (int s = 0; s < E; s++) v[s] = cmul(v[s], phasor<R>(Dturns[bin(s)], z));
+            if (f == 0) {
+                presync = pre;
             } else if (op == 1) {
-                if (TmLayout<LOGN, LOGE>::ENABLED && tm != kNoTmem) {
-                    TMS(tm).put(0, v);
+                put_all(0, v);
 #pragma unroll
-                    for (int s = 0; s < E; s++) v[s] = mk(g * abs2(v[s]), R(0));
-                } else {
-#pragma unroll
-                    for (int s = 0; s < E; s++) {
-                        scr0[bin(s)] = v[s];
-                        v[s] = mk(g * abs2(v[s]), R(0));
-                    }
-                }
+                for (int s = 0; s < E; s++) v[s] = mk(g * abs2(v[s]), R(0));
+                to_a = true;
             } else if (op == 2) {
 #pragma unroll
                 for (int s = 0; s < E; s++) v[s] = cmul(v[s], Heff[bin(s)]);
                 inv = true;
             } else if (op == 3) {
-                if (TmLayout<LOGN, LOGE>::ENABLED && tm != kNoTmem) {
-                    const TMS ts(tm);
 #pragma unroll
-                    for (int c = 0; c < TMS::CH; c++) {
-                        C u[VPC];
-                        ts.get(0, c, u);
+                for (int c = 0; c < CH; c++) {
+                    C u[VPC];
+                    get(0, c, u);
 #pragma unroll
-                        for (int j = 0; j < VPC; j++) {
-                            const int s = c * VPC + j;
-                            const R fac = ofr * (g * abs2(u[j])) + v[s].re * invn;
-                            v[s] = scale(u[j], fac);
-                        }
-                    }
-                } else {
-#pragma unroll
-                    for (int s = 0; s < E; s++) {
-                        const C ut = scr0[bin(s)];
-                        const R fac = ofr * (g * abs2(ut)) + v[s].re * invn;
-                        v[s] = scale(ut, fac);
+                    for (int j = 0; j < VPC; j++) {
+                        const int s = c * VPC + j;
+                        const R fac = ofr * (g * abs2(u[j])) + v[s].re * invn;
+                        v[s] = scale(u[j], fac);
                     }
                 }
-                inv = true;
-            } else if (op == 8) {
-#pragma unroll
-                for (int s = 0; s < E; s++) {
-                    const int b = bin(s);
-                    v[s] = scale(cmul(v[s], phasor<R>(Dturns[b], z)), ss[b]);
-                }
+                inv = to_a = true;
             } else if (op == 9) {
-                if (TmLayout<LOGN, LOGE>::ENABLED && tm != kNoTmem) {
-                    TMS(tm).put(0, v);
-                } else {
-#pragma unroll
-                    for (int s = 0; s < E; s++) scr0[bin(s)] = v[s];
-                }
-                load_u(v);
-#pragma unroll
-                for (int s = 0; s < E; s++) v[s] = cmul(v[s], phasor<R>(Dturns[bin(s)], z));
+                put_all(0, v);
+                get_all(1, v);
+                presync = true;  // f0's warps may still be in the region buffer
             } else if (op == 10) {
-                if (TmLayout<LOGN, LOGE>::ENABLED && tm != kNoTmem) {
-                    const TMS ts(tm);
-                    ts.put(1, v);
+                put_all(1, v);
 #pragma unroll
-                    for (int c = 0; c < TMS::CH; c++) {
-                        C l[VPC];
-                        ts.get(0, c, l);
+                for (int c = 0; c < CH; c++) {
+                    C l[VPC];
+                    get(0, c, l);
 #pragma unroll
-                        for (int j = 0; j < VPC; j++) {
-                            const int s = c * VPC + j;
-                            const R I = g * abs2(v[s]);
-                            const R Y = g * (l[j].im * v[s].re - l[j].re * v[s].im);
-                            v[s] = mk(I, Y);
-                        }
-                    }
-                } else {
-#pragma unroll
-                    for (int s = 0; s < E; s++) {
-                        const int b = bin(s);
-                        const C lt = scr0[b];
-                        scr1[b] = v[s];
+                    for (int j = 0; j < VPC; j++) {
+                        const int s = c * VPC + j;
                         const R I = g * abs2(v[s]);
-                        const R Y = g * (lt.im * v[s].re - lt.re * v[s].im);  // γ Im(λ u*)
+                        const R Y = g * (l[j].im * v[s].re - l[j].re * v[s].im);  // γ Im(λ u*)
                         v[s] = mk(I, Y);
                     }
                 }
+                to_a = true;
             } else if (op == 11) {
-                // split the two real spectra (I and Y) with X[k] and conj(X[-k]);
-                // Heff Î + i conj(Heff) Ŷ
-                const C* __restrict__ Hp = Heff;
-                split_pair_apply<R, LOGN, LOGE>(v, sm, [Hp](int b) { return Hp[b]; });
+                // split the two real spectra (I and Y) with X[k] and conj(X[-k]):
+                // Î = (X[k] + conj(X[-k]))/2, i Ŷ = (X[k] - conj(X[-k]))/2;
+                // Heff Î + i conj(Heff) Ŷ = Re Heff X[k] + i Im Heff conj(X[-k])
+                xf.mirror_apply(v, Heff);
                 inv = true;
             } else {  // op == 12
                 // η = λ_t (2(1-fR) I + h∗I) - (1-fR) γ λ_t* u_t² + 2i (h̃⋆Y) u_t
-                auto eta = [&](const C lt, const C ut, const C x) {
-                    const R I = g * abs2(ut);
-                    const R Rr = x.re * invn, Ri = x.im * invn;
-                    const C t1 = scale(lt, R(2) * ofr * I + Rr);
-                    const C t2 = scale(cmulc(cmul(ut, ut), lt), ofr * g);    // (1-fR)γ λ* u²
-                    const C t3 = mk(-R(2) * Ri * ut.im, R(2) * Ri * ut.re);  // 2i Ri u
-                    return t1 - t2 + t3;
-                };
-                if (TmLayout<LOGN, LOGE>::ENABLED && tm != kNoTmem) {
-                    const TMS ts(tm);
 #pragma unroll
-                    for (int c = 0; c < TMS::CH; c++) {
-                        C l[VPC], u[VPC];
-                        ts.get2(c, l, u);
-#pragma unroll
-                        for (int j = 0; j < VPC; j++) v[c * VPC + j] = eta(l[j], u[j], v[c * VPC + j]);
+                for (int c = 0; c < CH; c++) {
+                    C l[VPC], u[VPC];
+                    if (tmem()) {
+                        TMS(tm).get2(c, l, u);
+                    } else {
+                        get(0, c, l);
+                        get(1, c, u);
                     }
-                } else {
 #pragma unroll
-                    for (int s = 0; s < E; s++) {
-                        const int b = bin(s);
-                        v[s] = eta(scr0[b], scr1[b], v[s]);
+                    for (int j = 0; j < VPC; j++) {
+                        const C lt = l[j], ut = u[j], x = v[c * VPC + j];
+                        const R I = g * abs2(ut);
+                        const R Rr = x.re * invn, Ri = x.im * invn;
+                        const C t1 = scale(lt, R(2) * ofr * I + Rr);
+                        const C t2 = scale(cmulc(cmul(ut, ut), lt), ofr * g);    // (1-fR)γ λ* u²
+                        const C t3 = mk(-R(2) * Ri * ut.im, R(2) * Ri * ut.re);  // 2i Ri u
+                        v[c * VPC + j] = t1 - t2 + t3;
                     }
                 }
-                inv = true;
+                inv = to_a = true;
             }
             if (inv) conj_all(v);
-            block_fft<R, LOGN, LOGE>(v, sm, tw);
+            xf.transform(v, to_a, presync);
             if (inv) conj_all(v);
-        }
-#pragma unroll
-        for (int s = 0; s < E; s++) {
-            const int b = bin(s);
-            const C y = cmulc(v[s], phasor<R>(Dturns[b], z));  // e^{-iDz} x
-            const R sc = adj ? invn : ss[b] * invn;
-            v[s] = mk(-y.im * sc, y.re * sc);                      // i y (τ) / N
         }
     }
 
     // ---- stage helpers ---------------------------------------------------
     // logical stage i -> physical buffer; perm swaps stages 0 and 6 (FSAL)
-    __device__ __forceinline__ static C* kp(void* const (&k)[7], int perm, int i) {
+    __device__ __forceinline__ static C* kp(void* const* k, int perm, int i) {
         int p = (perm && (i == 0 || i == 6)) ? 6 - i : i;
         return (C*)k[p];
     }
 
-    // Stage combinations read the stage vectors stage-outer and point-inner:
-    // each thread issues the loads of SC of its points for one stage
-    // together, so SC loads are in flight per thread instead of one.  The
-    // per-point summation order (stage 0 first) is unchanged.
-    static constexpr int SC = E < 8 ? E : 8;                      // points per chunk
-    static constexpr int SC7 = E < 8 ? E : (sizeof(R) == 8 ? 4 : 8);  // stage 7: two sums
-    static_assert(E % SC == 0 && E % SC7 == 0, "chunks tile the thread's points");
-
-    // v = ũ_n + dt Σ_{j<st} a[st][j] k_j   (FP64 accumulation)
-    __device__ __forceinline__ void stage_input(int st, const double* u, void* const (&k)[7],
-                                                int perm, double dt, IO v) {
+    // The input field of stage st, with its phasors, into the slots: stages
+    // 1..5 ũ_n + dt Σ_{j<st} a[st][j] k_j (FP64 accumulation, stage 0
+    // first); 6 the new state, written to xnew in FP64, and the partial error
+    // dt Σ_{j<6} b̃_j k_j; 0 the probe field x + c k1.  All stage loads of a chunk are issued
+    // before the first is used: one L2 latency per chunk, where a loop over
+    // the stages waited for each.
+    template <bool ADJ, class Load>
+    __device__ __forceinline__ void input(const StageRun& in, const int st, const double z,
+                                          const Load& ld) const {
+        const C* k[6];
+        double a[6];
 #pragma unroll
-        for (int s0 = 0; s0 < E; s0 += SC) {
-            double ar[SC], ai[SC];
-#pragma unroll
-            for (int c = 0; c < SC; c++) ar[c] = ai[c] = 0.0;
+        for (int j = 0; j < 6; j++) {
+            k[j] = (const C*)in.stage_vec(j);
+            a[j] = kT5a[st][j];
+        }
+        const double dt = in.dt;
 #pragma unroll 1
-            for (int j = 0; j < st; j++) {
-                const C* __restrict__ kj = kp(k, perm, j);
-                const double a = kT5a[st][j];
-                C x[SC];
+        for (int c = 0; c < CH; c++) {
+            const int s0 = c * VPC;
+            C y[VPC], ph[VPC];
+            double Dt[VPC];
+            R tau[VPC];
+            cx<double> un[VPC];
+            typename Load::Raw raw;
+            if (st > 0) {
+                C x[6][VPC];
 #pragma unroll
-                for (int c = 0; c < SC; c++) x[c] = kj[bin(s0 + c)];
+                for (int j = 0; j < 6; j++)
+                    if (j < st) {
+#pragma unroll
+                        for (int i = 0; i < VPC; i++) x[j][i] = k[j][own(s0 + i)];
+                    }
+#pragma unroll
+                for (int i = 0; i < VPC; i++) un[i] = ld2(in.x, own(s0 + i));
+#pragma unroll
+                for (int i = 0; i < VPC; i++) Dt[i] = Dturns[bin(s0 + i)];
+                if constexpr (ADJ) {
+#pragma unroll
+                    for (int i = 0; i < VPC; i++) tau[i] = ss[bin(s0 + i)];
+                    ld.fetch(s0, raw);
+                }
+                double ar[VPC], ai[VPC];
+#pragma unroll
+                for (int i = 0; i < VPC; i++) ar[i] = ai[i] = 0.0;
+#pragma unroll
+                for (int j = 0; j < 6; j++)
+                    if (j < st) {
+#pragma unroll
+                        for (int i = 0; i < VPC; i++) {
+                            ar[i] += a[j] * (double)x[j][i].re;
+                            ai[i] += a[j] * (double)x[j][i].im;
+                        }
+                    }
+#pragma unroll
+                for (int i = 0; i < VPC; i++)
+                    y[i] = mk((R)(un[i].re + dt * ar[i]), (R)(un[i].im + dt * ai[i]));
+                if (st == 6) {
+                    double er[VPC], ei[VPC];
+#pragma unroll
+                    for (int i = 0; i < VPC; i++) er[i] = ei[i] = 0.0;
+#pragma unroll
+                    for (int j = 0; j < 6; j++) {
+                        const double bt = kT5bt[j];
+#pragma unroll
+                        for (int i = 0; i < VPC; i++) {
+                            er[i] += bt * (double)x[j][i].re;
+                            ei[i] += bt * (double)x[j][i].im;
+                        }
+                    }
+#pragma unroll
+                    for (int i = 0; i < VPC; i++) {
+                        const int b = own(s0 + i);
+                        const cx<double> u1 = mk(un[i].re + dt * ar[i], un[i].im + dt * ai[i]);
+                        st2(in.xnew, b, u1);
+                        if (in.want_err) st2(d.esv, b, mk(dt * er[i], dt * ei[i]));
+                    }
+                }
+            } else {
+                const C* k1 = (const C*)in.k1;
+#pragma unroll
+                for (int i = 0; i < VPC; i++) {
+                    const int s = s0 + i;
+                    Dt[i] = Dturns[bin(s)];
+                    if constexpr (ADJ) tau[i] = ss[bin(s)];
+                    const C f0 = k1 ? k1[own(s)] : mk(R(0), R(0));
+                    const cx<double> x = in.x ? ld2(in.x, in.xbin ? bin(s) : own(s)) : up(f0);
+                    if (in.copy) st2(in.copy, own(s), x);
+                    y[i] = k1 && in.x
+                               ? mk((R)(x.re + in.c * (double)f0.re), (R)(x.im + in.c * (double)f0.im))
+                               : down<R>(x);
+                }
+                if constexpr (ADJ) ld.fetch(s0, raw);
+            }
+#pragma unroll
+            for (int i = 0; i < VPC; i++) {
+                ph[i] = phasor<R>(Dt[i], z);
+                y[i] = cmul(y[i], ph[i]);
+                if constexpr (ADJ) y[i] = scale(y[i], tau[i]);
+            }
+            put(0, c, y);
+            if constexpr (ADJ) {
+                C u[VPC];
+                ld.eval(raw, s0, u);
+#pragma unroll
+                for (int i = 0; i < VPC; i++) u[i] = cmul(u[i], ph[i]);
+                put(1, c, u);
+            }
+            if constexpr (PHC) put(PHF, c, ph);
+        }
+        wait_put();
+    }
+
+    // slot 0 -> the derivative i e^{-iDz} (τ) x / N, stored in out; the
+    // thread's part of the error norm when the derivative is k7 of an attempt
+    template <bool ADJ>
+    __device__ __forceinline__ double output(const StageRun& in, const int st, const double z,
+                                             C* out) const {
+        const R invn = R(1) / R(N);
+#pragma unroll 1
+        for (int c = 0; c < CH; c++) {
+            const int s0 = c * VPC;
+            C v[VPC], ph[VPC];
+            R sc[VPC];
+            if constexpr (!PHC) {
+                double Dt[VPC];
+#pragma unroll
+                for (int i = 0; i < VPC; i++) Dt[i] = Dturns[bin(s0 + i)];
+#pragma unroll
+                for (int i = 0; i < VPC; i++) ph[i] = phasor<R>(Dt[i], z);
+            } else {
+                get(PHF, c, ph);
+            }
+#pragma unroll
+            for (int i = 0; i < VPC; i++) sc[i] = ADJ ? invn : ss[bin(s0 + i)] * invn;
+            get(0, c, v);
+#pragma unroll
+            for (int i = 0; i < VPC; i++) {
+                const C y = cmulc(v[i], ph[i]);  // e^{-iDz} x
+                v[i] = mk(-y.im * sc[i], y.re * sc[i]);
+                out[own(s0 + i)] = v[i];
+            }
+        }
+        return st == 6 && in.want_err ? error_norm(in, out) : 0.0;
+    }
+    // the thread's part of the error norm, k7 in k: Σ |dt Σ b̃_j k_j|² / w²,
+    // w = abstol + reltol max(|u_n|, |u_{n+1}|)
+    __device__ __forceinline__ double error_norm(const StageRun& in, const C* k) const {
+        const double dt = in.dt, bt = kT5bt[6];
+        constexpr int NC = E < 4 ? E : 4;
+        double acc = 0.0;
+#pragma unroll 1
+        for (int s0 = 0; s0 < E; s0 += NC) {
+            C v[NC];
+            cx<double> e6[NC], un[NC], u1[NC];
+#pragma unroll
+            for (int i = 0; i < NC; i++) {
+                const int b = own(s0 + i);
+                v[i] = k[b];
+                e6[i] = ld2(d.esv, b);
+                un[i] = ld2(in.x, b);
+                u1[i] = ld2(in.xnew, b);
+            }
+#pragma unroll
+            for (int i = 0; i < NC; i++) {
+                const double m0 = un[i].re * un[i].re + un[i].im * un[i].im;
+                const double m1 = u1[i].re * u1[i].re + u1[i].im * u1[i].im;
+                const double w = rcp_nb(in.at + sqrt_nb(fmax(m0, m1)) * in.rt);
+                const double er = e6[i].re + dt * bt * (double)v[i].re;
+                const double ei = e6[i].im + dt * bt * (double)v[i].im;
+                acc += (er * er + ei * ei) * (w * w);
+            }
+        }
+        return acc;
+    }
+
+    // The same with the thread's values unrolled, in registers from the input
+    // to the stored derivative, for 16 warps per SM.  There the warps hide
+    // one another's latencies and instruction fetches, and the loads in
+    // flight per thread decide: at Nt = 2^13 on one CTA the rolled loops
+    // above took 27.6 ms per gradient, this form 22.5.
+    static constexpr bool WIDE = XF::TC >= 512 && E >= 16;
+    static constexpr int SC = E < 8 ? E : 8;
+    template <bool ADJ, class Load>
+    __device__ __forceinline__ void input_wide(const StageRun& in, const int st, const double z,
+                                               const Load& ld, C (&v)[E]) const {
+        const double dt = in.dt;
+        if (st > 0 && st < 6) {
+#pragma unroll
+            for (int s0 = 0; s0 < E; s0 += SC) {
+                double ar[SC], ai[SC];
+#pragma unroll
+                for (int c = 0; c < SC; c++) ar[c] = ai[c] = 0.0;
+#pragma unroll 1
+                for (int j = 0; j < st; j++) {
+                    const C* __restrict__ kj = (const C*)in.stage_vec(j);
+                    const double a = kT5a[st][j];
+                    C x[SC];
+#pragma unroll
+                    for (int c = 0; c < SC; c++) x[c] = kj[own(s0 + c)];
+#pragma unroll
+                    for (int c = 0; c < SC; c++) {
+                        ar[c] += a * (double)x[c].re;
+                        ai[c] += a * (double)x[c].im;
+                    }
+                }
 #pragma unroll
                 for (int c = 0; c < SC; c++) {
-                    ar[c] += a * (double)x[c].re;
-                    ai[c] += a * (double)x[c].im;
+                    const cx<double> un = ld2(in.x, own(s0 + c));
+                    v[s0 + c] = mk((R)(un.re + dt * ar[c]), (R)(un.im + dt * ai[c]));
                 }
             }
+        } else if (st == 6) {
+            constexpr int SC7 = sizeof(R) == 8 ? 4 : 8;  // two sums per point
 #pragma unroll
-            for (int c = 0; c < SC; c++) {
-                const cx<double> un = ld2(u, bin(s0 + c));
-                v[s0 + c] = mk((R)(un.re + dt * ar[c]), (R)(un.im + dt * ai[c]));
-            }
-        }
-    }
-
-    // stage 7 input = ũ_{n+1} (written to unew in FP64), partial error
-    // dt Σ_{j<7} b̃_j k_j and the weights abstol + reltol max(|u_n|,|u_{n+1}|)
-    __device__ __forceinline__ void stage7_input(const double* u, double* unew,
-                                                 void* const (&k)[7], int perm, double dt,
-                                                 double abstol, double reltol, IO v,
-                                                 bool want_err) {
+            for (int s0 = 0; s0 < E; s0 += SC7) {
+                double ar[SC7], ai[SC7], er[SC7], ei[SC7];
 #pragma unroll
-        for (int s0 = 0; s0 < E; s0 += SC7) {
-            double ar[SC7], ai[SC7], er[SC7], ei[SC7];
-#pragma unroll
-            for (int c = 0; c < SC7; c++) ar[c] = ai[c] = er[c] = ei[c] = 0.0;
+                for (int c = 0; c < SC7; c++) ar[c] = ai[c] = er[c] = ei[c] = 0.0;
 #pragma unroll 1
-            for (int j = 0; j < 6; j++) {
-                const C* __restrict__ kj = kp(k, perm, j);
-                const double a = kT5a[6][j], bt = kT5bt[j];
-                C x[SC7];
+                for (int j = 0; j < 6; j++) {
+                    const C* __restrict__ kj = (const C*)in.stage_vec(j);
+                    const double a = kT5a[6][j], bt = kT5bt[j];
+                    C x[SC7];
 #pragma unroll
-                for (int c = 0; c < SC7; c++) x[c] = kj[bin(s0 + c)];
+                    for (int c = 0; c < SC7; c++) x[c] = kj[own(s0 + c)];
+#pragma unroll
+                    for (int c = 0; c < SC7; c++) {
+                        ar[c] += a * (double)x[c].re;
+                        ai[c] += a * (double)x[c].im;
+                        er[c] += bt * (double)x[c].re;
+                        ei[c] += bt * (double)x[c].im;
+                    }
+                }
 #pragma unroll
                 for (int c = 0; c < SC7; c++) {
-                    ar[c] += a * (double)x[c].re;
-                    ai[c] += a * (double)x[c].im;
-                    er[c] += bt * (double)x[c].re;
-                    ei[c] += bt * (double)x[c].im;
+                    const int b = own(s0 + c);
+                    const cx<double> un = ld2(in.x, b);
+                    const cx<double> u1 = mk(un.re + dt * ar[c], un.im + dt * ai[c]);
+                    st2(in.xnew, b, u1);
+                    if (in.want_err) st2(d.esv, b, mk(dt * er[c], dt * ei[c]));
+                    v[s0 + c] = down<R>(u1);
                 }
             }
+        } else {
+            const C* k1 = (const C*)in.k1;
+#pragma unroll 4
+            for (int s = 0; s < E; s++) {
+                const C f0 = k1 ? k1[own(s)] : mk(R(0), R(0));
+                const cx<double> x = in.x ? ld2(in.x, in.xbin ? bin(s) : own(s)) : up(f0);
+                if (in.copy) st2(in.copy, own(s), x);
+                scr0[own(s)] = k1 && in.x
+                                   ? mk((R)(x.re + in.c * (double)f0.re), (R)(x.im + in.c * (double)f0.im))
+                                   : down<R>(x);
+            }
 #pragma unroll
-            for (int c = 0; c < SC7; c++) {
-                const int b = bin(s0 + c);
-                const cx<double> un = ld2(u, b);
-                const cx<double> u1 = mk(un.re + dt * ar[c], un.im + dt * ai[c]);
-                st2(unew, b, u1);
-                if (want_err) {
-                    st2(d.esv, b, mk(dt * er[c], dt * ei[c]));
-                    const double m0 = sqrt(un.re * un.re + un.im * un.im);
-                    const double m1 = sqrt(u1.re * u1.re + u1.im * u1.im);
-                    d.skv[b] = abstol + fmax(m0, m1) * reltol;
-                }
-                v[s0 + c] = down<R>(u1);
+            for (int s = 0; s < E; s++) v[s] = scr0[own(s)];
+        }
+        phasors_and_field<ADJ>(z, ld);
+#pragma unroll
+        for (int c = 0; c < CH; c++) {
+            C ph[VPC];
+            get(PHS, c, ph);
+#pragma unroll
+            for (int i = 0; i < VPC; i++) {
+                const int s = c * VPC + i;
+                v[s] = cmul(v[s], ph[i]);
+                if constexpr (ADJ) v[s] = scale(v[s], ss[bin(s)]);
             }
         }
     }
-
-    // finish the error estimate with k7 (in v) -> EEst (block-uniform)
-    __device__ __forceinline__ double error_norm(IO k7, double dt) {
-        const double bt7 = kT5bt[6];
-        double acc = 0.0;
+    // the evaluation's phasors into a slot -- the one they stay in, or slot 0
+    // before and after the transforms need it -- and ũ(z) e^{iDz} into slot 1
+    static constexpr int PHS = PHC ? PHF : 0;
+    template <bool ADJ, class Load>
+    __device__ __forceinline__ void phasors_and_field(const double z, const Load& ld) const {
+#pragma unroll 1
+        for (int c = 0; c < CH; c++) {
+            typename Load::Raw raw;
+            C u[VPC], ph[VPC];
+            double Dt[VPC];
 #pragma unroll
-        for (int s = 0; s < E; s++) {
-            const int b = bin(s);
-            const cx<double> e6 = ld2(d.esv, b);
-            const double er = e6.re + dt * bt7 * (double)k7[s].re;
-            const double ei = e6.im + dt * bt7 * (double)k7[s].im;
-            const double w = d.skv[b];
-            acc += (er * er + ei * ei) / (w * w);
+            for (int i = 0; i < VPC; i++) Dt[i] = Dturns[bin(c * VPC + i)];
+            if constexpr (ADJ) ld.fetch(c * VPC, raw);
+#pragma unroll
+            for (int i = 0; i < VPC; i++) ph[i] = phasor<R>(Dt[i], z);
+            put(PHS, c, ph);
+            if constexpr (ADJ) {
+                ld.eval(raw, c * VPC, u);
+#pragma unroll
+                for (int i = 0; i < VPC; i++) u[i] = cmul(u[i], ph[i]);
+                put(1, c, u);
+            }
         }
-        const double tot = block_sum<T>(acc, red);
-        return sqrt(tot / (double)N);
+        wait_put();
+    }
+    template <bool ADJ>
+    __device__ __forceinline__ double output_wide(const StageRun& in, const int st, const double z,
+                                                  C (&v)[E], C* out) const {
+        const R invn = R(1) / R(N);
+        if constexpr (!PHC) phasors_and_field<false>(z, NoLoad{});
+#pragma unroll
+        for (int c = 0; c < CH; c++) {
+            C ph[VPC];
+            get(PHS, c, ph);
+#pragma unroll
+            for (int i = 0; i < VPC; i++) {
+                const int s = c * VPC + i;
+                const C y = cmulc(v[s], ph[i]);  // e^{-iDz} x
+                const R sc = ADJ ? invn : ss[bin(s)] * invn;
+                out[own(s)] = mk(-y.im * sc, y.re * sc);
+            }
+        }
+        return st == 6 && in.want_err ? error_norm(in, out) : 0.0;
+    }
+
+    // The run's evaluations; make_load(z) prepares the forward field's
+    // loader.  Returns the thread's part of the error norm after stage 6.
+    template <bool ADJ, class MakeLoad>
+    __device__ __forceinline__ double run(const StageRun& in, MakeLoad&& make_load) {
+        double acc = 0.0;
+        const int end = in.stage == 0 ? 1 : in.stage + in.count;
+        // E <= 8: the run starts at the first exchange buffer, which the run
+        // before may still be reading
+        if constexpr (XF::S::SMALL) XF::sync();
+#pragma unroll 1
+        for (int st = in.stage; st < end; st++) {
+            const double z = st == 0 ? in.z : in.cz + kT5c[st] * in.dt;
+            const auto ld = make_load(*this, st == 0 ? in.zload : z);
+            C* out = (C*)(st == 0 ? (char*)in.out : in.stage_vec(st));
+            C v[E];
+            if constexpr (WIDE) {
+                input_wide<ADJ>(in, st, z, ld, v);
+            } else {
+                input<ADJ>(in, st, z, ld);
+                get_all(0, v);
+            }
+            transforms(ADJ, v, in.pre && st == in.stage);
+            if constexpr (WIDE) {
+                acc = output_wide<ADJ>(in, st, z, v, out);
+            } else {
+                put_all(0, v);
+                acc = output<ADJ>(in, st, z, out);
+            }
+        }
+        return acc;
     }
 };
-
-// dense interpolant of a stored forward step (precision RF) at θ, into a
-// field of precision R
-template <typename RF, typename R, int LOGN, int LOGE>
-__device__ __forceinline__ void interp_step(const SlotDesc& d, int slot, double dtn, double th,
-                                            cx<R> (&w)[FftShape<LOGN, LOGE>::E]) {
-    using S = FftShape<LOGN, LOGE>;
-    constexpr int N = S::N, E = S::E, T = S::T;
-    const cx<RF>* sg = (const cx<RF>*)d.seg + (size_t)slot * 5 * N;
-    const double t2 = th * th, t3 = t2 * th, t4 = t3 * th;
-#pragma unroll
-    for (int s = 0; s < E; s++) {
-        const int b = threadIdx.x + T * s;
-        const cx<RF> c0 = sg[b], c1 = sg[N + b], c2 = sg[2 * N + b], c3 = sg[3 * N + b],
-                     c4 = sg[4 * N + b];
-        const double xr = (double)c0.re + dtn * (th * (double)c1.re + t2 * (double)c2.re +
-                                                 t3 * (double)c3.re + t4 * (double)c4.re);
-        const double xi = (double)c0.im + dtn * (th * (double)c1.im + t2 * (double)c2.im +
-                                                 t3 * (double)c3.im + t4 * (double)c4.im);
-        w[s] = mk((R)xr, (R)xi);
-    }
-}
 
 // PI controller: returns q and q11 (OrdinaryDiffEqCore stepsize_controller!)
 __device__ __forceinline__ double pi_q(double EEst, double qold, double& q11) {
@@ -665,118 +1013,146 @@ __device__ __forceinline__ double initdt_final(double dt0, double d1, double d2,
     return fmax(dtmin, fmin(fmin(100 * dt0, dt1), span));
 }
 
-// Forward field for the adjoint RHS: the dense interpolant of the stored step
-// of the current segment that holds zz, or an FP64 field given directly.
-template <typename RF, typename R, int LOGN, int LOGE>
-struct SegLoader {
-    static constexpr int E = FftShape<LOGN, LOGE>::E;
-    const SlotDesc& d;
-    int seg_lo, seg_hi;
-    double zz;
-    const double* direct;
-    __device__ void operator()(cx<R> (&w)[E]) const {
-        if (direct) {
-#pragma unroll
-            for (int s = 0; s < E; s++)
-                w[s] = down<R>(ld2(direct, threadIdx.x + FftShape<LOGN, LOGE>::T * s));
+// Forward field for the adjoint RHS: the dense interpolant (precision RF) of
+// the stored step of the current segment that holds zz, or an FP64 field
+// given directly (bin order).
+template <typename RF>
+struct SegNode {
+    int n = -1;              // the stored step found last, its start and length,
+    double z0, dt, z1;       // and the start of the next one
+    // the last stored step in [lo, hi) starting at or before zz (the logged
+    // step starts increase).  Successive evaluations mostly stay in one step
+    // or move to a neighbour, so the search starts from the last one found
+    // and reads the log only when it moves.
+    __device__ __forceinline__ void find(const double* lg, int lo, int hi, double zz) {
+        if (n < lo || n >= hi) {  // by bisection
+            int a = lo, b = hi - 1;
+            while (a < b) {
+                const int mid = (a + b + 1) >> 1;
+                if (lg[2 * mid] <= zz) a = mid;
+                else b = mid - 1;
+            }
+            set(lg, a, hi);
             return;
         }
-        // the last stored step of the segment starting at or before zz (the
-        // logged step starts increase): a bisection, so a long segment costs
-        // log2(length) dependent loads instead of one per step
-        const double* lg = d.steplog;
-        int n = seg_lo, hi = seg_hi - 1;
-        while (n < hi) {
-            const int mid = (n + hi + 1) >> 1;
-            if (lg[2 * mid] <= zz) n = mid;
-            else hi = mid - 1;
-        }
-        const double zn = lg[2 * n], dtn = lg[2 * n + 1];
-        interp_step<RF, R, LOGN, LOGE>(d, n - seg_lo, dtn, (zz - zn) / dtn, w);
+        while (n > lo && z0 > zz) set(lg, n - 1, hi);
+        while (n < hi - 1 && z1 <= zz) set(lg, n + 1, hi);
+    }
+    __device__ __forceinline__ void set(const double* lg, int i, int hi) {
+        n = i;
+        z0 = lg[2 * i];
+        dt = lg[2 * i + 1];
+        z1 = i + 1 < hi ? lg[2 * i + 2] : INFINITY;
     }
 };
-
-// Out-of-line RHS evaluations.  The FFT-heavy bodies get the full register
-// budget of the CTA instead of sharing it with the state machine's live
-// values; the 2E-register field crosses the call through local memory.
-template <typename R, int LOGN, int LOGE>
-__device__ __noinline__ void rhs_fwd_call(const SlotDesc* d, void* sm, double* red, double z,
-                                          FieldIO<cx<R>, LOGN, LOGE> vio,
-                                          uint32_t tm = kNoTmem) {
-    using Sol = SmSolver<R, LOGN, LOGE>;
-    Sol S(*d, sm, red, tm);
-    cx<R> v[Sol::E];
+template <typename RF, class Sol>
+struct SegLoader {
+    static constexpr int N = Sol::N, VPC = Sol::VPC;
+    const Sol& S;
+    const double* direct;
+    const cx<RF>* sg;
+    double th, dtn;
+    // the stored values of a chunk
+    struct Raw {
+        cx<RF> c[5][VPC];
+    };
+    __device__ __forceinline__ void fetch(int s0, Raw& w) const {
+        if (!direct) {
 #pragma unroll
-    for (int s = 0; s < Sol::E; s++) v[s] = vio[s];
-    if constexpr (FieldIO<cx<R>, LOGN, LOGE>::SMEM) __syncthreads();
-    S.rhs(false, z, v, [](cx<R>(&)[Sol::E]) {});
+            for (int q = 0; q < 5; q++)
 #pragma unroll
-    for (int s = 0; s < Sol::E; s++) vio[s] = v[s];
+                for (int j = 0; j < VPC; j++) w.c[q][j] = sg[(size_t)q * N + S.own(s0 + j)];
+        }
+    }
+    // ũ at values s0 .. s0 + VPC - 1 of this thread
+    __device__ __forceinline__ void eval(const Raw& r, int s0, typename Sol::C (&w)[VPC]) const {
+        if (direct) {
+#pragma unroll
+            for (int j = 0; j < VPC; j++) {
+                const cx<double> x = ld2(direct, S.bin(s0 + j));
+                w[j].re = x.re;
+                w[j].im = x.im;
+            }
+            return;
+        }
+        const double t2 = th * th, t3 = t2 * th, t4 = t3 * th;
+#pragma unroll
+        for (int j = 0; j < VPC; j++) {
+            w[j].re = (double)r.c[0][j].re +
+                      dtn * (th * (double)r.c[1][j].re + t2 * (double)r.c[2][j].re +
+                             t3 * (double)r.c[3][j].re + t4 * (double)r.c[4][j].re);
+            w[j].im = (double)r.c[0][j].im +
+                      dtn * (th * (double)r.c[1][j].im + t2 * (double)r.c[2][j].im +
+                             t3 * (double)r.c[3][j].im + t4 * (double)r.c[4][j].im);
+        }
+    }
+};
+// Out-of-line runs of RHS evaluations: the transform bodies get the full
+// register budget of the CTA instead of sharing it with the state machine's
+// live values.
+template <typename R, typename RMAX, int LOGN, int CL>
+__device__ __noinline__ double rhs_fwd_call(const SlotDesc* d, unsigned char* sm, int rank,
+                                            const StageRun* in, uint32_t tm = kNoTmem) {
+    using Sol = SmSolver<R, RMAX, LOGN, CL>;
+    Sol S(*d, sm, rank, tm);
+    return S.template run<false>(*in, [](const Sol&, double) { return NoLoad{}; });
 }
 
-template <typename RF, typename R, int LOGN, int LOGE>
-__device__ __noinline__ void rhs_adj_call(const SlotDesc* d, void* sm, double* red, double z,
-                                          FieldIO<cx<R>, LOGN, LOGE> vio, int seg_lo, int seg_hi,
-                                          double zload, const double* ufwd,
-                                          uint32_t tm = kNoTmem) {
-    using Sol = SmSolver<R, LOGN, LOGE>;
-    Sol S(*d, sm, red, tm);
-    cx<R> v[Sol::E];
-#pragma unroll
-    for (int s = 0; s < Sol::E; s++) v[s] = vio[s];
-    if constexpr (FieldIO<cx<R>, LOGN, LOGE>::SMEM) __syncthreads();
-    SegLoader<RF, R, LOGN, LOGE> ld{*d, seg_lo, seg_hi, zload, ufwd};
-    S.rhs(true, z, v, ld);
-#pragma unroll
-    for (int s = 0; s < Sol::E; s++) vio[s] = v[s];
+template <typename RF, typename R, int LOGN, int CL>
+__device__ __noinline__ double rhs_adj_call(const SlotDesc* d, unsigned char* sm, int rank,
+                                            const StageRun* in, uint32_t tm = kNoTmem) {
+    using Sol = SmSolver<R, R, LOGN, CL>;
+    Sol S(*d, sm, rank, tm);
+    SegNode<RF> node;
+    return S.template run<true>(*in, [&](const Sol& sol, double zz) {
+        SegLoader<RF, Sol> ld{sol, in->ufwd, nullptr, 0.0, 0.0};
+        if (!in->ufwd) {
+            node.find(d->steplog, in->seg_lo, in->seg_hi, zz);
+            ld.dtn = node.dt;
+            ld.th = (zz - node.z0) / node.dt;
+            ld.sg = (const cx<RF>*)d->seg + (size_t)(node.n - in->seg_lo) * 5 * Sol::N;
+        }
+        return ld;
+    });
 }
 
-// transform buffer (sized for the adjoint precision), 32 reduction doubles
-// and the two twiddle tables
-template <typename RA, int LOGN>
-constexpr size_t smem_bytes() {
-    return SmemPlan<RA, LOGN>::BYTES + 32 * sizeof(double) +
-           sizeof(cx<float>) * Twiddles<float, LOGN>::SIZE +
-           sizeof(cx<double>) * Twiddles<double, LOGN>::SIZE + 16;  // + the tensor-memory slot
-}
 // the shared-memory word tcgen05.alloc writes the tensor-memory address to
-template <typename RA, int LOGN>
+template <typename RMAX, int LOGN, int CL>
 __device__ __forceinline__ uint32_t* tm_slot(unsigned char* smraw) {
-    return reinterpret_cast<uint32_t*>(smraw + smem_bytes<RA, LOGN>() - 16);
+    return reinterpret_cast<uint32_t*>(smraw + SmShared<RMAX, LOGN, CL>::SLOT);
 }
 
 // One RHS evaluation on one CTA (unit parity of the right-hand sides):
 // in/ufwd/out are N complex doubles; forward in RF, adjoint in RA.
-template <typename RF, typename RA, int LOGN, int LOGE>
-__global__ void __launch_bounds__(FftShape<LOGN, LOGE>::T, 1)
+template <typename RF, typename RA, int LOGN>
+__global__ void __launch_bounds__(XShape<LOGN, 1>::T, 1)
     sm_rhs_kernel(const SlotDesc* __restrict__ d, int adjoint, double z,
                   const double* __restrict__ in, const double* __restrict__ ufwd,
                   double* __restrict__ out) {
-    using S = FftShape<LOGN, LOGE>;
+    using XF = XForm<RA, RA, LOGN, 1>;
     extern __shared__ __align__(16) unsigned char smraw[];
-    double* red = reinterpret_cast<double*>(smraw + SmemPlan<RA, LOGN>::BYTES);
-    const uint32_t tm = tm_alloc<LOGN, LOGE>(tm_slot<RA, LOGN>(smraw));
-    load_twiddles<LOGN>(*d, red);
+    const uint32_t tm = tm_alloc<LOGN, 1>(tm_slot<RA, LOGN, 1>(smraw));
+    load_tables<RA, LOGN, 1>(*d, smraw, 0);
+    StageRun si{};
+    si.x = in;
+    si.xbin = 1;
+    si.z = si.zload = z;
+    si.pre = 1;
+    si.ufwd = ufwd;
+    si.out = adjoint ? d->ka[0] : d->kf[0];
+    const XF xf(smraw, nullptr, 0);
     if (adjoint) {
-        using IO = FieldIO<cx<RA>, LOGN, LOGE>;
-        cx<RA> vl[IO::SMEM ? 1 : S::E];
-        const IO v{IO::SMEM ? reinterpret_cast<cx<RA>*>(smraw) : vl};
+        rhs_adj_call<RF, RA, LOGN, 1>(d, smraw, 0, &si, tm);
+        const cx<RA>* k = (const cx<RA>*)d->ka[0];
 #pragma unroll
-        for (int s = 0; s < S::E; s++) v[s] = down<RA>(ld2(in, threadIdx.x + S::T * s));
-        rhs_adj_call<RF, RA, LOGN, LOGE>(d, smraw, red, z, v, 0, 0, 0.0, ufwd, tm);
-#pragma unroll
-        for (int s = 0; s < S::E; s++) st2(out, threadIdx.x + S::T * s, up(v[s]));
+        for (int s = 0; s < XF::E; s++) st2(out, xf.bin(s), up(k[xf.own(s)]));
     } else {
-        using IO = FieldIO<cx<RF>, LOGN, LOGE>;
-        cx<RF> vl[IO::SMEM ? 1 : S::E];
-        const IO v{IO::SMEM ? reinterpret_cast<cx<RF>*>(smraw) : vl};
+        rhs_fwd_call<RF, RA, LOGN, 1>(d, smraw, 0, &si, tm);
+        const cx<RF>* k = (const cx<RF>*)d->kf[0];
 #pragma unroll
-        for (int s = 0; s < S::E; s++) v[s] = down<RF>(ld2(in, threadIdx.x + S::T * s));
-        rhs_fwd_call<RF, LOGN, LOGE>(d, smraw, red, z, v, tm);
-#pragma unroll
-        for (int s = 0; s < S::E; s++) st2(out, threadIdx.x + S::T * s, up(v[s]));
+        for (int s = 0; s < XF::E; s++) st2(out, xf.bin(s), up(k[xf.own(s)]));
     }
-    tm_free<LOGN, LOGE>(tm);
+    tm_free<LOGN, 1>(tm);
 }
 
 // Steps [lo, hi) of the current sub-segment: the segment of checkpoint seg
@@ -813,44 +1189,45 @@ __device__ __forceinline__ int last_sub(const Desc& d, const State& st, int seg)
 }
 
 // Dense interpolant of an accepted step into sg (5 fields): c0 = ũ_n,
-// c_p = Σ_i r_ip k_i (Tsit5's free 4th-order interpolant), read stage-outer
-// over chunks of 4 points per thread as in stage_input.
-template <typename RF, int LOGN, int LOGE>
-__device__ __forceinline__ void store_interp(const SlotDesc& d, const double* u, int kperm,
+// c_p = Σ_i r_ip k_i (Tsit5's free 4th-order interpolant); all stage loads
+// of a chunk of points in flight together, as in stage_input.
+template <typename RF, class Sol>
+__device__ __forceinline__ void store_interp(const Sol& S, const double* u, int kperm,
                                              cx<RF>* sg) {
-    using S = FftShape<LOGN, LOGE>;
-    using Sol = SmSolver<RF, LOGN, LOGE>;
     using CF = cx<RF>;
-    constexpr int N = S::N, E = S::E;
+    const SlotDesc& d = S.d;
+    constexpr int N = Sol::N, E = Sol::E;
     constexpr int RC = E < 4 ? E : 4;
     static_assert(E % RC == 0, "chunks tile the thread's points");
+    const CF* k[7];
+    const size_t kfs = (CF*)d.kf[1] - (CF*)d.kf[0];
 #pragma unroll
-    for (int s0 = 0; s0 < E; s0 += RC) {
-        double cr[RC][4], ci[RC][4];
-#pragma unroll
-        for (int c = 0; c < RC; c++)
-#pragma unroll
-            for (int q = 0; q < 4; q++) cr[c][q] = ci[c][q] = 0.0;
+    for (int i = 0; i < 7; i++)
+        k[i] = (const CF*)d.kf[0] + (size_t)(kperm && (i == 0 || i == 6) ? 6 - i : i) * kfs;
 #pragma unroll 1
-        for (int i = 0; i < 7; i++) {
-            const CF* __restrict__ kv = Sol::kp(d.kf, kperm, i);
-            CF x[RC];
+    for (int s0 = 0; s0 < E; s0 += RC) {
+        CF x[7][RC];
+        cx<double> un[RC];
 #pragma unroll
-            for (int c = 0; c < RC; c++) x[c] = kv[Sol::bin(s0 + c)];
+        for (int i = 0; i < 7; i++)
 #pragma unroll
-            for (int c = 0; c < RC; c++)
+            for (int c = 0; c < RC; c++) x[i][c] = k[i][S.own(s0 + c)];
 #pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    cr[c][q] += kT5r[i][q] * (double)x[c].re;
-                    ci[c][q] += kT5r[i][q] * (double)x[c].im;
-                }
-        }
+        for (int c = 0; c < RC; c++) un[c] = ld2(u, S.own(s0 + c));
 #pragma unroll
         for (int c = 0; c < RC; c++) {
-            const int b = Sol::bin(s0 + c);
-            sg[b] = down<RF>(ld2(u, b));
+            const int b = S.own(s0 + c);
+            sg[b] = down<RF>(un[c]);
 #pragma unroll
-            for (int q = 0; q < 4; q++) sg[(q + 1) * N + b] = mk((RF)cr[c][q], (RF)ci[c][q]);
+            for (int q = 0; q < 4; q++) {
+                double cr = 0.0, ci = 0.0;
+#pragma unroll
+                for (int i = 0; i < 7; i++) {
+                    cr += kT5r[i][q] * (double)x[i][c].re;
+                    ci += kT5r[i][q] * (double)x[i][c].im;
+                }
+                sg[(size_t)(q + 1) * N + b] = mk((RF)cr, (RF)ci);
+            }
         }
     }
 }
@@ -883,13 +1260,13 @@ __device__ __forceinline__ bool state_in_bounds(const Desc& d, const State& st) 
     return ok;
 }
 
-template <typename RF, int LOGN, int LOGE>
-__device__ __forceinline__ void restore_checkpoint(const SlotDesc& d, int seg, SlotState& st) {
-    using S = FftShape<LOGN, LOGE>;
-    constexpr int N = S::N, E = S::E, T = S::T;
-#pragma unroll
+template <typename RF, class Sol>
+__device__ __forceinline__ void restore_checkpoint(const Sol& S, int seg, SlotState& st) {
+    const SlotDesc& d = S.d;
+    constexpr int N = Sol::N, E = Sol::E;
+#pragma unroll 4
     for (int s = 0; s < E; s++) {
-        const int b = threadIdx.x + T * s;
+        const int b = S.own(s);
         reinterpret_cast<double2*>(d.u[0])[b] =
             reinterpret_cast<const double2*>(d.ck_u)[(size_t)seg * N + b];
         ((cx<RF>*)d.kf[0])[b] = ((const cx<RF>*)d.ck_k1)[(size_t)seg * N + b];
@@ -900,29 +1277,25 @@ __device__ __forceinline__ void restore_checkpoint(const SlotDesc& d, int seg, S
     st.stage = 0;
 }
 
-// Hairer initial step, part 1 (after f0): stores f0 as the FSAL derivative,
-// returns the probe step dt0 (> 0) or, when no probe is needed, -dtinit.
-template <typename K, int LOGN, int LOGE>
-__device__ __forceinline__ double init_after_f0(const double* x0, cx<K>* k1,
-                                                FieldIO<cx<K>, LOGN, LOGE> v,
-                                                double at, double rt, double L, double dtmin,
-                                                double* red, double& d1_out) {
-    using S = FftShape<LOGN, LOGE>;
-    constexpr int N = S::N, E = S::E, T = S::T;
+// Hairer initial step, part 1 (after f0, in k1): the probe step dt0 (> 0)
+// or, when no probe is needed, -dtinit.  x0 in bin order for the launch.
+template <typename K, class Sol, class SumF>
+__device__ __forceinline__ double init_after_f0(const Sol& S, const double* x0, bool xbin,
+                                                const cx<K>* k1, double at, double rt, double L,
+                                                double dtmin, SumF&& sum, double& d1_out) {
+    constexpr int N = Sol::N, E = Sol::E;
     double s0 = 0.0, s1 = 0.0;
-#pragma unroll
+#pragma unroll 4
     for (int s = 0; s < E; s++) {
-        const int b = threadIdx.x + T * s;
-        k1[b] = v[s];
-        const cx<double> x = ld2(x0, b);
+        const cx<double> x = ld2(x0, xbin ? S.bin(s) : S.own(s));
         const double ax = sqrt(x.re * x.re + x.im * x.im);
         const double sk = at + ax * rt;
         s0 += (ax / sk) * (ax / sk);
-        const double af = sqrt(abs2(up(v[s])));
+        const double af = sqrt(abs2(up(k1[S.own(s)])));
         s1 += (af / sk) * (af / sk);
     }
-    const double d0 = sqrt(block_sum<T>(s0, red) / N);
-    const double d1 = sqrt(block_sum<T>(s1, red) / N);
+    const double d0 = sqrt(sum(s0) / N);
+    const double d1 = sqrt(sum(s1) / N);
     d1_out = d1;
     const double dt0 = initdt_first(d0, d1, L);
     if (!isfinite(d1)) return -dtmin;
@@ -930,62 +1303,64 @@ __device__ __forceinline__ double init_after_f0(const double* x0, cx<K>* k1,
     return dt0;
 }
 
-// Hairer initial step, part 2 (after the probe f1 at x0 ± dt0 f0)
-template <typename K, int LOGN, int LOGE>
-__device__ __forceinline__ double init_after_f1(const double* x0, const cx<K>* k1,
-                                                FieldIO<cx<K>, LOGN, LOGE> v,
-                                                double at, double rt, double dt0, double d1,
-                                                double L, double dtmin, double* red) {
-    using S = FftShape<LOGN, LOGE>;
-    constexpr int N = S::N, E = S::E, T = S::T;
+// Hairer initial step, part 2 (after the probe f1 at x0 ± dt0 f0, in kp)
+template <typename K, class Sol, class SumF>
+__device__ __forceinline__ double init_after_f1(const Sol& S, const double* x0, bool xbin,
+                                                const cx<K>* k1, const cx<K>* kp, double at,
+                                                double rt, double dt0, double d1, double L,
+                                                double dtmin, SumF&& sum) {
+    constexpr int N = Sol::N, E = Sol::E;
     double s2 = 0.0, ndiff = 0.0;
-#pragma unroll
+#pragma unroll 4
     for (int s = 0; s < E; s++) {
-        const int b = threadIdx.x + T * s;
-        const cx<double> x = ld2(x0, b);
+        const cx<double> x = ld2(x0, xbin ? S.bin(s) : S.own(s));
         const double sk = at + sqrt(x.re * x.re + x.im * x.im) * rt;
-        const cx<K> f0 = k1[b];
-        const double dr = (double)v[s].re - (double)f0.re;
-        const double di = (double)v[s].im - (double)f0.im;
+        const cx<K> f0 = k1[S.own(s)], f1 = kp[S.own(s)];
+        const double dr = (double)f1.re - (double)f0.re;
+        const double di = (double)f1.im - (double)f0.im;
         s2 += (dr * dr + di * di) / (sk * sk);
         ndiff += (dr != 0.0 || di != 0.0) ? 1.0 : 0.0;
     }
-    const double d2 = sqrt(block_sum<T>(s2, red) / N) / dt0;
-    const double nd = block_sum<T>(ndiff, red);
+    const double d2 = sqrt(sum(s2) / N) / dt0;
+    const double nd = sum(ndiff);
     return initdt_final(dt0, d1, d2, nd, dtmin, L);
 }
 
 // The state machine.  Each loop iteration performs at most one RHS
 // evaluation (forward in RF, adjoint in RA) plus the bookkeeping around it,
 // so the FFT code exists once per precision in the kernel.
-template <typename RF, typename RA, int LOGN, int LOGE>
-__global__ void __launch_bounds__(FftShape<LOGN, LOGE>::T, 1)
+// 128 registers per thread up to 2^12: 512 threads per SM
+constexpr int sm_min_ctas(int logn) {
+    return logn <= 7 ? 16 : logn <= 10 ? 1 << (11 - logn) : logn == 11 ? 2 : 1;
+}
+template <typename RF, typename RA, int LOGN, int CL>
+__global__ void __launch_bounds__(XShape<LOGN, CL>::TC, sm_min_ctas(LOGN))
     sm_advance_kernel(const SlotDesc* __restrict__ descs, SlotState* __restrict__ states,
                       const int* __restrict__ active, int max_evals) {
-    using SolF = SmSolver<RF, LOGN, LOGE>;
-    using SolA = SmSolver<RA, LOGN, LOGE>;
+    using SolF = SmSolver<RF, RA, LOGN, CL>;
+    using SolA = SmSolver<RA, RA, LOGN, CL>;
     using CF = cx<RF>;
     using CA = cx<RA>;
-    constexpr int N = SolF::N, E = SolF::E, T = SolF::T;
+    constexpr int N = SolF::N, E = SolF::E, T = SolF::XF::T;
     extern __shared__ __align__(16) unsigned char smraw[];
-    double* red = reinterpret_cast<double*>(smraw + SmemPlan<RA, LOGN>::BYTES);
+    double* red = reinterpret_cast<double*>(smraw + SmShared<RA, LOGN, CL>::RED);
 
-    const int slot = active[blockIdx.x];
+    const int slot = active[blockIdx.x / CL], rank = blockIdx.x % CL;
     const SlotDesc& d = descs[slot];
-    const uint32_t tm = tm_alloc<LOGN, LOGE>(tm_slot<RA, LOGN>(smraw));
-    load_twiddles<LOGN>(d, red);
-    SlotState st = states[slot];  // block-uniform copy
-    SolF SF(d, smraw, red);
-    SolA SA(d, smraw, red);
-    const int tid = threadIdx.x;
+    SlotState st = states[slot];  // group-uniform copy
+    if (st.phase == PH_DONE) return;
+    const uint32_t tm = tm_alloc<LOGN, CL>(tm_slot<RA, LOGN, CL>(smraw));
+    load_tables<RA, LOGN, CL>(d, smraw, rank);
+    SolF SF(d, smraw, rank);
+    const bool lead = rank == 0 && threadIdx.x == 0;
     const double L = d.L, dtmin = kEps * L;
-    using IOF = FieldIO<CF, LOGN, LOGE>;
-    using IOA = FieldIO<CA, LOGN, LOGE>;
-    CF vfl[IOF::SMEM ? 1 : E];  // local-memory field (Nt = 2^14 only)
-    CA val[IOA::SMEM ? 1 : E];
-    const IOF vf{IOF::SMEM ? reinterpret_cast<CF*>(smraw) : vfl};
-    const IOA va{IOA::SMEM ? reinterpret_cast<CA*>(smraw) : val};
+    int flip = 0;
+    auto sum = [&](double v) { return x_reduce<T, CL, false>(v, red, flip, rank); };
+    auto maxv = [&](double v) { return x_reduce<T, CL, true>(v, red, flip, rank); };
+    // the stage vectors of a slot lie one stride apart (work_create)
+    const size_t kfs = (char*)d.kf[1] - (char*)d.kf[0], kas = (char*)d.ka[1] - (char*)d.ka[0];
     int evals = 0;
+    int last = -1;  // precision of the last evaluation (its buffers may still be read)
 
     while (st.phase != PH_DONE && evals < max_evals) {
 #ifdef FL_CHECKED
@@ -1008,29 +1383,29 @@ __global__ void __launch_bounds__(FftShape<LOGN, LOGE>::T, 1)
                 // in-band bin (lowest index among equals) in place of the band.
                 const bool peak = d.objective == OBJ_RAMAN_PEAK;
                 double et = 0.0, eb = 0.0, emax = -1.0;
-#pragma unroll
+#pragma unroll 4
                 for (int s = 0; s < E; s++) {
-                    const int b = SolF::bin(s);
-                    const double e = energy(ld2(uf, b));
+                    const int b = SF.bin(s);
+                    const double e = energy(ld2(uf, SF.own(s)));
                     et += e;
                     if (d.mask[b]) {
                         eb += e;
                         emax = fmax(emax, e);
                     }
                 }
-                const double tot = block_sum<T>(et, red);
-                double band = block_sum<T>(eb, red);
+                const double tot = sum(et);
+                double band = sum(eb);
                 int pk = -1;
                 if (peak) {
-                    band = block_max<T>(emax, red);
+                    band = maxv(emax);
                     // lowest index as the largest key N - b (block_max folds from 0)
                     double key = 0.0;
-#pragma unroll
+#pragma unroll 4
                     for (int s = 0; s < E; s++) {
-                        const int b = SolF::bin(s);
-                        if (d.mask[b] && energy(ld2(uf, b)) == band) key = fmax(key, (double)(N - b));
+                        const int b = SF.bin(s);
+                        if (d.mask[b] && energy(ld2(uf, SF.own(s))) == band) key = fmax(key, (double)(N - b));
                     }
-                    pk = N - (int)block_max<T>(key, red);
+                    pk = N - (int)maxv(key);
                 }
                 const double cost = band / tot;
                 double sc = 1.0 / tot;
@@ -1040,34 +1415,34 @@ __global__ void __launch_bounds__(FftShape<LOGN, LOGE>::T, 1)
                     sc *= cost <= 1e-15 ? 0.0 : 10.0 / (log(10.0) * cost);
                 }
                 // e^{-iDL} (u_L (sel - J)/E) = ũ(L) (sel - J)/E, sel the band or peak bin
-#pragma unroll
+#pragma unroll 4
                 for (int s = 0; s < E; s++) {
-                    const int b = SolF::bin(s);
-                    const cx<double> x = ld2(uf, b);
+                    const int b = SF.bin(s);
+                    const cx<double> x = ld2(uf, SF.own(s));
                     const double sel = peak ? (b == pk ? 1.0 : 0.0) : (d.mask[b] ? 1.0 : 0.0);
                     const double f = (sel - cost) * sc;
-                    st2(lam, b, mk(x.re * f, x.im * f));
+                    st2(lam, SF.own(s), mk(x.re * f, x.im * f));
                 }
             } else {
                 st.J = 0.0;
-#pragma unroll
+#pragma unroll 4
                 for (int s = 0; s < E; s++) {
-                    const int b = SolF::bin(s);
+                    const int b = SF.bin(s);
                     const cx<double> x = ld2(d.lamL, b);
                     const cx<double> p = phasor<double>(d.Dturns[b], L);
-                    st2(lam, b, mk(x.re * p.re + x.im * p.im, x.im * p.re - x.re * p.im));
+                    st2(lam, SF.own(s), mk(x.re * p.re + x.im * p.im, x.im * p.re - x.re * p.im));
                 }
             }
             double mx = 0.0;
             bool finite = true;
-#pragma unroll
+#pragma unroll 4
             for (int s = 0; s < E; s++) {
-                const cx<double> x = ld2(lam, SolF::bin(s));
+                const cx<double> x = ld2(lam, SF.own(s));
                 const double a = sqrt(x.re * x.re + x.im * x.im);
                 if (!isfinite(a)) finite = false;
                 mx = fmax(mx, a);
             }
-            const double scl = block_max<T>(finite ? mx : INFINITY, red);
+            const double scl = maxv(finite ? mx : INFINITY);
             if (!isfinite(scl)) {
                 st.status = ST_NONFINITE;
                 st.phase = PH_DONE;
@@ -1090,17 +1465,17 @@ __global__ void __launch_bounds__(FftShape<LOGN, LOGE>::T, 1)
             }
             st.seg = (st.nsteps + st.ck_stride - 1) / st.ck_stride - 1;
             st.sub = last_sub(d, st, st.seg);
-            restore_checkpoint<RF, LOGN, LOGE>(d, st.seg, st);
+            restore_checkpoint<RF>(SF, st.seg, st);
             st.phase = PH_REC;
             continue;
         }
         if (st.phase == PH_FINAL) {
             // λ(0) = λ̃(0); ∂J/∂φ = 2 Re(conj(λ0) i u_shaped) (physics_models.jl:1042)
             const double* lam = d.lam[st.acur];
-#pragma unroll
+#pragma unroll 4
             for (int s = 0; s < E; s++) {
-                const int b = SolF::bin(s);
-                const cx<double> l = ld2(lam, b);
+                const int b = SF.bin(s);
+                const cx<double> l = ld2(lam, SF.own(s));
                 if (d.lam0_out) st2(d.lam0_out, b, l);
                 if (d.grad_out) {
                     const cx<double> us = ld2(d.u0, b);
@@ -1113,23 +1488,15 @@ __global__ void __launch_bounds__(FftShape<LOGN, LOGE>::T, 1)
 
         // ------------------------------------------------ build the stage input
         const bool adj = st.phase == PH_ADJ_INIT || st.phase == PH_ADJ;
-        double ze = 0.0, zload = 0.0;
+        StageRun in{};
         if (st.phase == PH_FWD_INIT) {
-            const CF* k1 = (const CF*)d.kf[0];
-#pragma unroll
-            for (int s = 0; s < E; s++) {
-                const int b = SolF::bin(s);
-                const cx<double> x = ld2(d.u0, b);
-                if (st.stage == 0) {
-                    st2(d.u[0], b, x);
-                    vf[s] = down<RF>(x);
-                } else {
-                    const CF f0 = k1[b];
-                    vf[s] = mk((RF)(x.re + st.cdt * (double)f0.re),
-                               (RF)(x.im + st.cdt * (double)f0.im));
-                }
-            }
-            ze = st.stage == 0 ? 0.0 : st.cdt;
+            in.x = d.u0;
+            in.xbin = 1;
+            in.copy = st.stage == 0 ? d.u[0] : nullptr;
+            in.k1 = st.stage == 0 ? nullptr : d.kf[0];
+            in.c = st.cdt;
+            in.out = d.kf[st.stage == 0 ? 0 : 1];
+            in.z = st.stage == 0 ? 0.0 : st.cdt;
         } else if (st.phase == PH_FWD || st.phase == PH_REC) {
             if (st.stage == 0) {
                 if (st.phase == PH_REC) {
@@ -1156,30 +1523,21 @@ __global__ void __launch_bounds__(FftShape<LOGN, LOGE>::T, 1)
                 }
                 st.stage = 1;
             }
-            const double* u = d.u[st.cur];
-            if (st.stage < 6)
-                SF.stage_input(st.stage, u, d.kf, st.kperm, st.cdt, vf);
-            else
-                SF.stage7_input(u, d.u[st.cur ^ 1], d.kf, st.kperm, st.cdt, d.abstol, d.reltol,
-                                vf, st.phase == PH_FWD);
-            ze = st.cz + kT5c[st.stage] * st.cdt;
+            in.x = d.u[st.cur];
+            in.kb = (char*)d.kf[0];
+            in.ks = kfs;
+            in.perm = st.kperm;
+            in.xnew = d.u[st.cur ^ 1];
+            in.want_err = st.phase == PH_FWD;
+            in.at = d.abstol;
+            in.rt = d.reltol;
         } else if (st.phase == PH_ADJ_INIT) {
-            const double* lam = d.lam[0];
-            const CA* k1 = (const CA*)d.ka[0];
-#pragma unroll
-            for (int s = 0; s < E; s++) {
-                const int b = SolF::bin(s);
-                const cx<double> x = ld2(lam, b);
-                if (st.stage == 0) {
-                    va[s] = down<RA>(x);
-                } else {
-                    const CA f0 = k1[b];
-                    va[s] = mk((RA)(x.re - st.cdt * (double)f0.re),
-                               (RA)(x.im - st.cdt * (double)f0.im));
-                }
-            }
-            ze = st.stage == 0 ? L : L - st.cdt;
-            zload = st.stage == 0 ? L : fmax(ze, d.steplog[2 * sub_segment(d, st).lo]);
+            in.x = d.lam[0];
+            in.k1 = st.stage == 0 ? nullptr : d.ka[0];
+            in.c = -st.cdt;
+            in.out = d.ka[st.stage == 0 ? 0 : 1];
+            in.z = st.stage == 0 ? L : L - st.cdt;
+            in.zload = st.stage == 0 ? L : fmax(in.z, d.steplog[2 * sub_segment(d, st).lo]);
         } else {  // PH_ADJ
             const double zlo = d.steplog[2 * sub_segment(d, st).lo];
             if (st.stage == 0) {
@@ -1203,36 +1561,47 @@ __global__ void __launch_bounds__(FftShape<LOGN, LOGE>::T, 1)
                 st.cdt = -adt;
                 st.stage = 1;
             }
-            const double* lam = d.lam[st.acur];
-            if (st.stage < 6)
-                SA.stage_input(st.stage, lam, d.ka, st.akperm, st.cdt, va);
-            else
-                SA.stage7_input(lam, d.lam[st.acur ^ 1], d.ka, st.akperm, st.cdt, st.abstol_adj,
-                                d.reltol, va, true);
-            ze = zload = st.cz + kT5c[st.stage] * st.cdt;
+            in.x = d.lam[st.acur];
+            in.kb = (char*)d.ka[0];
+            in.ks = kas;
+            in.perm = st.akperm;
+            in.xnew = d.lam[st.acur ^ 1];
+            in.want_err = 1;
+            in.at = st.abstol_adj;
+            in.rt = d.reltol;
         }
 
-        // ------------------------------------------------ one RHS evaluation
+        // ------------------------- the probe's evaluation, or the attempt's stages
+        const bool probe = st.phase == PH_FWD_INIT || st.phase == PH_ADJ_INIT;
+        in.stage = probe ? 0 : st.stage;
+        in.count = probe ? 1 : min(7 - st.stage, max_evals - evals);
+        in.cz = st.cz;
+        in.dt = st.cdt;
+        // another precision's transforms, or none, ran before: their buffers
+        // overlap, so the first exchange waits for the group
+        in.pre = last != (int)adj;
+        last = adj;
+        double acc;
         if (adj) {
             const SubSeg sb = sub_segment(d, st);
-            rhs_adj_call<RF, RA, LOGN, LOGE>(&d, smraw, red, ze, va, sb.lo, sb.hi, zload,
-                                             nullptr, tm);
+            in.seg_lo = sb.lo;
+            in.seg_hi = sb.hi;
+            acc = rhs_adj_call<RF, RA, LOGN, CL>(&d, smraw, rank, &in, tm);
         } else {
-            rhs_fwd_call<RF, LOGN, LOGE>(&d, smraw, red, ze, vf, tm);
+            acc = rhs_fwd_call<RF, RA, LOGN, CL>(&d, smraw, rank, &in, tm);
         }
-        evals++;
+        evals += in.count;
 
         // ------------------------------------------------ consume the derivative
         if (st.phase == PH_FWD_INIT || st.phase == PH_ADJ_INIT) {
             const bool fw = st.phase == PH_FWD_INIT;
             if (st.stage == 0) {
                 double d1;
-                const double r = fw ? init_after_f0<RF, LOGN, LOGE>(d.u0, (CF*)d.kf[0], vf,
-                                                                    d.abstol, d.reltol, L, dtmin,
-                                                                    red, d1)
-                                    : init_after_f0<RA, LOGN, LOGE>(d.lam[0], (CA*)d.ka[0], va,
-                                                                    st.abstol_adj, d.reltol, L,
-                                                                    dtmin, red, d1);
+                const double r =
+                    fw ? init_after_f0<RF>(SF, d.u0, true, (const CF*)d.kf[0], d.abstol, d.reltol, L,
+                                           dtmin, sum, d1)
+                       : init_after_f0<RA>(SF, d.lam[0], false, (const CA*)d.ka[0], st.abstol_adj,
+                                           d.reltol, L, dtmin, sum, d1);
                 if (r > 0.0) {  // probe step
                     st.cdt = r;
                     st.cz = d1;
@@ -1241,12 +1610,12 @@ __global__ void __launch_bounds__(FftShape<LOGN, LOGE>::T, 1)
                 }
                 st.cdt = -r;
             } else {
-                st.cdt = fw ? init_after_f1<RF, LOGN, LOGE>(d.u0, (const CF*)d.kf[0], vf,
-                                                            d.abstol, d.reltol, st.cdt, st.cz, L,
-                                                            dtmin, red)
-                            : init_after_f1<RA, LOGN, LOGE>(d.lam[0], (const CA*)d.ka[0], va,
-                                                            st.abstol_adj, d.reltol, st.cdt,
-                                                            st.cz, L, dtmin, red);
+                st.cdt =
+                    fw ? init_after_f1<RF>(SF, d.u0, true, (const CF*)d.kf[0], (const CF*)d.kf[1],
+                                           d.abstol, d.reltol, st.cdt, st.cz, L, dtmin, sum)
+                       : init_after_f1<RA>(SF, d.lam[0], false, (const CA*)d.ka[0],
+                                           (const CA*)d.ka[1], st.abstol_adj, d.reltol, st.cdt,
+                                           st.cz, L, dtmin, sum);
             }
             st.stage = 0;
             if (fw) {
@@ -1261,19 +1630,19 @@ __global__ void __launch_bounds__(FftShape<LOGN, LOGE>::T, 1)
                 st.nf = 3;
                 if (d.ck_cap > 0) {
                     const CF* k1 = (const CF*)d.kf[0];
-#pragma unroll
+#pragma unroll 4
                     for (int s = 0; s < E; s++) {
-                        const int b = SolF::bin(s);
+                        const int b = SF.own(s);
                         reinterpret_cast<double2*>(d.ck_u)[b] =
-                            reinterpret_cast<const double2*>(d.u0)[b];
+                            reinterpret_cast<const double2*>(d.u0)[SF.bin(s)];
                         ((CF*)d.ck_k1)[b] = k1[b];
                     }
                 }
                 st.save_idx = 0;
                 while (st.save_idx < d.nsave && d.zsave[st.save_idx] == 0.0) {
                     double* o = d.save_out + (size_t)st.save_idx * 2 * N;
-#pragma unroll
-                    for (int s = 0; s < E; s++) st2(o, SolF::bin(s), ld2(d.u0, SolF::bin(s)));
+#pragma unroll 4
+                    for (int s = 0; s < E; s++) st2(o, SF.bin(s), ld2(d.u0, SF.bin(s)));
                     st.save_idx++;
                 }
                 st.phase = PH_FWD;
@@ -1291,13 +1660,8 @@ __global__ void __launch_bounds__(FftShape<LOGN, LOGE>::T, 1)
 
         if (st.phase == PH_FWD || st.phase == PH_REC) {
             const bool rec = st.phase == PH_REC;
-            CF* ko = SolF::kp(d.kf, st.kperm, st.stage);
-#pragma unroll
-            for (int s = 0; s < E; s++) ko[SolF::bin(s)] = vf[s];
-            if (st.stage < 6) {
-                st.stage++;
-                continue;
-            }
+            st.stage += in.count;
+            if (st.stage < 7) continue;
             st.stage = 0;
             const double z = st.cz, dt = st.cdt;
             const double* u = d.u[st.cur];
@@ -1307,8 +1671,8 @@ __global__ void __launch_bounds__(FftShape<LOGN, LOGE>::T, 1)
                 const SubSeg sb = sub_segment(d, st);
                 const int n = sb.seg_lo + st.rec_pos;
                 if (n >= sb.lo)
-                    store_interp<RF, LOGN, LOGE>(d, u, st.kperm,
-                                                 (CF*)d.seg + (size_t)(n - sb.lo) * 5 * N);
+                    store_interp<RF>(SF, u, st.kperm,
+                                     (CF*)d.seg + (size_t)(n - sb.lo) * 5 * N);
                 st.cur ^= 1;
                 st.kperm ^= 1;
                 st.rec_pos++;
@@ -1316,7 +1680,7 @@ __global__ void __launch_bounds__(FftShape<LOGN, LOGE>::T, 1)
                 if (n + 1 >= sb.hi) st.phase = st.a_nf == 0 ? PH_ADJ_INIT : PH_ADJ;
                 continue;
             }
-            const double EEst = SF.error_norm(vf, dt);
+            const double EEst = sqrt(sum(acc) / (double)N);
             if (!isfinite(EEst)) {
                 st.status = ST_NONFINITE;
                 st.phase = PH_DONE;
@@ -1337,15 +1701,15 @@ __global__ void __launch_bounds__(FftShape<LOGN, LOGE>::T, 1)
                     st.phase = PH_DONE;
                     continue;
                 }
-                if (tid == 0) {
+                if (lead) {
                     d.steplog[2 * st.nsteps] = z;
                     d.steplog[2 * st.nsteps + 1] = dt;
                 }
                 // while the solve fits the interpolant buffer, keep each
                 // step's interpolant now: the adjoint then needs no recompute
                 if (st.nsteps < d.seg_cap)
-                    store_interp<RF, LOGN, LOGE>(d, u, st.kperm,
-                                                 (CF*)d.seg + (size_t)st.nsteps * 5 * N);
+                    store_interp<RF>(SF, u, st.kperm,
+                                     (CF*)d.seg + (size_t)st.nsteps * 5 * N);
             }
             double znew = z + dt;
             if (fabs(znew - L) < 100.0 * kEps * fmax(z, L)) znew = L;  // snap to the tstop
@@ -1356,9 +1720,9 @@ __global__ void __launch_bounds__(FftShape<LOGN, LOGE>::T, 1)
                 const double zs = d.zsave[st.save_idx];
                 const double th = (zs - z) / dt;
                 double* o = d.save_out + (size_t)st.save_idx * 2 * N;
-#pragma unroll
+#pragma unroll 4
                 for (int s = 0; s < E; s++) {
-                    const int b = SolF::bin(s);
+                    const int b = SF.own(s), f = SF.bin(s);
                     double xr = 0.0, xi = 0.0;
                     for (int i = 0; i < 7; i++) {
                         double bi = 0.0, tp = th;
@@ -1372,8 +1736,8 @@ __global__ void __launch_bounds__(FftShape<LOGN, LOGE>::T, 1)
                     }
                     const cx<double> un = ld2(u, b);
                     const cx<double> x = mk(un.re + dt * xr, un.im + dt * xi);
-                    const cx<double> p = phasor<double>(d.Dturns[b], zs);
-                    st2(o, b, mk(x.re * p.re - x.im * p.im, x.re * p.im + x.im * p.re));
+                    const cx<double> p = phasor<double>(d.Dturns[f], zs);
+                    st2(o, f, mk(x.re * p.re - x.im * p.im, x.re * p.im + x.im * p.re));
                 }
                 st.save_idx++;
             }
@@ -1388,9 +1752,9 @@ __global__ void __launch_bounds__(FftShape<LOGN, LOGE>::T, 1)
                 int slotc = st.nsteps / st.ck_stride;
                 if (slotc >= d.ck_cap) {
                     for (int j = 1; j < d.ck_cap / 2; j++) {
-#pragma unroll
+#pragma unroll 4
                         for (int s = 0; s < E; s++) {
-                            const int b = SolF::bin(s);
+                            const int b = SF.own(s);
                             reinterpret_cast<double2*>(d.ck_u)[(size_t)j * N + b] =
                                 reinterpret_cast<double2*>(d.ck_u)[(size_t)2 * j * N + b];
                             ((CF*)d.ck_k1)[(size_t)j * N + b] =
@@ -1409,9 +1773,9 @@ __global__ void __launch_bounds__(FftShape<LOGN, LOGE>::T, 1)
 #endif
                 const double* un = d.u[st.cur];
                 const CF* k1 = SolF::kp(d.kf, st.kperm, 0);
-#pragma unroll
+#pragma unroll 4
                 for (int s = 0; s < E; s++) {
-                    const int b = SolF::bin(s);
+                    const int b = SF.own(s);
                     reinterpret_cast<double2*>(d.ck_u)[(size_t)slotc * N + b] =
                         reinterpret_cast<const double2*>(un)[b];
                     ((CF*)d.ck_k1)[(size_t)slotc * N + b] = k1[b];
@@ -1419,10 +1783,10 @@ __global__ void __launch_bounds__(FftShape<LOGN, LOGE>::T, 1)
             }
             if (st.z == L) {
                 const double* uf = d.u[st.cur];
-#pragma unroll
+#pragma unroll 4
                 for (int s = 0; s < E; s++) {
-                    const int b = SolF::bin(s);
-                    const cx<double> x = ld2(uf, b);
+                    const int b = SF.bin(s);
+                    const cx<double> x = ld2(uf, SF.own(s));
                     const cx<double> p = phasor<double>(d.Dturns[b], L);
                     const cx<double> y = mk(x.re * p.re - x.im * p.im, x.re * p.im + x.im * p.re);
                     for (int si = st.save_idx; si < d.nsave; si++)
@@ -1437,17 +1801,12 @@ __global__ void __launch_bounds__(FftShape<LOGN, LOGE>::T, 1)
 
         // PH_ADJ
         {
-            CA* ko = SolA::kp(d.ka, st.akperm, st.stage);
-#pragma unroll
-            for (int s = 0; s < E; s++) ko[SolF::bin(s)] = va[s];
-            if (st.stage < 6) {
-                st.stage++;
-                continue;
-            }
+            st.stage += in.count;
+            if (st.stage < 7) continue;
             st.stage = 0;
             const double z = st.cz, dt = st.cdt;
             const double zlo = d.steplog[2 * sub_segment(d, st).lo];
-            const double EEst = SA.error_norm(va, dt);
+            const double EEst = sqrt(sum(acc) / (double)N);
             if (!isfinite(EEst)) {
                 st.status = ST_NONFINITE;
                 st.phase = PH_DONE;
@@ -1475,22 +1834,22 @@ __global__ void __launch_bounds__(FftShape<LOGN, LOGE>::T, 1)
             if (st.az == zlo) {
                 if (st.sub > 0) {  // the previous sub-segment of this segment
                     st.sub--;
-                    restore_checkpoint<RF, LOGN, LOGE>(d, st.seg, st);
+                    restore_checkpoint<RF>(SF, st.seg, st);
                     st.phase = PH_REC;
                 } else if (st.seg == 0) {
                     st.phase = PH_FINAL;
                 } else {
                     st.seg--;
                     st.sub = last_sub(d, st, st.seg);
-                    restore_checkpoint<RF, LOGN, LOGE>(d, st.seg, st);
+                    restore_checkpoint<RF>(SF, st.seg, st);
                     st.phase = PH_REC;
                 }
             }
         }
     }
-    __syncthreads();
-    if (tid == 0) states[slot] = st;
-    tm_free<LOGN, LOGE>(tm);
+    SolF::XF::sync();  // no CTA leaves while another still writes into it
+    if (lead) states[slot] = st;
+    tm_free<LOGN, CL>(tm);
 }
 
 }  // namespace fl

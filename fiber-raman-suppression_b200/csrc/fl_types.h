@@ -75,11 +75,11 @@ struct SlotDesc {
     // workspace
     double* u[2];           // FP64 forward states
     double* lam[2];         // FP64 adjoint states
-    void* kf[7];            // forward stages, cx<RF>
-    void* ka[7];            // adjoint stages, cx<RA>
+    void* kf[7];            // forward stages, cx<RF>, equally spaced
+    void* ka[7];            // adjoint stages, cx<RA>, equally spaced
     void* scr[2];           // per-thread scratch fields, cx<double>-sized
     double* esv;            // error partial, N complex doubles
-    double* skv;            // error weights, N doubles
+    double* skv;            // error weights, N doubles (pump-gain solve only)
     double* ck_u;           // ck_cap * N complex doubles
     void* ck_k1;            // ck_cap * N cx<RF>
     double* steplog;        // 2 * step_cap doubles (z_n, dt_n)

@@ -138,6 +138,18 @@ __global__ void shaped_launch_kernel(const double2* __restrict__ u0,
     }
 }
 
+// exp(-2 pi i k / nt), rounded from the FP64 value (the allocation-free entry
+// point forms its table the same way, so both solve with the same twiddles)
+template <typename R>
+__global__ void twiddle_kernel(R* __restrict__ tw, int nt) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= nt) return;
+    double s, c;
+    sincospi(-2.0 * (double)k / (double)nt, &s, &c);
+    tw[2 * k] = (R)c;
+    tw[2 * k + 1] = (R)s;
+}
+
 __global__ void gather_stats_kernel(const SlotState* __restrict__ st, int n,
                                     double* __restrict__ J) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -419,22 +431,21 @@ template <typename R>
 int upload_table_set(fl_problem* pr, const double* hR, const double* ss, int q) {
     fl_ctx* ctx = pr->ctx;
     const int nt = pr->nt;
-    std::vector<R> heff(2 * (size_t)nt), ssv(nt), tw(2 * (size_t)nt);
+    std::vector<R> heff(2 * (size_t)nt), ssv(nt);
     for (int k = 0; k < nt; k++) {
         const double sg = (k & 1) ? -1.0 : 1.0;  // fftshift folded into the response
         heff[2 * k] = (R)(hR[2 * k] * sg);
         heff[2 * k + 1] = (R)(hR[2 * k + 1] * sg);
         ssv[k] = (R)ss[k];
-        const double a = -2.0 * M_PI * (double)k / (double)nt;
-        tw[2 * k] = (R)std::cos(a);
-        tw[2 * k + 1] = (R)std::sin(a);
     }
     CU(cudaMalloc(&pr->d_Heff[q], sizeof(R) * heff.size()));
     CU(cudaMalloc(&pr->d_ss[q], sizeof(R) * ssv.size()));
-    CU(cudaMalloc(&pr->d_tw[q], sizeof(R) * tw.size()));
+    CU(cudaMalloc(&pr->d_tw[q], 2 * sizeof(R) * nt));
     CU(cudaMemcpy(pr->d_Heff[q], heff.data(), sizeof(R) * heff.size(), cudaMemcpyHostToDevice));
     CU(cudaMemcpy(pr->d_ss[q], ssv.data(), sizeof(R) * ssv.size(), cudaMemcpyHostToDevice));
-    CU(cudaMemcpy(pr->d_tw[q], tw.data(), sizeof(R) * tw.size(), cudaMemcpyHostToDevice));
+    twiddle_kernel<R><<<(nt + 255) / 256, 256>>>(static_cast<R*>(pr->d_tw[q]), nt);
+    CU(cudaGetLastError());
+    CU(cudaStreamSynchronize(0));
     return FL_OK;
 }
 

@@ -50,9 +50,9 @@ struct Layout {
         state = take(sizeof(SlotState));
         active = take(sizeof(int));
         dturns = take(8 * (size_t)nt);
-        heff = take(8 * (size_t)nt);
-        ss = take(4 * (size_t)nt);
-        tw = take(8 * (size_t)nt);
+        heff = take(16 * (size_t)nt);
+        ss = take(8 * (size_t)nt);
+        tw = take(16 * (size_t)nt);
         u0b = take(16 * (size_t)nt);
         u1b = take(16 * (size_t)nt);
         for (int i = 0; i < 7; i++) kf[i] = take(8 * (size_t)nt);
@@ -73,12 +73,11 @@ __global__ void noalloc_prepare(SlotDesc desc, unsigned char* base, Layout lay, 
     if (i < nt) {
         reinterpret_cast<double*>(base + lay.dturns)[i] = D[i] / (2.0 * M_PI);
         const double sg = (i & 1) ? -1.0 : 1.0;  // fftshift folded into the response
-        reinterpret_cast<float2*>(base + lay.heff)[i] =
-            make_float2((float)(hR[2 * i] * sg), (float)(hR[2 * i + 1] * sg));
-        reinterpret_cast<float*>(base + lay.ss)[i] = (float)selfsteep[i];
+        reinterpret_cast<double2*>(base + lay.heff)[i] = make_double2(hR[2 * i] * sg, hR[2 * i + 1] * sg);
+        reinterpret_cast<double*>(base + lay.ss)[i] = selfsteep[i];
         double s, c;
         sincospi(-2.0 * (double)i / (double)nt, &s, &c);
-        reinterpret_cast<float2*>(base + lay.tw)[i] = make_float2((float)c, (float)s);
+        reinterpret_cast<double2*>(base + lay.tw)[i] = make_double2(c, s);
     }
     if (i == 0) {
         *reinterpret_cast<SlotDesc*>(base + lay.desc) = desc;
@@ -151,9 +150,9 @@ extern "C" int fl_forward_noalloc(int device, int nt, const double* d_D, double 
 
     SlotDesc d{};
     d.Dturns = reinterpret_cast<const double*>(base + lay.dturns);
-    d.Heff[0] = base + lay.heff;
-    d.ss[0] = base + lay.ss;
-    d.tw[0] = base + lay.tw;
+    d.Heff[1] = base + lay.heff;
+    d.ss[1] = base + lay.ss;
+    d.tw[1] = base + lay.tw;
     d.gamma = gamma;
     d.one_m_fR = one_m_fR;
     d.L = L;

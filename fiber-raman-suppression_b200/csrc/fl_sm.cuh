@@ -23,13 +23,14 @@
 // complex conjugates of each other and combine into the single real
 // correlation of Y; h∗I and h̃⋆Y share one complex transform pair.
 //
-// Precision: the forward solve and its recompute run in RF (FP32 in the
-// default mode) with FP64 phase arguments, FP64 state accumulation and an FP64
-// error norm; the dense interpolant is stored in RF.  The adjoint integration
-// (the gradient accumulation along z) runs in RA = FP64: an FP32 adjoint
-// amplifies its round-off through the modulation-instability gain of the
-// anomalous-dispersion fiber and misses 1e-3 gradient accuracy (measured
-// 2e-3..7e-3 on the Nt = 2^13 band-objective problem; 4e-6 in FP64).
+// Precision (FP32 mode, RF = float): states, phase arguments, transforms,
+// stage sums, error norm and reductions in FP64; the forward's stage vectors
+// and the dense interpolant are stored in RF (see SmSolver).  The adjoint
+// integration (the gradient accumulation along z) is FP64 throughout, stage
+// vectors included: an FP32 adjoint amplifies its round-off through the
+// modulation-instability gain of the anomalous-dispersion fiber and misses
+// 1e-3 gradient accuracy (measured 2e-3..7e-3 on the Nt = 2^13 band-objective
+// problem).  The FP64 mode stores everything in FP64.
 #pragma once
 #include <type_traits>
 
@@ -200,35 +201,29 @@ __device__ __forceinline__ double block_max(double v, double* red) {
 }
 
 // Shared-memory layout of the stepper: [transform buffers][64 reduction
-// doubles][FP32 tables][FP64 tables][tensor-memory slot].
+// doubles][transform tables][tensor-memory slot].
 template <typename RMAX, int LOGN, int C>
 struct SmShared {
     static constexpr size_t RED = XPlan<RMAX, RMAX, LOGN, C>::BYTES;
-    static constexpr size_t TAB32 = RED + 64 * sizeof(double);
-    static constexpr size_t TAB64 =
-        (TAB32 + sizeof(cx<float>) * XTables<float, LOGN, C>::SIZE + 15) & ~size_t(15);
-    static constexpr size_t SLOT = TAB64 + sizeof(cx<double>) * XTables<double, LOGN, C>::SIZE;
+    static constexpr size_t TAB = RED + 64 * sizeof(double);
+    static constexpr size_t SLOT =
+        (TAB + sizeof(cx<RMAX>) * XTables<RMAX, LOGN, C>::SIZE + 15) & ~size_t(15);
     // a cluster's CTAs hold tensor memory until their siblings finish: at
     // most one such CTA fits an SM, so that no two clusters wait for each
     // other's columns
     static constexpr size_t BYTES = C > 1 && SLOT + 16 < 116 * 1024 ? 116 * 1024 : SLOT + 16;
     static_assert(BYTES <= 227 * 1024, "shared memory of one CTA");
 };
-template <typename R, typename RMAX, int LOGN, int C>
+template <typename R, int LOGN, int C>
 __device__ __forceinline__ cx<R>* smem_tables(unsigned char* smraw) {
-    using M = SmShared<RMAX, LOGN, C>;
-    return reinterpret_cast<cx<R>*>(smraw + (sizeof(R) == 8 ? M::TAB64 : M::TAB32));
+    return reinterpret_cast<cx<R>*>(smraw + SmShared<R, LOGN, C>::TAB);
 }
 
-// Fill both precisions' tables (the FP64 table is absent when no adjoint
-// will run) and wait for the group.
-template <typename RMAX, int LOGN, int C>
+// Fill the transform tables and wait for the group.
+template <typename R, int LOGN, int C>
 __device__ __forceinline__ void load_tables(const SlotDesc& d, unsigned char* smraw, int rank) {
-    x_fill<float, LOGN, C>(smem_tables<float, RMAX, LOGN, C>(smraw), (const cx<float>*)d.tw[0], rank);
-    if (d.tw[1])
-        x_fill<double, LOGN, C>(smem_tables<double, RMAX, LOGN, C>(smraw), (const cx<double>*)d.tw[1],
-                                rank);
-    XForm<float, RMAX, LOGN, C>::sync();
+    x_fill<R, LOGN, C>(smem_tables<R, LOGN, C>(smraw), (const cx<R>*)d.tw[sizeof(R) == 8], rank);
+    XForm<R, R, LOGN, C>::sync();
 }
 
 // ---------------------------------------------------------------------------
@@ -446,7 +441,6 @@ struct StageRun {
     // adjoint: the stored steps [seg_lo, seg_hi) of the forward, or a field
     int seg_lo, seg_hi;
     const double* ufwd;
-    int pre;             // the first exchange waits for the group
 };
 
 // Pieces of one problem's solve in RHS precision R over a group of C CTAs.
@@ -462,17 +456,27 @@ struct StageRun {
 // through the scratch slots (tensor memory).  Unrolling those as well made
 // the forward evaluation 147 KB of code instead of 44 KB and every part of
 // it slower (Nt = 2^10: radix-16 pass with twiddles 711 against 474 cycles).
-template <typename R, typename RMAX, int LOGN, int CL>
+//
+// Arithmetic runs in R, the stage vectors are stored in K.  The FP32 mode
+// stores its forward stages and interpolants in FP32 but transforms in FP64:
+// of the forward solve's error against FP64 nearly all comes from the two
+// transforms of the field itself (rounding each to FP32 costs 0.5e-6 ..
+// 2.5e-6 at the fiber's end, amplified by the modulation-instability gain;
+// every other rounding 0.2e-6 together), and on an FP64 pipe at half the FP32
+// rate the solves stay latency-bound: error 2e-7 instead of 1e-6 .. 2e-6.
+template <typename R, typename K, int LOGN, int CL>
 struct SmSolver {
-    using XF = XForm<R, RMAX, LOGN, CL>;
+    using XF = XForm<R, R, LOGN, CL>;
     static constexpr int N = XF::N, E = XF::E;
     static constexpr int P = sizeof(R) == 8 ? 1 : 0;  // table precision index
     using C = cx<R>;
+    using CK = cx<K>;
     using TM = TmLayout<LOGN, CL>;
     using TMS = TmScratch<R, LOGN, CL>;
     static constexpr int VPC = TMS::VPC, CH = TMS::CH;
-    static constexpr bool PHC = TM::template phasors<R>();  // phasors kept in tensor memory
-    static constexpr int PHF = sizeof(R) == 8 ? 2 : 1;       // ... in this slot
+    static constexpr bool REGS = E == 2;  // slots in registers (2^6)
+    static constexpr bool PHC = REGS || TM::template phasors<R>();  // phasors kept in a slot
+    static constexpr int PHF = sizeof(R) == 8 || REGS ? 2 : 1;       // ... this one
 
     const SlotDesc& d;
     XF xf;
@@ -482,9 +486,10 @@ struct SmSolver {
     C* scr0;
     C* scr1;
     uint32_t tm;  // tensor-memory scratch of the CTA, or kNoTmem: scr0 / scr1 in global memory
+    mutable C slot_[REGS ? 3 : 1][E];
 
     __device__ SmSolver(const SlotDesc& dd, unsigned char* smem, int rank, uint32_t tmaddr = kNoTmem)
-        : d(dd), xf(smem, smem_tables<R, RMAX, LOGN, CL>(smem), rank),
+        : d(dd), xf(smem, smem_tables<R, LOGN, CL>(smem), rank),
           Heff((const C*)dd.Heff[P]), ss((const R*)dd.ss[P]), Dturns(dd.Dturns),
           scr0((C*)dd.scr[0]), scr1((C*)dd.scr[1]), tm(tmaddr) {}
 
@@ -494,7 +499,10 @@ struct SmSolver {
 
     // ---- scratch slots: chunk c (values c VPC ..) of slot f ----
     __device__ __forceinline__ void put(int f, int c, const C (&v)[VPC]) const {
-        if (tmem()) {
+        if constexpr (REGS) {
+#pragma unroll
+            for (int j = 0; j < VPC; j++) slot_[f][j] = v[j];
+        } else if (tmem()) {
             TMS(tm).put_chunk(f, c, v);
         } else {
             C* s = f ? scr1 : scr0;
@@ -503,7 +511,10 @@ struct SmSolver {
         }
     }
     __device__ __forceinline__ void get(int f, int c, C (&v)[VPC]) const {
-        if (tmem()) {
+        if constexpr (REGS) {
+#pragma unroll
+            for (int j = 0; j < VPC; j++) v[j] = slot_[f][j];
+        } else if (tmem()) {
             TMS(tm).get(f, c, v);
         } else {
             const C* s = f ? scr1 : scr0;
@@ -545,16 +556,14 @@ struct SmSolver {
     //            f2: (I, Y) -F-> X            f3: split X into Î, Ŷ;
     //                Heff Î + i conj(Heff) Ŷ -F⁻¹-> N (h∗I + i h̃⋆Y)
     //            f4: η -F⁻¹->
-    __device__ __forceinline__ void transforms(const bool adj, C (&v)[E], const bool pre) const {
+    __device__ __forceinline__ void transforms(const bool adj, C (&v)[E]) const {
         const R g = (R)d.gamma, ofr = (R)d.one_m_fR, invn = R(1) / R(N);
         const int nfft = adj ? 5 : 4;
 #pragma unroll 1
         for (int f = 0; f < nfft; f++) {
             bool inv = false, to_a = false, presync = false;
             const int op = adj ? 8 + f : f;
-            if (f == 0) {
-                presync = pre;
-            } else if (op == 1) {
+            if (op == 1) {
                 put_all(0, v);
 #pragma unroll
                 for (int s = 0; s < E; s++) v[s] = mk(g * abs2(v[s]), R(0));
@@ -601,7 +610,7 @@ struct SmSolver {
                 // Heff Î + i conj(Heff) Ŷ = Re Heff X[k] + i Im Heff conj(X[-k])
                 xf.mirror_apply(v, Heff);
                 inv = true;
-            } else {  // op == 12
+            } else if (op == 12) {
                 // η = λ_t (2(1-fR) I + h∗I) - (1-fR) γ λ_t* u_t² + 2i (h̃⋆Y) u_t
 #pragma unroll
                 for (int c = 0; c < CH; c++) {
@@ -633,9 +642,9 @@ struct SmSolver {
 
     // ---- stage helpers ---------------------------------------------------
     // logical stage i -> physical buffer; perm swaps stages 0 and 6 (FSAL)
-    __device__ __forceinline__ static C* kp(void* const* k, int perm, int i) {
+    __device__ __forceinline__ static CK* kp(void* const* k, int perm, int i) {
         int p = (perm && (i == 0 || i == 6)) ? 6 - i : i;
-        return (C*)k[p];
+        return (CK*)k[p];
     }
 
     // The input field of stage st, with its phasors, into the slots: stages
@@ -647,11 +656,11 @@ struct SmSolver {
     template <bool ADJ, class Load>
     __device__ __forceinline__ void input(const StageRun& in, const int st, const double z,
                                           const Load& ld) const {
-        const C* k[6];
+        const CK* k[6];
         double a[6];
 #pragma unroll
         for (int j = 0; j < 6; j++) {
-            k[j] = (const C*)in.stage_vec(j);
+            k[j] = (const CK*)in.stage_vec(j);
             a[j] = kT5a[st][j];
         }
         const double dt = in.dt;
@@ -664,7 +673,7 @@ struct SmSolver {
             cx<double> un[VPC];
             typename Load::Raw raw;
             if (st > 0) {
-                C x[6][VPC];
+                CK x[6][VPC];
 #pragma unroll
                 for (int j = 0; j < 6; j++)
                     if (j < st) {
@@ -717,13 +726,13 @@ struct SmSolver {
                     }
                 }
             } else {
-                const C* k1 = (const C*)in.k1;
+                const CK* k1 = (const CK*)in.k1;
 #pragma unroll
                 for (int i = 0; i < VPC; i++) {
                     const int s = s0 + i;
                     Dt[i] = Dturns[bin(s)];
                     if constexpr (ADJ) tau[i] = ss[bin(s)];
-                    const C f0 = k1 ? k1[own(s)] : mk(R(0), R(0));
+                    const CK f0 = k1 ? k1[own(s)] : mk(K(0), K(0));
                     const cx<double> x = in.x ? ld2(in.x, in.xbin ? bin(s) : own(s)) : up(f0);
                     if (in.copy) st2(in.copy, own(s), x);
                     y[i] = k1 && in.x
@@ -755,7 +764,7 @@ struct SmSolver {
     // thread's part of the error norm when the derivative is k7 of an attempt
     template <bool ADJ>
     __device__ __forceinline__ double output(const StageRun& in, const int st, const double z,
-                                             C* out) const {
+                                             CK* out) const {
         const R invn = R(1) / R(N);
 #pragma unroll 1
         for (int c = 0; c < CH; c++) {
@@ -777,21 +786,20 @@ struct SmSolver {
 #pragma unroll
             for (int i = 0; i < VPC; i++) {
                 const C y = cmulc(v[i], ph[i]);  // e^{-iDz} x
-                v[i] = mk(-y.im * sc[i], y.re * sc[i]);
-                out[own(s0 + i)] = v[i];
+                out[own(s0 + i)] = mk((K)(-y.im * sc[i]), (K)(y.re * sc[i]));
             }
         }
         return st == 6 && in.want_err ? error_norm(in, out) : 0.0;
     }
     // the thread's part of the error norm, k7 in k: Σ |dt Σ b̃_j k_j|² / w²,
     // w = abstol + reltol max(|u_n|, |u_{n+1}|)
-    __device__ __forceinline__ double error_norm(const StageRun& in, const C* k) const {
+    __device__ __forceinline__ double error_norm(const StageRun& in, const CK* k) const {
         const double dt = in.dt, bt = kT5bt[6];
         constexpr int NC = E < 4 ? E : 4;
         double acc = 0.0;
 #pragma unroll 1
         for (int s0 = 0; s0 < E; s0 += NC) {
-            C v[NC];
+            CK v[NC];
             cx<double> e6[NC], un[NC], u1[NC];
 #pragma unroll
             for (int i = 0; i < NC; i++) {
@@ -819,7 +827,7 @@ struct SmSolver {
     // one another's latencies and instruction fetches, and the loads in
     // flight per thread decide: at Nt = 2^13 on one CTA the rolled loops
     // above took 27.6 ms per gradient, this form 22.5.
-    static constexpr bool WIDE = XF::TC >= 512 && E >= 16;
+    static constexpr bool WIDE = XF::TC >= 256 && E >= 16;
     static constexpr int SC = E < 8 ? E : 8;
     template <bool ADJ, class Load>
     __device__ __forceinline__ void input_wide(const StageRun& in, const int st, const double z,
@@ -833,9 +841,9 @@ struct SmSolver {
                 for (int c = 0; c < SC; c++) ar[c] = ai[c] = 0.0;
 #pragma unroll 1
                 for (int j = 0; j < st; j++) {
-                    const C* __restrict__ kj = (const C*)in.stage_vec(j);
+                    const CK* __restrict__ kj = (const CK*)in.stage_vec(j);
                     const double a = kT5a[st][j];
-                    C x[SC];
+                    CK x[SC];
 #pragma unroll
                     for (int c = 0; c < SC; c++) x[c] = kj[own(s0 + c)];
 #pragma unroll
@@ -859,9 +867,9 @@ struct SmSolver {
                 for (int c = 0; c < SC7; c++) ar[c] = ai[c] = er[c] = ei[c] = 0.0;
 #pragma unroll 1
                 for (int j = 0; j < 6; j++) {
-                    const C* __restrict__ kj = (const C*)in.stage_vec(j);
+                    const CK* __restrict__ kj = (const CK*)in.stage_vec(j);
                     const double a = kT5a[6][j], bt = kT5bt[j];
-                    C x[SC7];
+                    CK x[SC7];
 #pragma unroll
                     for (int c = 0; c < SC7; c++) x[c] = kj[own(s0 + c)];
 #pragma unroll
@@ -883,10 +891,10 @@ struct SmSolver {
                 }
             }
         } else {
-            const C* k1 = (const C*)in.k1;
+            const CK* k1 = (const CK*)in.k1;
 #pragma unroll 4
             for (int s = 0; s < E; s++) {
-                const C f0 = k1 ? k1[own(s)] : mk(R(0), R(0));
+                const CK f0 = k1 ? k1[own(s)] : mk(K(0), K(0));
                 const cx<double> x = in.x ? ld2(in.x, in.xbin ? bin(s) : own(s)) : up(f0);
                 if (in.copy) st2(in.copy, own(s), x);
                 scr0[own(s)] = k1 && in.x
@@ -936,7 +944,7 @@ struct SmSolver {
     }
     template <bool ADJ>
     __device__ __forceinline__ double output_wide(const StageRun& in, const int st, const double z,
-                                                  C (&v)[E], C* out) const {
+                                                  C (&v)[E], CK* out) const {
         const R invn = R(1) / R(N);
         if constexpr (!PHC) phasors_and_field<false>(z, NoLoad{});
 #pragma unroll
@@ -948,7 +956,7 @@ struct SmSolver {
                 const int s = c * VPC + i;
                 const C y = cmulc(v[s], ph[i]);  // e^{-iDz} x
                 const R sc = ADJ ? invn : ss[bin(s)] * invn;
-                out[own(s)] = mk(-y.im * sc, y.re * sc);
+                out[own(s)] = mk((K)(-y.im * sc), (K)(y.re * sc));
             }
         }
         return st == 6 && in.want_err ? error_norm(in, out) : 0.0;
@@ -967,7 +975,7 @@ struct SmSolver {
         for (int st = in.stage; st < end; st++) {
             const double z = st == 0 ? in.z : in.cz + kT5c[st] * in.dt;
             const auto ld = make_load(*this, st == 0 ? in.zload : z);
-            C* out = (C*)(st == 0 ? (char*)in.out : in.stage_vec(st));
+            CK* out = (CK*)(st == 0 ? (char*)in.out : in.stage_vec(st));
             C v[E];
             if constexpr (WIDE) {
                 input_wide<ADJ>(in, st, z, ld, v);
@@ -975,7 +983,7 @@ struct SmSolver {
                 input<ADJ>(in, st, z, ld);
                 get_all(0, v);
             }
-            transforms(ADJ, v, in.pre && st == in.stage);
+            transforms(ADJ, v);
             if constexpr (WIDE) {
                 acc = output_wide<ADJ>(in, st, z, v, out);
             } else {
@@ -1090,10 +1098,10 @@ struct SegLoader {
 // Out-of-line runs of RHS evaluations: the transform bodies get the full
 // register budget of the CTA instead of sharing it with the state machine's
 // live values.
-template <typename R, typename RMAX, int LOGN, int CL>
+template <typename R, typename K, int LOGN, int CL>
 __device__ __noinline__ double rhs_fwd_call(const SlotDesc* d, unsigned char* sm, int rank,
                                             const StageRun* in, uint32_t tm = kNoTmem) {
-    using Sol = SmSolver<R, RMAX, LOGN, CL>;
+    using Sol = SmSolver<R, K, LOGN, CL>;
     Sol S(*d, sm, rank, tm);
     return S.template run<false>(*in, [](const Sol&, double) { return NoLoad{}; });
 }
@@ -1137,7 +1145,6 @@ __global__ void __launch_bounds__(XShape<LOGN, 1>::T, 1)
     si.x = in;
     si.xbin = 1;
     si.z = si.zload = z;
-    si.pre = 1;
     si.ufwd = ufwd;
     si.out = adjoint ? d->ka[0] : d->kf[0];
     const XF xf(smraw, nullptr, 0);
@@ -1147,7 +1154,7 @@ __global__ void __launch_bounds__(XShape<LOGN, 1>::T, 1)
 #pragma unroll
         for (int s = 0; s < XF::E; s++) st2(out, xf.bin(s), up(k[xf.own(s)]));
     } else {
-        rhs_fwd_call<RF, RA, LOGN, 1>(d, smraw, 0, &si, tm);
+        rhs_fwd_call<RA, RF, LOGN, 1>(d, smraw, 0, &si, tm);
         const cx<RF>* k = (const cx<RF>*)d->kf[0];
 #pragma unroll
         for (int s = 0; s < XF::E; s++) st2(out, xf.bin(s), up(k[xf.own(s)]));
@@ -1337,7 +1344,7 @@ template <typename RF, typename RA, int LOGN, int CL>
 __global__ void __launch_bounds__(XShape<LOGN, CL>::TC, sm_min_ctas(LOGN))
     sm_advance_kernel(const SlotDesc* __restrict__ descs, SlotState* __restrict__ states,
                       const int* __restrict__ active, int max_evals) {
-    using SolF = SmSolver<RF, RA, LOGN, CL>;
+    using SolF = SmSolver<RA, RF, LOGN, CL>;
     using SolA = SmSolver<RA, RA, LOGN, CL>;
     using CF = cx<RF>;
     using CA = cx<RA>;
@@ -1360,7 +1367,6 @@ __global__ void __launch_bounds__(XShape<LOGN, CL>::TC, sm_min_ctas(LOGN))
     // the stage vectors of a slot lie one stride apart (work_create)
     const size_t kfs = (char*)d.kf[1] - (char*)d.kf[0], kas = (char*)d.ka[1] - (char*)d.ka[0];
     int evals = 0;
-    int last = -1;  // precision of the last evaluation (its buffers may still be read)
 
     while (st.phase != PH_DONE && evals < max_evals) {
 #ifdef FL_CHECKED
@@ -1577,10 +1583,6 @@ __global__ void __launch_bounds__(XShape<LOGN, CL>::TC, sm_min_ctas(LOGN))
         in.count = probe ? 1 : min(7 - st.stage, max_evals - evals);
         in.cz = st.cz;
         in.dt = st.cdt;
-        // another precision's transforms, or none, ran before: their buffers
-        // overlap, so the first exchange waits for the group
-        in.pre = last != (int)adj;
-        last = adj;
         double acc;
         if (adj) {
             const SubSeg sb = sub_segment(d, st);
@@ -1588,7 +1590,7 @@ __global__ void __launch_bounds__(XShape<LOGN, CL>::TC, sm_min_ctas(LOGN))
             in.seg_hi = sb.hi;
             acc = rhs_adj_call<RF, RA, LOGN, CL>(&d, smraw, rank, &in, tm);
         } else {
-            acc = rhs_fwd_call<RF, RA, LOGN, CL>(&d, smraw, rank, &in, tm);
+            acc = rhs_fwd_call<RA, RF, LOGN, CL>(&d, smraw, rank, &in, tm);
         }
         evals += in.count;
 

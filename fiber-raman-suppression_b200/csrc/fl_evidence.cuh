@@ -23,6 +23,37 @@
 
 namespace fl {
 
+// One transform group in natural order on both sides (the temporal edges are
+// positions): a CTA (C = 1) or a cluster.
+template <int LOGN, int LOGE, int C>
+struct EvGroup {
+    using CS = ClusterShape<LOGN, LOGE, C>;
+    static constexpr int N = CS::N, E = CS::E, TT = CS::TT, T = CS::T;
+    static constexpr size_t XBYTES =
+        C == 1 ? SmemPlan<double, LOGN>::BYTES : cluster_xbytes<double, LOGN, C>();
+    static constexpr size_t SMEM =
+        XBYTES + sizeof(cx<double>) * Twiddles<double, LOGN>::SIZE + 32 * sizeof(double);
+    int rank, g;
+    unsigned char* sm;
+    double* red;
+    Twiddles<double, LOGN> tw;
+    __device__ __forceinline__ void init(const MmDesc& d, unsigned char* smraw) {
+        rank = C == 1 ? 0 : (int)(blockIdx.x % C);
+        g = rank * T + threadIdx.x;
+        sm = smraw;
+        cx<double>* tws = reinterpret_cast<cx<double>*>(smraw + XBYTES);
+        red = reinterpret_cast<double*>(tws + Twiddles<double, LOGN>::SIZE);
+        Twiddles<double, LOGN>::fill(tws, static_cast<const cx<double>*>(d.tw[1]));
+        if constexpr (C == 1) __syncthreads();
+        else cluster_sync_all();
+        tw = Twiddles<double, LOGN>::at(tws);
+    }
+    __device__ __forceinline__ void fft(cx<double> (&v)[E]) const {
+        if constexpr (C == 1) block_fft<double, LOGN, LOGE>(v, sm, tw);
+        else cluster_fft<double, LOGN, LOGE, C>(v, reinterpret_cast<cx<double>*>(sm), tw, g);
+    }
+};
+
 // sum (or max) over the transform group: the CTA's block reduction, then,
 // for a cluster, the ranks' values in rank order through rank 0's shared
 // memory (xch holds one double per rank)
@@ -46,10 +77,10 @@ __device__ __forceinline__ double group_reduce(double v, bool is_max, double* re
 }
 
 template <int LOGN, int LOGE, int CL>
-__global__ void __launch_bounds__(MmGroup<double, LOGN, LOGE, CL>::T, 1)
+__global__ void __launch_bounds__(EvGroup<LOGN, LOGE, CL>::T, 1)
     evidence_kernel(const MmDesc tab, const double* __restrict__ spectra,
                     const double* __restrict__ ss, int M, double* __restrict__ out) {
-    using G = MmGroup<double, LOGN, LOGE, CL>;
+    using G = EvGroup<LOGN, LOGE, CL>;
     constexpr int N = G::N, E = G::E, TT = G::TT, T = G::T;
     extern __shared__ __align__(16) unsigned char smraw[];
     const int s = blockIdx.x / CL;
@@ -114,7 +145,7 @@ __global__ void __launch_bounds__(MmGroup<double, LOGN, LOGE, CL>::T, 1)
 
 template <int LOGN, int LOGE, int CL>
 cudaError_t launch_evidence(const EvidenceArgs& a) {
-    using G = MmGroup<double, LOGN, LOGE, CL>;
+    using G = EvGroup<LOGN, LOGE, CL>;
     const size_t smem = G::SMEM + 64 * sizeof(double);  // + the cluster exchange slots
     auto k = evidence_kernel<LOGN, LOGE, CL>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

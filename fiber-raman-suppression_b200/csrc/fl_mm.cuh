@@ -90,41 +90,63 @@ __device__ __forceinline__ void stcr(void* p, size_t i, cx<double> v, bool fp64)
     else static_cast<cx<float>*>(p)[i] = down<float>(v);
 }
 
-// One transform group: a CTA (C = 1) or a cluster of C CTAs (see
-// fl_cfft.cuh).  g is the thread's index in the group, TT the group's thread
-// count; a thread owns the positions g + TT*s.
+// One transform group: a CTA (C = 1, the transforms of fl_xfft.cuh) or a
+// cluster of C CTAs (see fl_cfft.cuh).  Value s of a thread is bin(s) of a
+// field in frequency and, after to_time, element own(s) of a field in time:
+// time fields lie in the order the transforms leave them in, which every
+// kernel between two transforms shares (their work is pointwise in time).
+__host__ __device__ constexpr int mm_loge(int logn) { return logn == 12 ? 3 : x_loge(logn); }
 template <typename R, int LOGN, int LOGE, int C>
 struct MmGroup {
-    using CS = ClusterShape<LOGN, LOGE, C>;
-    static constexpr int N = CS::N, E = CS::E, TT = CS::TT, T = CS::T;
+    static constexpr int LE = C == 1 ? mm_loge(LOGN) : LOGE;
+    using XS = XShape<LOGN, 1, LE>;
+    using XF = XForm<R, R, LOGN, 1, LE>;
+    static constexpr int N = 1 << LOGN, E = 1 << LE, TT = N / E, T = TT / C;
     // per-CTA exchange buffer bytes
     static constexpr size_t XBYTES =
-        C == 1 ? SmemPlan<R, LOGN>::BYTES : cluster_xbytes<R, LOGN, C>();
-    static constexpr size_t SMEM =
-        XBYTES + sizeof(cx<R>) * Twiddles<R, LOGN>::SIZE + 32 * sizeof(double);
-    int rank, g;
+        C == 1 ? XPlan<R, R, LOGN, 1, LE>::BYTES : cluster_xbytes<R, LOGN, C>();
+    static constexpr int TABLE =
+        C == 1 ? XTables<R, LOGN, 1, LE>::SIZE : Twiddles<R, LOGN>::SIZE;
+    static constexpr size_t SMEM = XBYTES + sizeof(cx<R>) * TABLE + 32 * sizeof(double) + 16;
+    int rank, g, flip;
     unsigned char* sm;
     double* red;
-    Twiddles<R, LOGN> tw;
+    cx<R>* tab;
 
-    __device__ __forceinline__ void sync() const {
-        if constexpr (C == 1) __syncthreads();
-        else cluster_sync_all();
-    }
     // every CTA of the group calls it (uniform early exits only before it)
     __device__ __forceinline__ void init(const MmDesc& d, unsigned char* smraw) {
         rank = C == 1 ? 0 : (int)(blockIdx.x % C);
         g = rank * T + threadIdx.x;
+        flip = 0;
         sm = smraw;
-        cx<R>* tws = reinterpret_cast<cx<R>*>(smraw + XBYTES);
-        red = reinterpret_cast<double*>(tws + Twiddles<R, LOGN>::SIZE);
-        Twiddles<R, LOGN>::fill(tws, static_cast<const cx<R>*>(d.tw[sizeof(R) == 8]));
-        sync();
-        tw = Twiddles<R, LOGN>::at(tws);
+        tab = reinterpret_cast<cx<R>*>(smraw + XBYTES);
+        red = reinterpret_cast<double*>(smraw + ((XBYTES + sizeof(cx<R>) * TABLE + 15) & ~size_t(15)));
+        const cx<R>* full = static_cast<const cx<R>*>(d.tw[sizeof(R) == 8]);
+        if constexpr (C == 1) {
+            x_fill<R, LOGN, 1, LE>(tab, full, 0);
+            __syncthreads();
+        } else {
+            Twiddles<R, LOGN>::fill(tab, full);
+            cluster_sync_all();
+        }
     }
-    __device__ __forceinline__ void fft(cx<R> (&v)[E]) const {
-        if constexpr (C == 1) block_fft<R, LOGN, LOGE>(v, sm, tw);
-        else cluster_fft<R, LOGN, LOGE, C>(v, reinterpret_cast<cx<R>*>(sm), tw, g);
+    __device__ __forceinline__ int own(int s) const { return g + TT * s; }
+    __device__ __forceinline__ int bin(int s) const {
+        if constexpr (C == 1 && LE >= 4) return x_col<LOGN, 1>(g, s >> 4) + (N / 16) * (s & 15);
+        else return g + TT * s;
+    }
+    // unnormalised transforms, exponent sign -1, between frequency and time
+    __device__ __forceinline__ void to_time(cx<R> (&v)[E]) { run(v, false); }
+    __device__ __forceinline__ void to_freq(cx<R> (&v)[E]) { run(v, true); }
+    __device__ __forceinline__ void run(cx<R> (&v)[E], bool to_a) {
+        if constexpr (C == 1) {
+            XF xf(sm, tab, 0);
+            xf.flip = flip;
+            xf.transform(v, to_a, true);
+            flip = xf.flip;
+        } else {
+            cluster_fft<R, LOGN, LOGE, C>(v, reinterpret_cast<cx<R>*>(sm), Twiddles<R, LOGN>::at(tab), g);
+        }
     }
 };
 
@@ -136,7 +158,7 @@ __global__ void __launch_bounds__(MmGroup<R, LOGN, LOGE, CL>::T, 1)
     mm_prologue_kernel(const MmDesc* __restrict__ descs, const MmState* __restrict__ states,
                        const int* __restrict__ active) {
     using G = MmGroup<R, LOGN, LOGE, CL>;
-    constexpr int N = G::N, E = G::E, T = G::T, TT = G::TT;
+    constexpr int N = G::N, E = G::E;
     constexpr int P = sizeof(R) == 8;
     using C = cx<R>;
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -152,7 +174,6 @@ __global__ void __launch_bounds__(MmGroup<R, LOGN, LOGE, CL>::T, 1)
     if (!mm_takes<R>(d, st) && !fwd_field) return;
     G grp;
     grp.init(d, smraw);
-    const int tid = grp.g;  // index in the transform group
     const size_t NM = (size_t)N * d.M, off = (size_t)m * N;
     const int ph = st.phase;
     const bool adj = mm_adjoint_phase(ph);
@@ -163,7 +184,7 @@ __global__ void __launch_bounds__(MmGroup<R, LOGN, LOGE, CL>::T, 1)
         // ---- stage input (FP64 accumulation, as the single-mode stepper)
         if (ph == PH_EVAL_FWD || ph == PH_EVAL_ADJ) {
 #pragma unroll
-            for (int s = 0; s < E; s++) v[s] = down<R>(ld2(d.u0, off + tid + TT * s));
+            for (int s = 0; s < E; s++) v[s] = down<R>(ld2(d.u0, off + grp.bin(s)));
         } else if (ph == PH_FWD_INIT || ph == PH_ADJ_INIT) {
             const bool fw = ph == PH_FWD_INIT;
             const double* x0 = fw ? d.u0 : d.lam[0];
@@ -171,7 +192,7 @@ __global__ void __launch_bounds__(MmGroup<R, LOGN, LOGE, CL>::T, 1)
             const double sg = fw ? st.cdt : -st.cdt;
 #pragma unroll
             for (int s = 0; s < E; s++) {
-                const size_t b = off + tid + TT * s;
+                const size_t b = off + grp.bin(s);
                 const cx<double> x = ld2(x0, b);
                 if (st.stage == 0) {
                     v[s] = down<R>(x);
@@ -205,7 +226,7 @@ __global__ void __launch_bounds__(MmGroup<R, LOGN, LOGE, CL>::T, 1)
                         const double a = kT5a[st.stage][j];
                         C xk[SC];
 #pragma unroll
-                        for (int c = 0; c < SC; c++) xk[c] = kj[off + tid + TT * (s0 + c)];
+                        for (int c = 0; c < SC; c++) xk[c] = kj[off + grp.bin(s0 + c)];
 #pragma unroll
                         for (int c = 0; c < SC; c++) {
                             ar[c] += a * (double)xk[c].re;
@@ -214,12 +235,12 @@ __global__ void __launch_bounds__(MmGroup<R, LOGN, LOGE, CL>::T, 1)
                         if (ckp && j == 0) {
 #pragma unroll
                             for (int c = 0; c < SC; c++)
-                                static_cast<C*>(d.ck_k1)[(size_t)(ckp - 1) * NM + off + tid + TT * (s0 + c)] = xk[c];
+                                static_cast<C*>(d.ck_k1)[(size_t)(ckp - 1) * NM + off + grp.bin(s0 + c)] = xk[c];
                         }
                     }
 #pragma unroll
                     for (int c = 0; c < SC; c++) {
-                        const size_t b = off + tid + TT * (s0 + c);
+                        const size_t b = off + grp.bin(s0 + c);
                         const cx<double> un = ld2(x, b);
                         if (ckp) st2(d.ck_u, (size_t)(ckp - 1) * NM + b, un);
                         v[s0 + c] = mk((R)(un.re + dt * ar[c]), (R)(un.im + dt * ai[c]));
@@ -243,7 +264,7 @@ __global__ void __launch_bounds__(MmGroup<R, LOGN, LOGE, CL>::T, 1)
                         const double a = kT5a[6][j], bt = kT5bt[j];
                         C xk[SC6];
 #pragma unroll
-                        for (int c = 0; c < SC6; c++) xk[c] = kj[off + tid + TT * (s0 + c)];
+                        for (int c = 0; c < SC6; c++) xk[c] = kj[off + grp.bin(s0 + c)];
 #pragma unroll
                         for (int c = 0; c < SC6; c++) {
                             ar[c] += a * (double)xk[c].re;
@@ -254,7 +275,7 @@ __global__ void __launch_bounds__(MmGroup<R, LOGN, LOGE, CL>::T, 1)
                     }
 #pragma unroll
                     for (int c = 0; c < SC6; c++) {
-                        const size_t b = off + tid + TT * (s0 + c);
+                        const size_t b = off + grp.bin(s0 + c);
                         const cx<double> un = ld2(x, b);
                         const cx<double> u1 = mk(un.re + dt * ar[c], un.im + dt * ai[c]);
                         st2(xnew, b, u1);
@@ -275,20 +296,20 @@ __global__ void __launch_bounds__(MmGroup<R, LOGN, LOGE, CL>::T, 1)
         C* out = static_cast<C*>(adj ? d.lt : d.ut);
 #pragma unroll
         for (int s = 0; s < E; s++) {
-            const int t = tid + TT * s;
+            const int t = grp.bin(s);
             v[s] = cmul(v[s], phasor<R>(Dt[t], st.ez));
             if (adj) v[s] = scale(v[s], ss[t]);
         }
-        grp.fft(v);
+        grp.to_time(v);
 #pragma unroll
-        for (int s = 0; s < E; s++) out[off + tid + TT * s] = v[s];
+        for (int s = 0; s < E; s++) out[off + grp.own(s)] = v[s];
         if (!adj || d.adj_mixed) return;  // (mixed: the FP32 kernel takes the forward field)
     }
 
     // ---- adjoint: the forward field at ezload, F(e^{iDz} ũ(z))
     if (ph == PH_EVAL_ADJ) {
 #pragma unroll
-        for (int s = 0; s < E; s++) v[s] = down<R>(ld2(d.lamL, off + tid + TT * s));
+        for (int s = 0; s < E; s++) v[s] = down<R>(ld2(d.lamL, off + grp.bin(s)));
     } else {
         const SubSeg sb = sub_segment(d, st);
         const int seg_lo = sb.lo;
@@ -306,7 +327,7 @@ __global__ void __launch_bounds__(MmGroup<R, LOGN, LOGE, CL>::T, 1)
         const size_t base = (size_t)(n - seg_lo) * 5 * NM;
 #pragma unroll
         for (int s = 0; s < E; s++) {
-            const size_t b = off + tid + TT * s;
+            const size_t b = off + grp.bin(s);
             cx<double> c[5];
 #pragma unroll
             for (int q = 0; q < 5; q++) c[q] = ldcr(d.seg, base + q * NM + b, d.fp64);
@@ -315,13 +336,12 @@ __global__ void __launch_bounds__(MmGroup<R, LOGN, LOGE, CL>::T, 1)
             v[s] = mk((R)xr, (R)xi);
         }
     }
-    grp.sync();  // the exchange buffer is reused
 #pragma unroll
-    for (int s = 0; s < E; s++) v[s] = cmul(v[s], phasor<R>(Dt[tid + TT * s], st.ez));
-    grp.fft(v);
+    for (int s = 0; s < E; s++) v[s] = cmul(v[s], phasor<R>(Dt[grp.bin(s)], st.ez));
+    grp.to_time(v);
     C* uo = static_cast<C*>(d.ut);
 #pragma unroll
-    for (int s = 0; s < E; s++) uo[off + tid + TT * s] = v[s];
+    for (int s = 0; s < E; s++) uo[off + grp.own(s)] = v[s];
 }
 
 // ---------------------------------------------------------------------------
@@ -338,7 +358,7 @@ __global__ void __launch_bounds__(MmGroup<R, LOGN, LOGE, CL>::T, 1)
     mm_pairs_kernel(const MmDesc* __restrict__ descs, const MmState* __restrict__ states,
                     const int* __restrict__ active) {
     using G = MmGroup<R, LOGN, LOGE, CL>;
-    constexpr int N = G::N, E = G::E, T = G::T, TT = G::TT;
+    constexpr int N = G::N, E = G::E;
     constexpr int P = sizeof(R) == 8;
     using C = cx<R>;
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -366,7 +386,6 @@ __global__ void __launch_bounds__(MmGroup<R, LOGN, LOGE, CL>::T, 1)
     const bool two = q1 < nseq;
     G grp;
     grp.init(d, smraw);
-    const int tid = grp.g;  // index in the transform group
     const C* ut = static_cast<const C*>(d.ut);
     const C* H = static_cast<const C*>(d.Heff[P]);
     R* sq = static_cast<R*>(d.sq);
@@ -379,7 +398,7 @@ __global__ void __launch_bounds__(MmGroup<R, LOGN, LOGE, CL>::T, 1)
     R p0[E], p1[E];
 #pragma unroll
     for (int s = 0; s < E; s++) {
-        const int t = tid + TT * s;
+        const int t = grp.own(s);
         if (ytask) {
             p0[s] = cq[(size_t)q0 * N + t];
             p1[s] = two ? cq[(size_t)q1 * N + t] : R(0);
@@ -399,20 +418,20 @@ __global__ void __launch_bounds__(MmGroup<R, LOGN, LOGE, CL>::T, 1)
         }
         v[s] = mk(p0[s], p1[s]);
     }
-    grp.fft(v);
+    grp.to_freq(v);
 #pragma unroll
     for (int s = 0; s < E; s++) {
-        const C h = H[tid + TT * s];
+        const C h = H[grp.bin(s)];
         v[s] = ytask ? cmulc(v[s], h) : cmul(v[s], h);  // conj(Heff): correlation
     }
     conj_all(v);
-    grp.fft(v);
+    grp.to_time(v);
     conj_all(v);
     // forward S = (1-fR) P + h∗P; adjoint S' = 2(1-fR) P + h∗P and C = h̃⋆Im X
     const R kf = adj ? R(2) * ofr : ofr;
 #pragma unroll
     for (int s = 0; s < E; s++) {
-        const int t = tid + TT * s;
+        const int t = grp.own(s);
         if (ytask) {
             cq[(size_t)q0 * N + t] = v[s].re * invn;
             if (two) cq[(size_t)q1 * N + t] = v[s].im * invn;
@@ -432,7 +451,7 @@ __global__ void __launch_bounds__(MmGroup<R, LOGN, LOGE, CL>::T, 1)
     mm_epilogue_kernel(const MmDesc* __restrict__ descs, const MmState* __restrict__ states,
                        const int* __restrict__ active) {
     using G = MmGroup<R, LOGN, LOGE, CL>;
-    constexpr int N = G::N, E = G::E, T = G::T, TT = G::TT;
+    constexpr int N = G::N, E = G::E, T = G::T;
     constexpr int P = sizeof(R) == 8;
     using C = cx<R>;
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -444,28 +463,27 @@ __global__ void __launch_bounds__(MmGroup<R, LOGN, LOGE, CL>::T, 1)
     if (!mm_takes<R>(d, st)) return;
     G grp;
     grp.init(d, smraw);
-    const int tid = grp.g;  // index in the transform group
     const size_t off = (size_t)m * N;
     const int ph = st.phase;
     const bool adj = mm_adjoint_phase(ph);
     const C* eta = static_cast<const C*>(d.eta);
     C v[E];
 #pragma unroll
-    for (int s = 0; s < E; s++) v[s] = conjc(eta[off + tid + TT * s]);
-    grp.fft(v);
+    for (int s = 0; s < E; s++) v[s] = conjc(eta[off + grp.own(s)]);
+    grp.to_freq(v);
     const double* Dt = d.Dturns + off;
     const R* ss = static_cast<const R*>(d.ss[P]);
     const R invn = R(1) / R(N);
 #pragma unroll
     for (int s = 0; s < E; s++) {
-        const int t = tid + TT * s;
+        const int t = grp.bin(s);
         const C y = cmulc(conjc(v[s]), phasor<R>(Dt[t], st.ez));  // e^{-iDz} x
         const R sc = adj ? invn : ss[t] * invn;
         v[s] = mk(-y.im * sc, y.re * sc);  // i y (τ) / N
     }
     if (ph == PH_EVAL_FWD || ph == PH_EVAL_ADJ) {
 #pragma unroll
-        for (int s = 0; s < E; s++) st2(d.lam0_out, off + tid + TT * s, up(v[s]));
+        for (int s = 0; s < E; s++) st2(d.lam0_out, off + grp.bin(s), up(v[s]));
         return;
     }
     C* dst;
@@ -474,7 +492,7 @@ __global__ void __launch_bounds__(MmGroup<R, LOGN, LOGE, CL>::T, 1)
     else if (adj) dst = static_cast<C*>(mm_kp(d.ka, st.akperm, st.stage));
     else dst = static_cast<C*>(mm_kp(d.kf, st.kperm, st.stage));
 #pragma unroll
-    for (int s = 0; s < E; s++) dst[off + tid + TT * s] = v[s];
+    for (int s = 0; s < E; s++) dst[off + grp.bin(s)] = v[s];
     // dense interpolant of this mode's part of the step: c0 = ũ_n,
     // c_p = Σ_i r_ip k_i (Tsit5's free 4th-order interpolant).  A replayed
     // step keeps it for the steps of the current sub-segment; a forward
@@ -504,7 +522,7 @@ __global__ void __launch_bounds__(MmGroup<R, LOGN, LOGE, CL>::T, 1)
 #pragma unroll
                 for (int c = 0; c < 2; c++)
                     ki[c] = i == 6 ? v[s0 + c]
-                                   : static_cast<const C*>(mm_kp(d.kf, st.kperm, i))[off + tid + TT * (s0 + c)];
+                                   : static_cast<const C*>(mm_kp(d.kf, st.kperm, i))[off + grp.bin(s0 + c)];
 #pragma unroll
                 for (int c = 0; c < 2; c++)
 #pragma unroll
@@ -515,7 +533,7 @@ __global__ void __launch_bounds__(MmGroup<R, LOGN, LOGE, CL>::T, 1)
             }
 #pragma unroll
             for (int c = 0; c < 2; c++) {
-                const size_t b = off + tid + TT * (s0 + c);
+                const size_t b = off + grp.bin(s0 + c);
                 sg[base + b] = down<R>(ld2(un, b));
 #pragma unroll
                 for (int q = 0; q < 4; q++) sg[base + (q + 1) * NM + b] = mk((R)cr[c][q], (R)ci[c][q]);
@@ -527,7 +545,7 @@ __global__ void __launch_bounds__(MmGroup<R, LOGN, LOGE, CL>::T, 1)
         double acc = 0.0;
 #pragma unroll
         for (int s = 0; s < E; s++) {
-            const size_t b = off + tid + TT * s;
+            const size_t b = off + grp.bin(s);
             const cx<double> e6 = ld2(d.esv, b);
             const double er = e6.re + dt * bt7 * (double)v[s].re;
             const double ei = e6.im + dt * bt7 * (double)v[s].im;

@@ -1,3 +1,3 @@
 // Multimode evaluation round instance: Nt = 2^9, 16 elements per thread.
 #include "fl_mm_inst.cuh"
-FL_MM_INSTANCE(9, 2, 1)
+FL_MM_INSTANCE(9, 4, 1)

@@ -174,13 +174,13 @@ __device__ __forceinline__ cx<double> x_shfl(cx<double> v, int src) {
 // ---------------------------------------------------------------------------
 // Geometry of a group of C CTAs for one problem of 2^LOGN points.
 // ---------------------------------------------------------------------------
-template <int LOGN, int C>
+template <int LOGN, int C, int LE = x_loge(LOGN)>
 struct XShape {
-    static constexpr int LOGE = x_loge(LOGN);
+    static constexpr int LOGE = LE;
     static constexpr int N = 1 << LOGN, E = 1 << LOGE;
     static constexpr int T = N / E;      // threads of the group
     static constexpr int TC = T / C;     // threads per CTA
-    static constexpr bool SMALL = LOGN <= 11;  // E <= 8: Stockham
+    static constexpr bool SMALL = LE <= 3;  // E <= 8: Stockham
     static constexpr int TT = N / 16;    // columns; points of a region
     static constexpr int L = E == 32 ? 32 : TT / 16;  // lanes per region
     // region stride in elements: room for the warp-local transposition
@@ -196,9 +196,9 @@ struct XShape {
 // the same bytes.  One CTA: one FP64 buffer (two would halve the CTAs per SM
 // or not fit), two FP32 ones where they fit in it; clusters: two of each.
 // FP64 at 2^14 points on one CTA exchanges real and imaginary parts in turn.
-template <typename R, typename RMAX, int LOGN, int C>
+template <typename R, typename RMAX, int LOGN, int C, int LE = x_loge(LOGN)>
 struct XPlan {
-    using S = XShape<LOGN, C>;
+    using S = XShape<LOGN, C, LE>;
     static constexpr bool SPLIT = C == 1 && 2 * sizeof(R) * (size_t)S::BUF > 200 * 1024;
     static constexpr size_t ONE = (SPLIT ? sizeof(R) : 2 * sizeof(R)) * (size_t)S::BUF;
     static constexpr bool SPLITM = C == 1 && 2 * sizeof(RMAX) * (size_t)S::BUF > 200 * 1024;
@@ -209,18 +209,17 @@ struct XPlan {
 };
 
 // Twiddle tables in shared memory, filled once per kernel from the full
-// table W_N^k: first-pass columns (FP32: every W_N^{xq}, correctly rounded,
-// up to 2^13; two-level products at 2^14; FP64: W_N^x, powers by products),
-// second pass (FP32: W_{N/16}^{lr}; FP64: W_{N/16}^l), W_32^i.
-template <typename R, int LOGN, int C>
+// table W_N^k.  E >= 16: first-pass columns (FP32: two-level products
+// W^e = hi[e >> 6] lo[e & 63]; FP64: W_N^x, powers by products), second pass
+// (FP32: W_{N/16}^{lr}; FP64: W_{N/16}^l), W_32^i.
+template <typename R, int LOGN, int C, int LE = x_loge(LOGN)>
 struct XTables {
-    using S = XShape<LOGN, C>;
+    using S = XShape<LOGN, C, LE>;
     static constexpr bool F32 = sizeof(R) == 4;
-    static constexpr bool TWO_LEVEL = F32 && S::E == 32;
+    static constexpr bool TWO_LEVEL = F32 && S::E >= 16;
     static constexpr int R2 = S::E == 32 ? 32 : 16;
     static constexpr int N1 = S::SMALL ? 0
-                              : F32 ? (TWO_LEVEL ? 64 + S::N / 64 : 15 * S::TC)
-                                    : S::TC * (S::E / 16);
+                              : F32 ? 64 + S::N / 64 : S::TC * (S::E / 16);
     static constexpr int N2 = S::SMALL ? 0 : (F32 ? R2 * S::L : S::L);
     static constexpr int N3 = !S::SMALL && S::L == 32 && S::E == 16 ? 16 : 0;
     // E <= 8: W_{E ns}^{m r}, m < ns, of each radix-E pass (ns = its stride)
@@ -262,10 +261,10 @@ __device__ __forceinline__ int x_owner(int x, int& half) {
     }
 }
 
-template <typename R, int LOGN, int C>
+template <typename R, int LOGN, int C, int LE = x_loge(LOGN)>
 __device__ __forceinline__ void x_fill(cx<R>* dst, const cx<R>* __restrict__ full, int rank) {
-    using S = XShape<LOGN, C>;
-    using X = XTables<R, LOGN, C>;
+    using S = XShape<LOGN, C, LE>;
+    using X = XTables<R, LOGN, C, LE>;
     if constexpr (S::SMALL) {
         for (int ns = X::FIRST; ns < S::N; ns *= X::RE)
             for (int i = threadIdx.x; i < X::NR * ns; i += S::TC)
@@ -275,10 +274,6 @@ __device__ __forceinline__ void x_fill(cx<R>* dst, const cx<R>* __restrict__ ful
         const int tid = threadIdx.x, g = rank * S::TC + tid;
         if constexpr (X::TWO_LEVEL) {
             for (int i = tid; i < X::N1; i += S::TC) dst[i] = i < 64 ? full[i] : full[(i - 64) * 64];
-        } else if constexpr (X::F32) {
-            const int x = x_col<LOGN, C>(g, 0);
-#pragma unroll
-            for (int q = 1; q < 16; q++) dst[(q - 1) * S::TC + tid] = full[(x * q) & (S::N - 1)];
         } else {
 #pragma unroll
             for (int h = 0; h < S::E / 16; h++) dst[h * S::TC + tid] = full[x_col<LOGN, C>(g, h)];
@@ -291,11 +286,11 @@ __device__ __forceinline__ void x_fill(cx<R>* dst, const cx<R>* __restrict__ ful
 }
 
 // One group's transform engine in precision R.
-template <typename R, typename RMAX, int LOGN, int C>
+template <typename R, typename RMAX, int LOGN, int C, int LE = x_loge(LOGN)>
 struct XForm {
-    using S = XShape<LOGN, C>;
-    using P = XPlan<R, RMAX, LOGN, C>;
-    using X = XTables<R, LOGN, C>;
+    using S = XShape<LOGN, C, LE>;
+    using P = XPlan<R, RMAX, LOGN, C, LE>;
+    using X = XTables<R, LOGN, C, LE>;
     using V = cx<R>;
     static constexpr int N = S::N, E = S::E, T = S::T, TC = S::TC, TT = S::TT, L = S::L, RS = S::RS;
 
@@ -432,9 +427,6 @@ struct XForm {
                     v[16 * h + q] = cmul(v[16 * h + q], cmul(tab[64 + (e >> 6)], tab[e & 63]));
                 }
             }
-        } else if constexpr (X::F32) {
-#pragma unroll
-            for (int q = 1; q < 16; q++) v[q] = cmul(v[q], tab[(q - 1) * TC + threadIdx.x]);
         } else {
             mul_powers<16, 0>(v, tab[threadIdx.x]);
             if constexpr (E == 32) mul_powers<16, 16>(v, tab[TC + threadIdx.x]);

@@ -120,10 +120,11 @@ bool gamma_symmetric(const double* g, int m) {
 }
 
 // u_shaped = u0 ⊙ cis(φ_b) (physics_models.jl:791-797): one phase per time
-// bin shared by the modes, or (per_mode) one per (t, m)
-__global__ void shaped_launch_kernel(const double2* __restrict__ u0,
-                                     const double* __restrict__ phases, int nt, int m,
-                                     int nbatch, double2* __restrict__ out, size_t out_stride,
+// bin shared by the modes, or (per_mode) one per (t, m); out may be u0 (one
+// launch).  Every path shapes here: a phase factor that differs in its last
+// bit flips roundings of the FP32 stage vectors.
+__global__ void shaped_launch_kernel(const double2* u0, const double* __restrict__ phases, int nt,
+                                     int m, int nbatch, double2* out, size_t out_stride,
                                      int per_mode = 0) {
     const long total = (long)nt * m * nbatch;
     for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total;
@@ -1185,7 +1186,8 @@ struct SrvRequest {
     int objective = OBJ_RAMAN_BAND;    // the problem's objective when submitted
     double obj_tau = 50.0;
     double L = 0;
-    std::vector<double> u0;            // shaped launch, (Nt, M) complex
+    std::vector<double> u0;            // launch, (Nt, M) complex
+    std::vector<double> phase;         // its spectral phase (Nt), or empty
     std::vector<unsigned char> mask;
     double* out_field = nullptr;
     double* out_grad = nullptr;
@@ -1331,12 +1333,27 @@ int srv_new_chunk(fl_server* sv, SrvBucket* b) {
     return FL_OK;
 }
 
+// the request's launch into u0, shaped there by its phase, which waits in the
+// slot's gradient buffer (nm >= Nt values, written when the solve ends)
+cudaError_t srv_upload_launch(fl_server* sv, SrvChunk* c, const fl_problem* pr, double* u0,
+                              double* phase, const SrvRequest* r) {
+    const size_t nm = (size_t)pr->nt * pr->m;
+    cudaError_t e = cudaMemcpyAsync(u0, r->u0.data(), 16 * nm, cudaMemcpyHostToDevice, c->stream);
+    if (e != cudaSuccess || r->phase.empty()) return e;
+    e = cudaMemcpyAsync(phase, r->phase.data(), 8 * (size_t)pr->nt, cudaMemcpyHostToDevice,
+                        c->stream);
+    if (e != cudaSuccess) return e;
+    shaped_launch_kernel<<<(int)((nm + 255) / 256), 256, 0, c->stream>>>(
+        (const double2*)u0, phase, pr->nt, pr->m, 1, (double2*)u0, nm, 0);
+    sv->launches++;
+    return cudaGetLastError();
+}
+
 // place request r into free slot i of chunk c (stream-ordered before the next launch)
 int srv_admit(fl_server* sv, SrvBucket* b, SrvChunk* c, int i, SrvRequest* r) {
     Nvtx nvtx_("fl: server admit");
     fl_ctx* ctx = sv->ctx;
     const fl_problem* pr = r->prob;
-    const size_t nm = (size_t)b->nt * b->m;
     const int mode = r->kind == FL_REQ_BAND_GRADIENT ? MODE_BAND_GRADIENT : MODE_FORWARD;
     unsigned char* dmask = c->d_masks + (size_t)i * b->nt;
     if (!r->mask.empty())
@@ -1369,7 +1386,7 @@ int srv_admit(fl_server* sv, SrvBucket* b, SrvChunk* c, int i, SrvRequest* r) {
         // a forward-only request keeps no checkpoints or step log
         d.ck_cap = mode == MODE_FORWARD ? 0 : c->mw->K;
         d.step_cap = mode == MODE_FORWARD ? 0 : c->mw->stepcap;
-        CU(cudaMemcpyAsync((double*)d.u0, r->u0.data(), 16 * nm, cudaMemcpyHostToDevice, c->stream));
+        CU(srv_upload_launch(sv, c, pr, (double*)d.u0, d.grad_out, r));
         CU(cudaMemcpyAsync((MmDesc*)c->mw->d_desc + i, &d, sizeof(MmDesc), cudaMemcpyHostToDevice,
                            c->stream));
         CU(cudaMemsetAsync(c->mw->d_state + i, 0, sizeof(MmState), c->stream));
@@ -1393,7 +1410,7 @@ int srv_admit(fl_server* sv, SrvBucket* b, SrvChunk* c, int i, SrvRequest* r) {
         // a forward-only request keeps no checkpoints or step log
         d.ck_cap = mode == MODE_FORWARD ? 0 : c->w->K;
         d.step_cap = mode == MODE_FORWARD ? 0 : c->w->stepcap;
-        CU(cudaMemcpyAsync((double*)d.u0, r->u0.data(), 16 * nm, cudaMemcpyHostToDevice, c->stream));
+        CU(srv_upload_launch(sv, c, pr, (double*)d.u0, d.grad_out, r));
         CU(cudaMemcpyAsync((SlotDesc*)c->w->d_desc + i, &d, sizeof(SlotDesc), cudaMemcpyHostToDevice,
                            c->stream));
         CU(cudaMemsetAsync(c->w->d_state + i, 0, sizeof(SlotState), c->stream));
@@ -2519,14 +2536,9 @@ int fl_server_submit(fl_server* sv, const fl_request* q, long* id) {
         r->mask.assign(q->mask, q->mask + pr->nt);
         for (auto x : r->mask) any |= x != 0;
         if (!any) return set_err(ctx, FL_EINVAL, "band mask must contain at least one bin");
-        // u_shaped = u0 ⊙ cis(φ) (physics_models.jl:791-797)
-        for (size_t k = 0; k < nm; k++) {
-            const double ph = q->phase[k % pr->nt];
-            if (!std::isfinite(ph)) return set_err(ctx, FL_EINVAL, "phase values must be finite");
-            const double c = std::cos(ph), s = std::sin(ph), a = r->u0[2 * k], b = r->u0[2 * k + 1];
-            r->u0[2 * k] = a * c - b * s;
-            r->u0[2 * k + 1] = a * s + b * c;
-        }
+        r->phase.assign(q->phase, q->phase + pr->nt);
+        for (double x : r->phase)
+            if (!std::isfinite(x)) return set_err(ctx, FL_EINVAL, "phase values must be finite");
         r->out_grad = q->out_grad;
     } else {
         r->out_field = q->out_field;

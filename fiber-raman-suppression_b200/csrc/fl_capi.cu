@@ -518,18 +518,13 @@ struct MmWork {
     double* d_uL = nullptr;
     double* d_zsave = nullptr;
     unsigned char* d_mask = nullptr;
-    // mm_run's batch of evaluation rounds as a CUDA graph, for graph_nactive slots
+    // mm_run's batch of evaluation rounds as a CUDA graph, for graph_nactive
+    // slots, with or without adjoint evaluations
     cudaGraphExec_t graph = nullptr;
-    int graph_nactive = -1;
-    // the rounds' side stream and its fork / join events
-    cudaStream_t side = nullptr;
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    int graph_nactive = -1, graph_adjoint = -1;
 
     ~MmWork() {
         if (graph) cudaGraphExecDestroy(graph);
-        if (ev_fork) cudaEventDestroy(ev_fork);
-        if (ev_join) cudaEventDestroy(ev_join);
-        if (side) cudaStreamDestroy(side);
         cudaFree(pool);
         cudaFree(d_desc);
         cudaFree(d_state);
@@ -582,9 +577,6 @@ int mm_work_create(fl_problem* pr, int B, int nsave, int mode, int per_mode, MmW
     CU(cudaMalloc(&w->pool, w->pool_bytes));
     CU(cudaMalloc(&w->d_desc, sizeof(MmDesc) * B));
     CU(cudaMalloc(&w->d_state, sizeof(MmState) * B));
-    CU(cudaStreamCreateWithFlags(&w->side, cudaStreamNonBlocking));
-    CU(cudaEventCreateWithFlags(&w->ev_fork, cudaEventDisableTiming));
-    CU(cudaEventCreateWithFlags(&w->ev_join, cudaEventDisableTiming));
     CU(cudaMalloc(&w->d_active, sizeof(int) * B));
     CU(cudaMalloc(&w->d_ndone, sizeof(int)));
     CU(cudaMallocHost(&w->h_ndone, sizeof(int)));
@@ -699,9 +691,6 @@ MmRound mm_round_args(fl_problem* pr, MmWork* w, int nactive) {
     a.fp64 = pr->precision == FL_PRECISION_FP64;
     a.lowrank_some = pr->rank > 0;  // one problem per batch
     a.fullrank_some = pr->rank == 0;
-    a.side = w->side;
-    a.ev_fork = w->ev_fork;
-    a.ev_join = w->ev_join;
     a.control = 1;
     a.tensor_cores = 1;
     a.ndone = nullptr;
@@ -720,35 +709,33 @@ int mm_run(fl_problem* pr, MmWork* w, int nactive) {
     MmRoundFn round = mm_round_launcher(ilog2i(pr->nt));
     if (!round) return set_err(ctx, FL_EUNSUPPORTED, "multimode Nt = %d is not built", pr->nt);
     MmRound a = mm_round_args(pr, w, nactive);
+    a.adjoint = w->h_desc[0].mode != MODE_FORWARD;  // one mode per batch
     CU(cudaEventRecord(ctx->ev[2], ctx->stream));
     CU(mm_launch_control(a, 0));
     ctx->launches++;
     const int per_batch = 8;
-    // one batch: 8 evaluation rounds, the counter of finished slots reset
-    // before the last round (which counts them)
+    // one batch: 8 evaluation rounds, the last of which counts the finished
+    // slots; the counter is reset first (a copy between two rounds would
+    // break their chain of programmatic launches)
     auto enqueue_batch = [&](cudaStream_t cs) -> cudaError_t {
         MmRound b = a;
         b.stream = cs;
-        for (int r = 0; r < per_batch; r++) {
-            b.ndone = nullptr;
-            if (r == per_batch - 1) {
-                const cudaError_t e = cudaMemsetAsync(w->d_ndone, 0, sizeof(int), cs);
-                if (e != cudaSuccess) return e;
-                b.ndone = w->d_ndone;
-            }
-            const cudaError_t e = round(b);
-            if (e != cudaSuccess) return e;
+        cudaError_t e = cudaMemsetAsync(w->d_ndone, 0, sizeof(int), cs);
+        for (int r = 0; e == cudaSuccess && r < per_batch; r++) {
+            b.chained = r > 0;
+            b.ndone = r == per_batch - 1 ? w->d_ndone : nullptr;
+            e = round(b);
         }
-        return cudaSuccess;
+        return e;
     };
     // The batch is captured once as a CUDA graph and replayed: each kernel
     // reads every slot's phase from device memory, so the same launches serve
-    // every batch, and a batch costs one graph launch instead of 8 x 7..10
+    // every batch, and a batch costs one graph launch instead of 8 x 5..8
     // kernel launches.  Capture is thread-local (other host threads, e.g. a
     // server's, keep launching) and runs on the context's private stream, so
     // a caller's stream (which may be the legacy default stream) is never put
     // in capture mode; the graph is launched on the context's current stream.
-    if (!w->graph || w->graph_nactive != nactive) {
+    if (!w->graph || w->graph_nactive != nactive || w->graph_adjoint != a.adjoint) {
         if (w->graph) cudaGraphExecDestroy(w->graph);
         w->graph = nullptr;
         w->graph_nactive = -1;
@@ -770,12 +757,13 @@ int mm_run(fl_problem* pr, MmWork* w, int nactive) {
                            cudaGetErrorString(e3));
         }
         w->graph_nactive = nactive;
+        w->graph_adjoint = a.adjoint;
     }
     const long max_rounds = 4 * 7 * (ctx->opts.max_iters + 2) + 64;
     long rounds = 0;
     for (;;) {
         CU(cudaGraphLaunch(w->graph, ctx->stream));
-        ctx->launches += per_batch * (a.fp64 ? 7 : 10);
+        ctx->launches += per_batch * mm_round_kernels(a);
         rounds += per_batch;
         CU(cudaMemcpyAsync(w->h_ndone, w->d_ndone, sizeof(int), cudaMemcpyDeviceToHost,
                            ctx->stream));
@@ -1103,8 +1091,10 @@ int mm_rhs_eval(fl_problem* pr, int adjoint, double z, const double* u_in, const
     CU(cudaMemcpyAsync(w->d_state, &st, sizeof st, cudaMemcpyHostToDevice, ctx->stream));
     MmRound a = mm_round_args(pr, w, 1);
     a.control = 0;
+    a.adjoint = adjoint;
+    a.chained = 0;
     CU(round(a));
-    ctx->launches += a.fp64 ? 6 : 9;
+    ctx->launches += mm_round_kernels(a);
     CU(cudaMemcpyAsync(du_out, w->d_lam0, 16 * nm, cudaMemcpyDeviceToHost, ctx->stream));
     CU(cudaStreamSynchronize(ctx->stream));
     return FL_OK;
@@ -1513,7 +1503,7 @@ int srv_launch(fl_server* sv, SrvBucket* b, SrvChunk* c) {
             }
         }
         CU(cudaGraphLaunch(c->graph, c->stream));
-        sv->launches += 1 + (long)sv->opts.evals_per_launch * (a.fp64 ? 7 : 10);
+        sv->launches += 1 + (long)sv->opts.evals_per_launch * mm_round_kernels(a);
     } else {
         // only the occupied slots, each over as many CTAs as the slots in
         // flight on the single-mode stepper leave it

@@ -99,7 +99,6 @@ __host__ __device__ constexpr int mm_loge(int logn) { return logn == 12 ? 3 : x_
 template <typename R, int LOGN, int LOGE, int C>
 struct MmGroup {
     static constexpr int LE = C == 1 ? mm_loge(LOGN) : LOGE;
-    using XS = XShape<LOGN, 1, LE>;
     using XF = XForm<R, R, LOGN, 1, LE>;
     static constexpr int N = 1 << LOGN, E = 1 << LE, TT = N / E, T = TT / C;
     // per-CTA exchange buffer bytes
@@ -107,28 +106,24 @@ struct MmGroup {
         C == 1 ? XPlan<R, R, LOGN, 1, LE>::BYTES : cluster_xbytes<R, LOGN, C>();
     static constexpr int TABLE =
         C == 1 ? XTables<R, LOGN, 1, LE>::SIZE : Twiddles<R, LOGN>::SIZE;
-    static constexpr size_t SMEM = XBYTES + sizeof(cx<R>) * TABLE + 32 * sizeof(double) + 16;
     int rank, g, flip;
     unsigned char* sm;
     double* red;
     cx<R>* tab;
 
-    // every CTA of the group calls it (uniform early exits only before it)
-    __device__ __forceinline__ void init(const MmDesc& d, unsigned char* smraw) {
-        rank = C == 1 ? 0 : (int)(blockIdx.x % C);
+    __device__ __forceinline__ MmGroup(unsigned char* buffer, cx<R>* table, double* sums)
+        : rank(C == 1 ? 0 : (int)(blockIdx.x % C)), flip(0), sm(buffer), red(sums), tab(table) {
         g = rank * T + threadIdx.x;
-        flip = 0;
-        sm = smraw;
-        tab = reinterpret_cast<cx<R>*>(smraw + XBYTES);
-        red = reinterpret_cast<double*>(smraw + ((XBYTES + sizeof(cx<R>) * TABLE + 15) & ~size_t(15)));
+    }
+    __device__ __forceinline__ void fill(const MmDesc& d) const {
         const cx<R>* full = static_cast<const cx<R>*>(d.tw[sizeof(R) == 8]);
-        if constexpr (C == 1) {
-            x_fill<R, LOGN, 1, LE>(tab, full, 0);
-            __syncthreads();
-        } else {
-            Twiddles<R, LOGN>::fill(tab, full);
-            cluster_sync_all();
-        }
+        if constexpr (C == 1) x_fill<R, LOGN, 1, LE>(tab, full, 0);
+        else Twiddles<R, LOGN>::fill(tab, full);
+    }
+    // the table is there and (clusters) every CTA has started
+    __device__ __forceinline__ void begin() const {
+        if constexpr (C == 1) __syncthreads();
+        else cluster_sync_all();
     }
     __device__ __forceinline__ int own(int s) const { return g + TT * s; }
     __device__ __forceinline__ int bin(int s) const {
@@ -151,32 +146,95 @@ struct MmGroup {
 };
 
 // ---------------------------------------------------------------------------
+// The three transform kernels serve a mixed batch in one launch each: a CTA
+// (cluster) reads its slot's phase and runs its task in FP32 or FP64.  MIX:
+// an FP32 batch (FP64 batches have no FP32 task).
+//
+// All kernels of a round form one chain of programmatic dependent launches:
+// each lets its successor start at once (mm_chain_start) and waits for its
+// predecessor (mm_chain_wait) before it touches what the chain writes; every
+// thread waits, so a kernel's end implies the end of all before it.  Before
+// the wait only what the chain never writes is read: the active list, the
+// descriptors, the twiddle tables.  State pointers are not __restrict__ (an
+// invariant load could move above the wait).
+//
+// What bounds a round of one slot is the chain itself: six to eight kernels
+// of 3..32 CTAs, each a launch, its descriptor and table loads, and one pass
+// over its data.  Separate FP32 and FP64 launches per stage on two joined
+// streams ran 10 kernels, 54 us, per forward round of 6 modes at Nt = 2^12
+// and 42 us (3 modes, FP64, Nt = 2^11); the chain runs 46 and 33 us (whole
+// gradient 29.1 -> 23.5 ms, forward 3.8 -> 2.9 ms).  In a large batch it
+// saves the empty CTAs: 64 x 10 modes at 2^14, 560 -> 503 ms together with
+// the pair sequences read twice (mm_pairs).
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void mm_chain_start() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void mm_chain_wait() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <bool MIX, int LOGN, int LOGE, int CL>
+struct MmTasks {
+    using GF = MmGroup<float, LOGN, LOGE, CL>;
+    using GD = MmGroup<double, LOGN, LOGE, CL>;
+    static constexpr int T = GD::T;
+    // several CTAs per SM on the smaller grids (128 registers per thread)
+    static constexpr int CTAS = T >= 512 || CL > 1 ? 1 : T >= 128 ? 512 / T : 4;
+    static constexpr size_t XB = MIX && GF::XBYTES > GD::XBYTES ? GF::XBYTES : GD::XBYTES;
+    static constexpr size_t TABD = (XB + 15) & ~size_t(15);
+    static constexpr size_t TABF = TABD + sizeof(cx<double>) * GD::TABLE;
+    static constexpr size_t RED =
+        (TABF + (MIX ? sizeof(cx<float>) * GF::TABLE : 0) + 15) & ~size_t(15);
+    static constexpr size_t SMEM = RED + 32 * sizeof(double);
+
+    // body(group of the task's precision) for the slot's task: task(state) is
+    // 0 (none), 4 (FP32) or 8 (FP64).  Small launches fill the tables while
+    // the predecessor still runs; in large ones the CTAs come in waves and
+    // fill the one they need.
+    template <class Task, class Body>
+    __device__ static __forceinline__ void run(const MmDesc& d, const MmState* state,
+                                               unsigned char* smraw, Task&& task, Body&& body) {
+        GD gd(smraw, reinterpret_cast<cx<double>*>(smraw + TABD),
+              reinterpret_cast<double*>(smraw + RED));
+        GF gf(smraw, reinterpret_cast<cx<float>*>(smraw + TABF),
+              reinterpret_cast<double*>(smraw + RED));
+        const bool early = gridDim.x * gridDim.y <= 148;
+        mm_chain_start();
+        if (early) {
+            gd.fill(d);
+            if constexpr (MIX) gf.fill(d);
+        }
+        mm_chain_wait();
+        const MmState st = *state;
+        const int t = task(st);
+        if (t == 8) {
+            if (!early) gd.fill(d);
+            gd.begin();
+            body(gd, st);
+        } else if (MIX && t == 4) {
+            if constexpr (MIX) {
+                if (!early) gf.fill(d);
+                gf.begin();
+                body(gf, st);
+            }
+        }
+    }
+};
+
+// ---------------------------------------------------------------------------
 // prologue: stage input of mode m and its transform(s) to time
 // ---------------------------------------------------------------------------
 template <typename R, int LOGN, int LOGE, int CL>
-__global__ void __launch_bounds__(MmGroup<R, LOGN, LOGE, CL>::T, 1)
-    mm_prologue_kernel(const MmDesc* __restrict__ descs, const MmState* __restrict__ states,
-                       const int* __restrict__ active) {
+__device__ __forceinline__ void mm_prologue(MmGroup<R, LOGN, LOGE, CL>& grp, const MmDesc& d,
+                                            const MmState& st, int m, bool fwd_field) {
     using G = MmGroup<R, LOGN, LOGE, CL>;
     constexpr int N = G::N, E = G::E;
     constexpr int P = sizeof(R) == 8;
     using C = cx<R>;
-    extern __shared__ __align__(16) unsigned char smraw[];
-    const int slot = active[blockIdx.y];
-    const MmDesc& d = descs[slot];
-    const int m = blockIdx.x / CL;
-    if (m >= d.M) return;
-    const MmState st = states[slot];
-    // a mixed-precision adjoint (mm_adj_mixed) transforms λ in the FP64
-    // kernel and the forward field in the FP32 one
-    const bool fwd_field = sizeof(R) == 4 && d.adj_mixed && mm_rhs_phase(st.phase) &&
-                           mm_adjoint_phase(st.phase);
-    if (!mm_takes<R>(d, st) && !fwd_field) return;
-    G grp;
-    grp.init(d, smraw);
     const size_t NM = (size_t)N * d.M, off = (size_t)m * N;
     const int ph = st.phase;
-    const bool adj = mm_adjoint_phase(ph);
+    const bool adj = P && mm_adjoint_phase(ph);
     const double* Dt = d.Dturns + off;
     C v[E];
 
@@ -344,6 +402,28 @@ __global__ void __launch_bounds__(MmGroup<R, LOGN, LOGE, CL>::T, 1)
     for (int s = 0; s < E; s++) uo[off + grp.own(s)] = v[s];
 }
 
+// units [0, M): the mode's stage input (adjoint: FP64), units [M, 2M) of a
+// mixed-precision adjoint (mm_adj_mixed): the forward field, in FP32
+template <bool MIX, int LOGN, int LOGE, int CL>
+__global__ void __launch_bounds__(MmTasks<MIX, LOGN, LOGE, CL>::T, MmTasks<MIX, LOGN, LOGE, CL>::CTAS)
+    mm_prologue_kernel(const MmDesc* __restrict__ descs, const MmState* states,
+                       const int* __restrict__ active) {
+    extern __shared__ __align__(16) unsigned char smraw[];
+    const int slot = active[blockIdx.y];
+    const MmDesc& d = descs[slot];
+    const int unit = blockIdx.x / CL;
+    const bool field = unit >= d.M;
+    MmTasks<MIX, LOGN, LOGE, CL>::run(
+        d, states + slot, smraw,
+        [&](const MmState& st) {
+            if (!mm_rhs_phase(st.phase)) return 0;
+            const bool adj = mm_adjoint_phase(st.phase);
+            if (field) return adj && d.adj_mixed && unit < 2 * d.M ? 4 : 0;
+            return adj || d.fp64 ? 8 : 4;
+        },
+        [&](auto& grp, const MmState& st) { mm_prologue(grp, d, st, field ? unit - d.M : unit, field); });
+}
+
 // ---------------------------------------------------------------------------
 // pairs: Raman convolutions of the symmetric pair products.  Two real
 // sequences of the same kind share one complex transform pair (the kernels
@@ -354,38 +434,22 @@ __global__ void __launch_bounds__(MmGroup<R, LOGN, LOGE, CL>::T, 1)
 // smaller Im X would leave Im X with the rounding of P.
 // ---------------------------------------------------------------------------
 template <typename R, int LOGN, int LOGE, int CL>
-__global__ void __launch_bounds__(MmGroup<R, LOGN, LOGE, CL>::T, 1)
-    mm_pairs_kernel(const MmDesc* __restrict__ descs, const MmState* __restrict__ states,
-                    const int* __restrict__ active) {
+__device__ __forceinline__ void mm_pairs(MmGroup<R, LOGN, LOGE, CL>& grp, const MmDesc& d,
+                                         const MmState& st, int unit) {
     using G = MmGroup<R, LOGN, LOGE, CL>;
     constexpr int N = G::N, E = G::E;
     constexpr int P = sizeof(R) == 8;
     using C = cx<R>;
-    extern __shared__ __align__(16) unsigned char smraw[];
-    const int slot = active[blockIdx.y];
-    const MmDesc& d = descs[slot];
-    const MmState st = states[slot];
-    const bool adj = mm_rhs_phase(st.phase) && mm_adjoint_phase(st.phase);
-    // a mixed-precision adjoint (mm_adj_mixed) forms the products P of the
-    // forward field in the FP32 kernel and the Im X correlations in FP64
-    const bool mixed = adj && d.adj_mixed;
-    if (!mm_takes<R>(d, st) && !(mixed && sizeof(R) == 4)) return;
+    const bool adj = mm_adjoint_phase(st.phase);
     const int M = d.M, NP = d.NP, ntp = (NP + 1) / 2;
-    const int unit = blockIdx.x / CL;
-    const bool ytask = unit >= ntp;  // correlation of Im X (adjoint only)
-    if (ytask && !adj) return;
-    if (mixed && ytask != (sizeof(R) == 8)) return;
+    const bool ytask = P && unit >= ntp;  // correlation of Im X (adjoint only)
     // the low-rank form (rank > 0, FP32 kernels only) convolves pairs of the
     // rank sequences Z_k = Σ_q V[q][k] P_q instead of the NP products
     // (and the adjoint correlates the rank sequences Yz_k = Σ_q V[q][k] Y_q)
     const bool zmode = !ytask && d.rank > 0;
     const int nseq = d.rank > 0 ? d.rank : NP;
-    const int q0 = 2 * (ytask ? unit - ntp : unit);
-    if (q0 >= nseq) return;
-    const int q1 = q0 + 1;
+    const int q0 = 2 * (ytask ? unit - ntp : unit), q1 = q0 + 1;
     const bool two = q1 < nseq;
-    G grp;
-    grp.init(d, smraw);
     const C* ut = static_cast<const C*>(d.ut);
     const C* H = static_cast<const C*>(d.Heff[P]);
     R* sq = static_cast<R*>(d.sq);
@@ -394,29 +458,35 @@ __global__ void __launch_bounds__(MmGroup<R, LOGN, LOGE, CL>::T, 1)
     int k0, l0, k1 = 0, l1 = 0;
     pair_kl(q0, M, k0, l0);
     if (two) pair_kl(q1, M, k1, l1);
-    C v[E];
-    R p0[E], p1[E];
-#pragma unroll
-    for (int s = 0; s < E; s++) {
-        const int t = grp.own(s);
+    // the two sequences at time element t
+    auto load = [&](int t) -> C {
+        R a0, a1 = R(0);
         if (ytask) {
-            p0[s] = cq[(size_t)q0 * N + t];
-            p1[s] = two ? cq[(size_t)q1 * N + t] : R(0);
+            a0 = cq[(size_t)q0 * N + t];
+            if (two) a1 = cq[(size_t)q1 * N + t];
         } else if (zmode) {
             const R* zq = sq + (size_t)NP * N;  // Z_k rows (upper half of the pair table)
-            p0[s] = zq[(size_t)q0 * N + t];
-            p1[s] = two ? zq[(size_t)q1 * N + t] : R(0);
+            a0 = zq[(size_t)q0 * N + t];
+            if (two) a1 = zq[(size_t)q1 * N + t];
         } else {
             const C a = ut[(size_t)k0 * N + t], b = ut[(size_t)l0 * N + t];
-            p0[s] = a.re * b.re + a.im * b.im;  // Re(u_k u_l*)
+            a0 = a.re * b.re + a.im * b.im;  // Re(u_k u_l*)
             if (two) {
-                const C a1 = ut[(size_t)k1 * N + t], b1 = ut[(size_t)l1 * N + t];
-                p1[s] = a1.re * b1.re + a1.im * b1.im;
-            } else {
-                p1[s] = R(0);
+                const C c = ut[(size_t)k1 * N + t], e = ut[(size_t)l1 * N + t];
+                a1 = c.re * e.re + c.im * e.im;
             }
         }
-        v[s] = mk(p0[s], p1[s]);
+        return mk(a0, a1);
+    };
+    // with 32 values per thread the sequences are read again after the
+    // transforms (they are in L2) instead of held in 64 registers: the FP32
+    // pairs of 64 x 10 modes at 2^14 (rank form) take 197 us for 337
+    constexpr bool HOLD = E < 32;
+    C v[E], p[HOLD ? E : 1];
+#pragma unroll
+    for (int s = 0; s < E; s++) {
+        v[s] = load(grp.own(s));
+        if constexpr (HOLD) p[s] = v[s];
     }
     grp.to_freq(v);
 #pragma unroll
@@ -436,10 +506,37 @@ __global__ void __launch_bounds__(MmGroup<R, LOGN, LOGE, CL>::T, 1)
             cq[(size_t)q0 * N + t] = v[s].re * invn;
             if (two) cq[(size_t)q1 * N + t] = v[s].im * invn;
         } else {
-            sq[(size_t)q0 * N + t] = kf * p0[s] + v[s].re * invn;
-            if (two) sq[(size_t)q1 * N + t] = kf * p1[s] + v[s].im * invn;
+            C x;
+            if constexpr (HOLD) x = p[s];
+            else x = load(t);
+            sq[(size_t)q0 * N + t] = kf * x.re + v[s].re * invn;
+            if (two) sq[(size_t)q1 * N + t] = kf * x.im + v[s].im * invn;
         }
     }
+}
+
+// a mixed-precision adjoint (mm_adj_mixed) convolves the products P of the
+// forward field in FP32 and correlates Im X in FP64
+template <bool MIX, int LOGN, int LOGE, int CL>
+__global__ void __launch_bounds__(MmTasks<MIX, LOGN, LOGE, CL>::T, MmTasks<MIX, LOGN, LOGE, CL>::CTAS)
+    mm_pairs_kernel(const MmDesc* __restrict__ descs, const MmState* states,
+                    const int* __restrict__ active) {
+    extern __shared__ __align__(16) unsigned char smraw[];
+    const int slot = active[blockIdx.y];
+    const MmDesc& d = descs[slot];
+    const int unit = blockIdx.x / CL;
+    MmTasks<MIX, LOGN, LOGE, CL>::run(
+        d, states + slot, smraw,
+        [&](const MmState& st) {
+            if (!mm_rhs_phase(st.phase)) return 0;
+            const bool adj = mm_adjoint_phase(st.phase);
+            const int ntp = (d.NP + 1) / 2;
+            const bool ytask = unit >= ntp;
+            if (ytask && !adj) return 0;
+            if (2 * (ytask ? unit - ntp : unit) >= (d.rank > 0 ? d.rank : d.NP)) return 0;
+            return d.fp64 || ytask || (adj && !d.adj_mixed) ? 8 : 4;
+        },
+        [&](auto& grp, const MmState& st) { mm_pairs(grp, d, st, unit); });
 }
 
 // ---------------------------------------------------------------------------
@@ -447,25 +544,15 @@ __global__ void __launch_bounds__(MmGroup<R, LOGN, LOGE, CL>::T, 1)
 // as the stage derivative; the stage-7 error partial of the mode
 // ---------------------------------------------------------------------------
 template <typename R, int LOGN, int LOGE, int CL>
-__global__ void __launch_bounds__(MmGroup<R, LOGN, LOGE, CL>::T, 1)
-    mm_epilogue_kernel(const MmDesc* __restrict__ descs, const MmState* __restrict__ states,
-                       const int* __restrict__ active) {
+__device__ __forceinline__ void mm_epilogue(MmGroup<R, LOGN, LOGE, CL>& grp, const MmDesc& d,
+                                            const MmState& st, int m) {
     using G = MmGroup<R, LOGN, LOGE, CL>;
     constexpr int N = G::N, E = G::E, T = G::T;
     constexpr int P = sizeof(R) == 8;
     using C = cx<R>;
-    extern __shared__ __align__(16) unsigned char smraw[];
-    const int slot = active[blockIdx.y];
-    const MmDesc& d = descs[slot];
-    const int m = blockIdx.x / CL;
-    if (m >= d.M) return;
-    const MmState st = states[slot];
-    if (!mm_takes<R>(d, st)) return;
-    G grp;
-    grp.init(d, smraw);
     const size_t off = (size_t)m * N;
     const int ph = st.phase;
-    const bool adj = mm_adjoint_phase(ph);
+    const bool adj = P && mm_adjoint_phase(ph);
     const C* eta = static_cast<const C*>(d.eta);
     C v[E];
 #pragma unroll
@@ -555,6 +642,23 @@ __global__ void __launch_bounds__(MmGroup<R, LOGN, LOGE, CL>::T, 1)
         const double tot = block_sum<T>(acc, grp.red);
         if (threadIdx.x == 0) d.part[m * CL + grp.rank] = tot;
     }
+}
+
+template <bool MIX, int LOGN, int LOGE, int CL>
+__global__ void __launch_bounds__(MmTasks<MIX, LOGN, LOGE, CL>::T, MmTasks<MIX, LOGN, LOGE, CL>::CTAS)
+    mm_epilogue_kernel(const MmDesc* __restrict__ descs, const MmState* states,
+                       const int* __restrict__ active) {
+    extern __shared__ __align__(16) unsigned char smraw[];
+    const int slot = active[blockIdx.y];
+    const MmDesc& d = descs[slot];
+    const int m = blockIdx.x / CL;
+    MmTasks<MIX, LOGN, LOGE, CL>::run(
+        d, states + slot, smraw,
+        [&](const MmState& st) {
+            if (m >= d.M || !mm_rhs_phase(st.phase)) return 0;
+            return d.fp64 || mm_adjoint_phase(st.phase) ? 8 : 4;
+        },
+        [&](auto& grp, const MmState& st) { mm_epilogue(grp, d, st, m); });
 }
 
 // ---------------------------------------------------------------------------
@@ -732,10 +836,12 @@ __device__ __forceinline__ void mm_contract_adj(const MmDesc& d, int t, int j) {
 // which = 0: forward contraction in R; 1: adjoint Im X; 2: adjoint assembly
 template <typename R, int M>
 __global__ void __launch_bounds__(kMmTB)
-    mm_contract_kernel(const MmDesc* __restrict__ descs, const MmState* __restrict__ states,
+    mm_contract_kernel(const MmDesc* __restrict__ descs, const MmState* states,
                        const int* __restrict__ active, int which) {
+    mm_chain_start();
     const int slot = active[blockIdx.y];
     const MmDesc& d = descs[slot];
+    mm_chain_wait();
     if (d.M != M) return;
     const MmState st = states[slot];
     if (!mm_takes<R>(d, st)) return;

@@ -40,12 +40,22 @@ int mm_cluster_ctas(int logn) { return logn == 15 ? 4 : 1; }
 
 bool mm_supported_modes(int M) { return M >= 2 && M <= 10; }
 
+int mm_round_kernels(const MmRound& a) {
+    const bool mixed = mm_adj_mixed(a.M, a.N, a.fp64);
+    int n = 4 + (a.control ? 1 : 0);  // prologue, pairs, forward contraction, epilogue
+    if (mixed && a.lowrank_some) n++;
+    if (a.adjoint) n += 1 + (!mixed || a.fullrank_some ? 1 : 0);
+    return n;
+}
+
 __global__ void __launch_bounds__(kMmCtl)
-    mm_control_kernel(const MmDesc* __restrict__ descs, MmState* __restrict__ states,
+    mm_control_kernel(const MmDesc* __restrict__ descs, MmState* states,
                       const int* __restrict__ active, int consume, int* __restrict__ ndone) {
     __shared__ double red[32];
+    mm_chain_start();
     const int slot = active[blockIdx.x];
     const MmDesc& d = descs[slot];
+    mm_chain_wait();
     MmState st = states[slot];
     MmCtl c{d, st, red, (size_t)d.N * d.M, d.N};
     if (consume && mm_rhs_phase(st.phase) && st.phase != PH_EVAL_FWD && st.phase != PH_EVAL_ADJ)
@@ -71,11 +81,13 @@ __global__ void __launch_bounds__(kMmCtl)
 // of 128): CTAs loop over a slot's 128-point tiles.
 template <int M>
 __global__ void __launch_bounds__(kTcRows)
-    mm_contract_tc_kernel(const MmDesc* __restrict__ descs, const MmState* __restrict__ states,
+    mm_contract_tc_kernel(const MmDesc* __restrict__ descs, const MmState* states,
                           const int* __restrict__ active) {
     extern __shared__ __align__(16) unsigned char tc_smem[];
+    mm_chain_start();
     const int slot = active[blockIdx.y];
     const MmDesc& d = descs[slot];
+    mm_chain_wait();
     if (d.M != M) return;
     const MmState st = states[slot];
     if (!mm_takes<float>(d, st) || mm_adjoint_phase(st.phase)) return;
@@ -87,11 +99,13 @@ __global__ void __launch_bounds__(kTcRows)
 // 128-point tile per CTA.
 template <int M>
 __global__ void __launch_bounds__(kTcRows, 2)
-    mm_contract_adj_tc_kernel(const MmDesc* __restrict__ descs, const MmState* __restrict__ states,
+    mm_contract_adj_tc_kernel(const MmDesc* __restrict__ descs, const MmState* states,
                               const int* __restrict__ active) {
     extern __shared__ __align__(16) unsigned char tc_smem[];
+    mm_chain_start();
     const int slot = active[blockIdx.y];
     const MmDesc& d = descs[slot];
+    mm_chain_wait();
     if (d.M != M || !d.adj_mixed) return;
     const MmState st = states[slot];
     if (!mm_takes<double>(d, st) || !mm_adjoint_phase(st.phase)) return;
@@ -102,11 +116,13 @@ __global__ void __launch_bounds__(kTcRows, 2)
 // cores (M >= 6, Nt a multiple of 128): one 128-point tile per CTA.
 template <int M>
 __global__ void __launch_bounds__(kTcRows, 2)
-    mm_imx_tc_kernel(const MmDesc* __restrict__ descs, const MmState* __restrict__ states,
+    mm_imx_tc_kernel(const MmDesc* __restrict__ descs, const MmState* states,
                      const int* __restrict__ active) {
     extern __shared__ __align__(16) unsigned char tc_smem[];
+    mm_chain_start();
     const int slot = active[blockIdx.y];
     const MmDesc& d = descs[slot];
+    mm_chain_wait();
     // (with a low-rank form the Z kernel reduces Y to the rank instead)
     if (d.M != M || !d.adj_mixed || d.rank > 0) return;
     const MmState st = states[slot];
@@ -118,11 +134,13 @@ __global__ void __launch_bounds__(kTcRows, 2)
 // FP32 batch (forward, and the mixed adjoint's forward field).
 template <int M>
 __global__ void __launch_bounds__(kTcRows, 2)
-    mm_z_tc_kernel(const MmDesc* __restrict__ descs, const MmState* __restrict__ states,
+    mm_z_tc_kernel(const MmDesc* __restrict__ descs, const MmState* states,
                    const int* __restrict__ active) {
     extern __shared__ __align__(16) unsigned char tc_smem[];
+    mm_chain_start();
     const int slot = active[blockIdx.y];
     const MmDesc& d = descs[slot];
+    mm_chain_wait();
     if (d.M != M || d.rank <= 0 || d.fp64) return;
     const MmState st = states[slot];
     if (!mm_rhs_phase(st.phase)) return;
@@ -138,9 +156,8 @@ cudaError_t z_tc(const MmRound& a) {
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     const dim3 grid(a.N / kTcRows, a.nactive);
-    mm_z_tc_kernel<M><<<grid, kTcRows, smem, a.stream>>>(static_cast<const MmDesc*>(a.desc),
-                                                        a.state, a.active);
-    return cudaGetLastError();
+    return mm_chain_launch(mm_z_tc_kernel<M>, grid, kTcRows, smem, a.stream, 1, true, static_cast<const MmDesc*>(a.desc),
+                           static_cast<const MmState*>(a.state), a.active);
 }
 
 template <int M>
@@ -150,9 +167,8 @@ cudaError_t imx_tc(const MmRound& a) {
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     const dim3 grid(a.N / kTcRows, a.nactive);
-    mm_imx_tc_kernel<M><<<grid, kTcRows, smem, a.stream>>>(static_cast<const MmDesc*>(a.desc),
-                                                          a.state, a.active);
-    return cudaGetLastError();
+    return mm_chain_launch(mm_imx_tc_kernel<M>, grid, kTcRows, smem, a.stream, 1, true, static_cast<const MmDesc*>(a.desc),
+                           static_cast<const MmState*>(a.state), a.active);
 }
 
 template <int M>
@@ -162,9 +178,8 @@ cudaError_t contract_adj_tc(const MmRound& a) {
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     const dim3 grid(a.N / kTcRows, a.nactive);
-    mm_contract_adj_tc_kernel<M><<<grid, kTcRows, smem, a.stream>>>(
-        static_cast<const MmDesc*>(a.desc), a.state, a.active);
-    return cudaGetLastError();
+    return mm_chain_launch(mm_contract_adj_tc_kernel<M>, grid, kTcRows, smem, a.stream, 1, true, static_cast<const MmDesc*>(a.desc),
+                           static_cast<const MmState*>(a.state), a.active);
 }
 
 template <int M>
@@ -176,9 +191,8 @@ cudaError_t contract_tc(const MmRound& a) {
     // one 128-point tile per CTA (many CTAs in flight hide each tile's
     // load -> MMA -> drain chain better than a persistent loop)
     const dim3 grid(a.N / kTcRows, a.nactive);
-    mm_contract_tc_kernel<M><<<grid, kTcRows, smem, a.stream>>>(
-        static_cast<const MmDesc*>(a.desc), a.state, a.active);
-    return cudaGetLastError();
+    return mm_chain_launch(mm_contract_tc_kernel<M>, grid, kTcRows, smem, a.stream, 1, true, static_cast<const MmDesc*>(a.desc),
+                           static_cast<const MmState*>(a.state), a.active);
 }
 
 template <typename R, int M>
@@ -204,9 +218,9 @@ cudaError_t contract_m(const MmRound& a, int which) {
     }
     const int n = which == 2 ? a.N * M : a.N;
     const dim3 grid((n + kMmTB - 1) / kMmTB, a.nactive);
-    mm_contract_kernel<R, M><<<grid, kMmTB, 0, a.stream>>>(static_cast<const MmDesc*>(a.desc),
-                                                          a.state, a.active, which);
-    return cudaGetLastError();
+    return mm_chain_launch(mm_contract_kernel<R, M>, grid, kMmTB, 0, a.stream, 1, true,
+                           static_cast<const MmDesc*>(a.desc), static_cast<const MmState*>(a.state),
+                           a.active, which);
 }
 
 template <typename R>
@@ -236,9 +250,8 @@ cudaError_t mm_launch_contract(const MmRound& a, int which) {
 }
 
 cudaError_t mm_launch_control(const MmRound& a, int consume) {
-    mm_control_kernel<<<a.nactive, kMmCtl, 0, a.stream>>>(static_cast<const MmDesc*>(a.desc),
-                                                          a.state, a.active, consume, a.ndone);
-    return cudaGetLastError();
+    return mm_chain_launch(mm_control_kernel, dim3(a.nactive), kMmCtl, 0, a.stream, 1, consume != 0,
+                           static_cast<const MmDesc*>(a.desc), a.state, a.active, consume, a.ndone);
 }
 
 }  // namespace fl

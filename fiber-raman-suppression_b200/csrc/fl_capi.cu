@@ -18,6 +18,7 @@
 #include <memory>
 #include <new>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include <nvtx3/nvToolsExt.h>
@@ -28,8 +29,91 @@
 
 using namespace fl;
 
+// Device blocks of a context's problems and workspaces.  Mapping and unmapping
+// device memory is what a short call on a fresh problem used to wait for: of
+// 5.4 ms for a propagation at Nt = 2^12 with five save positions, 0.8 ms in
+// cudaMalloc and 0.8 ms in cudaFree, beside 3.5 ms of kernels.  Released
+// blocks are kept for the next object: at most kKeep bytes, given back with
+// the context, and before an allocation fails.  A block is reused only after
+// the context's stream has run dry, and by objects of the same context.
+struct BlockCache {
+    static constexpr size_t kKeep = size_t(256) << 20;
+    struct Block {
+        void* p;
+        size_t bytes;
+    };
+    std::mutex mu;
+    bool open = true;                // the context is alive
+    cudaStream_t stream = nullptr;   // its stream
+    std::vector<Block> live, spare;  // spare: oldest first
+    size_t kept = 0;
+
+    cudaError_t alloc(void** out, size_t bytes) {
+        std::lock_guard<std::mutex> lk(mu);
+        *out = nullptr;
+        bytes = (std::max<size_t>(bytes, 1) + 511) & ~size_t(511);
+        // the smallest spare block that wastes no more than half of itself
+        size_t best = spare.size();
+        for (size_t i = 0; i < spare.size(); i++)
+            if (spare[i].bytes >= bytes && spare[i].bytes <= 2 * bytes &&
+                (best == spare.size() || spare[i].bytes < spare[best].bytes))
+                best = i;
+        Block b{nullptr, bytes};
+        if (best < spare.size()) {
+            b = spare[best];
+            spare.erase(spare.begin() + best);
+            kept -= b.bytes;
+        } else {
+            cudaError_t e = cudaMalloc(&b.p, bytes);
+            if (e == cudaErrorMemoryAllocation && !spare.empty()) {
+                cudaGetLastError();
+                trim(0);
+                e = cudaMalloc(&b.p, bytes);
+            }
+            if (e != cudaSuccess) return e;
+        }
+        live.push_back(b);
+        *out = b.p;
+        return cudaSuccess;
+    }
+    void release(void* p) {
+        if (!p) return;
+        std::lock_guard<std::mutex> lk(mu);
+        for (size_t i = 0; i < live.size(); i++) {
+            if (live[i].p != p) continue;
+            const Block b = live[i];
+            live.erase(live.begin() + i);
+            if (!open || b.bytes > kKeep / 2 || cudaStreamSynchronize(stream) != cudaSuccess) {
+                cudaFree(p);
+                return;
+            }
+            spare.push_back(b);
+            kept += b.bytes;
+            trim(kKeep);
+            return;
+        }
+    }
+    void close() {
+        std::lock_guard<std::mutex> lk(mu);
+        open = false;
+        trim(0);
+    }
+
+private:
+    void trim(size_t limit) {
+        size_t n = 0;
+        while (kept > limit && n < spare.size()) {
+            kept -= spare[n].bytes;
+            cudaFree(spare[n++].p);
+        }
+        spare.erase(spare.begin(), spare.begin() + n);
+    }
+};
+
 struct fl_ctx {
     int device = 0;
+    // shared with the objects that hold blocks (they may outlive the context)
+    std::shared_ptr<BlockCache> blocks = std::make_shared<BlockCache>();
     cudaStream_t stream = nullptr;  // the stream every call of this context runs on
     cudaStream_t own = nullptr;     // the context's private stream (the default for stream)
     std::string err;
@@ -63,6 +147,17 @@ int set_err(fl_ctx* c, int code, const char* fmt, ...) {
         c->err = buf;
     }
     return code;
+}
+
+// a cache that keeps nothing
+std::shared_ptr<BlockCache> closed_blocks() {
+    auto c = std::make_shared<BlockCache>();
+    c->close();
+    return c;
+}
+template <class T>
+cudaError_t block_alloc(const std::shared_ptr<BlockCache>& c, T** out, size_t bytes) {
+    return c->alloc(reinterpret_cast<void**>(out), bytes);
 }
 
 #define CU(call)                                                                         \
@@ -161,12 +256,14 @@ __global__ void gather_stats_kernel(const SlotState* __restrict__ st, int n,
 
 struct fl_problem {
     fl_ctx* ctx = nullptr;
+    std::shared_ptr<BlockCache> blocks;    // of its tables and staging areas
     int nt = 0, m = 0, precision = 0;
     double one_m_fR = 0, L = 0, reltol = 0, abstol = 0, gamma0 = 0;
     bool gamma_sym = true;
     int objective = OBJ_RAMAN_BAND;        // terminal objective of the gradient entry points
     double obj_tau = 50.0;                 // worst-mode smoothness
     bool use_mm = false;  // multimode runtime: M > 1, or M = 1 beyond one CTA's transform (2^15)
+    char* d_tables = nullptr;              // one block of the four tables below
     double* d_Dturns = nullptr;
     void* d_Heff[2] = {nullptr, nullptr};  // [0] float, [1] double
     void* d_ss[2] = {nullptr, nullptr};
@@ -193,6 +290,7 @@ struct fl_problem {
 // Per-batch workspace: one allocation carved into per-slot buffers.
 struct Work {
     fl_ctx* ctx = nullptr;
+    std::shared_ptr<BlockCache> blocks;  // a server chunk (its own stream) has its own
     int B = 0, nt = 0, rsize = 4, K = 0, segcap = 0, stepcap = 0, nsave = 0;
     char* pool = nullptr;
     size_t pool_bytes = 0;
@@ -210,10 +308,7 @@ struct Work {
     unsigned char* d_mask = nullptr;
 
     ~Work() {
-        cudaFree(pool);
-        cudaFree(d_desc);
-        cudaFree(d_state);
-        cudaFree(d_active);
+        for (void* p : {(void*)pool, d_desc, (void*)d_state, (void*)d_active}) blocks->release(p);
     }
 };
 
@@ -256,6 +351,7 @@ int work_create(fl_problem* pr, int B, int nsave, int mode, Work** out,
     cudaStream_t strm = opt ? stream : ctx->stream;
     auto w = std::make_unique<Work>();
     w->ctx = ctx;
+    w->blocks = opt ? closed_blocks() : ctx->blocks;
     w->B = B;
     w->nt = pr->nt;
     w->rsize = (int)rf;
@@ -270,10 +366,10 @@ int work_create(fl_problem* pr, int B, int nsave, int mode, Work** out,
     if (o.hbm_budget_bytes && w->pool_bytes > o.hbm_budget_bytes)
         return set_err(ctx, FL_OOM_ADMISSION, "workspace of %zu bytes exceeds the HBM budget",
                        w->pool_bytes);
-    CU(cudaMalloc(&w->pool, w->pool_bytes));
-    CU(cudaMalloc(&w->d_desc, sizeof(SlotDesc) * B));
-    CU(cudaMalloc(&w->d_state, sizeof(SlotState) * B));
-    CU(cudaMalloc(&w->d_active, sizeof(int) * B));
+    CU(block_alloc(w->blocks, &w->pool, w->pool_bytes));
+    CU(block_alloc(w->blocks, &w->d_desc, sizeof(SlotDesc) * B));
+    CU(block_alloc(w->blocks, &w->d_state, sizeof(SlotState) * B));
+    CU(block_alloc(w->blocks, &w->d_active, sizeof(int) * B));
     char* p = w->pool;
     w->d_zsave = (double*)carve(p, 8 * (size_t)std::max(nsave, 1));
     w->d_mask = (unsigned char*)carve(p, nt);
@@ -428,40 +524,43 @@ int check_problem(fl_problem* pr) {
     return FL_OK;
 }
 
-template <typename R>
-int upload_table_set(fl_problem* pr, const double* hR, const double* ss, int q) {
+// The spectral tables in both precisions (the adjoint is FP64 in every mode):
+// one block, one copy
+int upload_tables(fl_problem* pr, const double* D, const double* hR, const double* ss) {
     fl_ctx* ctx = pr->ctx;
-    const int nt = pr->nt;
-    std::vector<R> heff(2 * (size_t)nt), ssv(nt);
-    for (int k = 0; k < nt; k++) {
-        const double sg = (k & 1) ? -1.0 : 1.0;  // fftshift folded into the response
-        heff[2 * k] = (R)(hR[2 * k] * sg);
-        heff[2 * k + 1] = (R)(hR[2 * k + 1] * sg);
-        ssv[k] = (R)ss[k];
+    const size_t nt = pr->nt, nd = nt * pr->m;
+    auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
+    const size_t heff[2] = {al(8 * nd), al(8 * nd) + al(8 * nt)};
+    const size_t ssv[2] = {heff[1] + al(16 * nt), heff[1] + al(16 * nt) + al(4 * nt)};
+    const size_t host = ssv[1] + al(8 * nt);  // the twiddles follow, formed on the device
+    CU(block_alloc(pr->blocks, &pr->d_tables, host + al(8 * nt) + al(16 * nt)));
+    std::vector<char> img(host);
+    double* dturn = reinterpret_cast<double*>(img.data());
+    for (size_t i = 0; i < nd; i++) dturn[i] = D[i] / (2.0 * M_PI);
+    auto fill = [&](auto* h, auto* s) {
+        using R = std::remove_pointer_t<decltype(h)>;
+        for (size_t k = 0; k < nt; k++) {
+            const double sg = (k & 1) ? -1.0 : 1.0;  // fftshift folded into the response
+            h[2 * k] = (R)(hR[2 * k] * sg);
+            h[2 * k + 1] = (R)(hR[2 * k + 1] * sg);
+            s[k] = (R)ss[k];
+        }
+    };
+    fill(reinterpret_cast<float*>(&img[heff[0]]), reinterpret_cast<float*>(&img[ssv[0]]));
+    fill(reinterpret_cast<double*>(&img[heff[1]]), reinterpret_cast<double*>(&img[ssv[1]]));
+    pr->d_Dturns = reinterpret_cast<double*>(pr->d_tables);
+    for (int q = 0; q < 2; q++) {
+        pr->d_Heff[q] = pr->d_tables + heff[q];
+        pr->d_ss[q] = pr->d_tables + ssv[q];
+        pr->d_tw[q] = pr->d_tables + host + (q ? al(8 * nt) : 0);
     }
-    CU(cudaMalloc(&pr->d_Heff[q], sizeof(R) * heff.size()));
-    CU(cudaMalloc(&pr->d_ss[q], sizeof(R) * ssv.size()));
-    CU(cudaMalloc(&pr->d_tw[q], 2 * sizeof(R) * nt));
-    CU(cudaMemcpy(pr->d_Heff[q], heff.data(), sizeof(R) * heff.size(), cudaMemcpyHostToDevice));
-    CU(cudaMemcpy(pr->d_ss[q], ssv.data(), sizeof(R) * ssv.size(), cudaMemcpyHostToDevice));
-    twiddle_kernel<R><<<(nt + 255) / 256, 256>>>(static_cast<R*>(pr->d_tw[q]), nt);
+    CU(cudaMemcpy(pr->d_tables, img.data(), host, cudaMemcpyHostToDevice));
+    const int blocks = (int)((nt + 255) / 256);
+    twiddle_kernel<float><<<blocks, 256>>>(static_cast<float*>(pr->d_tw[0]), pr->nt);
+    twiddle_kernel<double><<<blocks, 256>>>(static_cast<double*>(pr->d_tw[1]), pr->nt);
     CU(cudaGetLastError());
     CU(cudaStreamSynchronize(0));
     return FL_OK;
-}
-
-// both precisions of the spectral tables (the adjoint is FP64 in every mode)
-int upload_tables(fl_problem* pr, const double* D, const double* hR, const double* ss) {
-    fl_ctx* ctx = pr->ctx;
-    const int nt = pr->nt, m = pr->m;
-    std::vector<double> dturn((size_t)nt * m);
-    for (size_t i = 0; i < dturn.size(); i++) dturn[i] = D[i] / (2.0 * M_PI);
-    CU(cudaMalloc(&pr->d_Dturns, sizeof(double) * dturn.size()));
-    CU(cudaMemcpy(pr->d_Dturns, dturn.data(), sizeof(double) * dturn.size(),
-                  cudaMemcpyHostToDevice));
-    int rc = upload_table_set<float>(pr, hR, ss, 0);
-    if (rc) return rc;
-    return upload_table_set<double>(pr, hR, ss, 1);
 }
 
 int status_of_slots(fl_ctx* ctx, const std::vector<SlotState>& st) {
@@ -500,6 +599,7 @@ int set_mode(fl_ctx* ctx, Work* w, int mode, int log_cost, int objective = OBJ_R
 // Per-batch multimode workspace, carved like Work.
 struct MmWork {
     fl_ctx* ctx = nullptr;
+    std::shared_ptr<BlockCache> blocks;  // a server chunk (its own stream) has its own
     int B = 0, nt = 0, m = 0, np = 0, K = 0, segcap = 0, stepcap = 0, nsave = 0;
     int per_mode = 0;
     char* pool = nullptr;
@@ -525,11 +625,8 @@ struct MmWork {
 
     ~MmWork() {
         if (graph) cudaGraphExecDestroy(graph);
-        cudaFree(pool);
-        cudaFree(d_desc);
-        cudaFree(d_state);
-        cudaFree(d_active);
-        cudaFree(d_ndone);
+        for (void* p : {(void*)pool, d_desc, (void*)d_state, (void*)d_active, (void*)d_ndone})
+            blocks->release(p);
         cudaFreeHost(h_ndone);
     }
 };
@@ -557,6 +654,7 @@ int mm_work_create(fl_problem* pr, int B, int nsave, int mode, int per_mode, MmW
     const size_t rf = pr->precision == FL_PRECISION_FP64 ? 8 : 4;
     auto w = std::make_unique<MmWork>();
     w->ctx = ctx;
+    w->blocks = opt ? closed_blocks() : ctx->blocks;
     w->B = B;
     w->nt = pr->nt;
     w->m = pr->m;
@@ -574,11 +672,11 @@ int mm_work_create(fl_problem* pr, int B, int nsave, int mode, int per_mode, MmW
     if (o.hbm_budget_bytes && w->pool_bytes > o.hbm_budget_bytes)
         return set_err(ctx, FL_OOM_ADMISSION, "workspace of %zu bytes exceeds the HBM budget",
                        w->pool_bytes);
-    CU(cudaMalloc(&w->pool, w->pool_bytes));
-    CU(cudaMalloc(&w->d_desc, sizeof(MmDesc) * B));
-    CU(cudaMalloc(&w->d_state, sizeof(MmState) * B));
-    CU(cudaMalloc(&w->d_active, sizeof(int) * B));
-    CU(cudaMalloc(&w->d_ndone, sizeof(int)));
+    CU(block_alloc(w->blocks, &w->pool, w->pool_bytes));
+    CU(block_alloc(w->blocks, &w->d_desc, sizeof(MmDesc) * B));
+    CU(block_alloc(w->blocks, &w->d_state, sizeof(MmState) * B));
+    CU(block_alloc(w->blocks, &w->d_active, sizeof(int) * B));
+    CU(block_alloc(w->blocks, &w->d_ndone, sizeof(int)));
     CU(cudaMallocHost(&w->h_ndone, sizeof(int)));
     char* p = w->pool;
     w->d_zsave = (double*)carve(p, 8 * (size_t)std::max(nsave, 1));
@@ -882,7 +980,7 @@ std::vector<unsigned char> tc_image(int rows, int K, F&& f) {
 }
 
 int upload_image(fl_ctx* ctx, const std::vector<unsigned char>& img, float** dst) {
-    CU(cudaMalloc(dst, img.size()));
+    CU(block_alloc(ctx->blocks, dst, img.size()));
     CU(cudaMemcpy(*dst, img.data(), img.size(), cudaMemcpyHostToDevice));
     return FL_OK;
 }
@@ -955,9 +1053,9 @@ int mm_upload_G(fl_problem* pr, const double* gamma) {
                     Ga[((size_t)j * NP + q) * MP + i] = v;
                 }
         }
-    CU(cudaMalloc(&pr->d_G[0], sizeof(float) * Gf.size()));
-    CU(cudaMalloc(&pr->d_G[1], sizeof(double) * G.size()));
-    CU(cudaMalloc(&pr->d_Ga, sizeof(double) * Ga.size()));
+    CU(block_alloc(pr->blocks, &pr->d_G[0], sizeof(float) * Gf.size()));
+    CU(block_alloc(pr->blocks, &pr->d_G[1], sizeof(double) * G.size()));
+    CU(block_alloc(pr->blocks, &pr->d_Ga, sizeof(double) * Ga.size()));
     CU(cudaMemcpy(pr->d_G[0], Gf.data(), sizeof(float) * Gf.size(), cudaMemcpyHostToDevice));
     CU(cudaMemcpy(pr->d_G[1], G.data(), sizeof(double) * G.size(), cudaMemcpyHostToDevice));
     CU(cudaMemcpy(pr->d_Ga, Ga.data(), sizeof(double) * Ga.size(), cudaMemcpyHostToDevice));
@@ -984,7 +1082,7 @@ int mm_upload_G(fl_problem* pr, const double* gamma) {
                 memcpy(&img[off], &hi, 4);
                 memcpy(&img[bbytes + off], &lo, 4);
             }
-        CU(cudaMalloc(&pr->d_Gtc, img.size()));
+        CU(block_alloc(pr->blocks, &pr->d_Gtc, img.size()));
         CU(cudaMemcpy(pr->d_Gtc, img.data(), img.size(), cudaMemcpyHostToDevice));
         // the symmetric B operand of the adjoint contractions: row p holds
         // G[i][j][.] = G[j][i][.] for the pairs p = (i <= j) (rows padded to
@@ -1002,7 +1100,7 @@ int mm_upload_G(fl_problem* pr, const double* gamma) {
                     memcpy(&aimg[off], &hi, 4);
                     memcpy(&aimg[abytes + off], &lo, 4);
                 }
-        CU(cudaMalloc(&pr->d_Gtcs, aimg.size()));
+        CU(block_alloc(pr->blocks, &pr->d_Gtcs, aimg.size()));
         CU(cudaMemcpy(pr->d_Gtcs, aimg.data(), aimg.size(), cudaMemcpyHostToDevice));
         if (pr->gamma_sym && mm_adj_mixed(M, pr->nt, pr->precision == FL_PRECISION_FP64)) {
             const int rc = mm_lowrank_setup(pr, gamma);
@@ -1716,7 +1814,7 @@ int fl_ctx_create(int device, const fl_ctx_opts* opts, fl_ctx** out) {
         delete ctx;
         return FL_ECUDA;
     }
-    ctx->stream = ctx->own;
+    ctx->blocks->stream = ctx->stream = ctx->own;
     for (auto& e : ctx->ev)
         if (cudaEventCreate(&e) != cudaSuccess) {
             fl_ctx_destroy(ctx);
@@ -1730,6 +1828,7 @@ int fl_ctx_destroy(fl_ctx* ctx) {
     if (!ctx) return FL_EINVAL;
     for (auto& e : ctx->ev)
         if (e) cudaEventDestroy(e);
+    ctx->blocks->close();
     if (ctx->own) cudaStreamDestroy(ctx->own);
     delete ctx;
     return FL_OK;
@@ -1741,7 +1840,8 @@ int fl_ctx_set_stream(fl_ctx* ctx, void* stream) {
     // work already queued on the previous stream completes before the switch,
     // so the context's device buffers are never used by two streams at once
     CU(cudaStreamSynchronize(ctx->stream));
-    ctx->stream = stream ? static_cast<cudaStream_t>(stream) : ctx->own;
+    std::lock_guard<std::mutex> lk(ctx->blocks->mu);
+    ctx->blocks->stream = ctx->stream = stream ? static_cast<cudaStream_t>(stream) : ctx->own;
     return FL_OK;
 }
 
@@ -1793,6 +1893,7 @@ int fl_problem_create(fl_ctx* ctx, int nt, int m, const double* D, const double*
         return set_err(ctx, FL_EINVAL, "Raman response spectrum must be Hermitian");
     auto pr = std::make_unique<fl_problem>();
     pr->ctx = ctx;
+    pr->blocks = ctx->blocks;
     pr->nt = nt;
     pr->m = m;
     pr->precision = precision;
@@ -1836,22 +1937,17 @@ int fl_problem_destroy(fl_problem* pr) {
     if (!pr) return FL_EINVAL;
     delete pr->last;
     delete pr->mlast;
-    cudaFree(pr->d_stage);
-    cudaFree(pr->d_ev);
-    cudaFree(pr->d_G[0]);
-    cudaFree(pr->d_G[1]);
-    cudaFree(pr->d_Ga);
-    cudaFree(pr->d_Gtc);
-    cudaFree(pr->d_Gtcs);
-    cudaFree(pr->d_Vz);
-    cudaFree(pr->d_Utc);
-    cudaFree(pr->d_Utcs);
-    cudaFree(pr->d_Dturns);
-    for (int q = 0; q < 2; q++) {
-        cudaFree(pr->d_Heff[q]);
-        cudaFree(pr->d_ss[q]);
-        cudaFree(pr->d_tw[q]);
-    }
+    pr->blocks->release(pr->d_stage);
+    pr->blocks->release(pr->d_ev);
+    pr->blocks->release(pr->d_G[0]);
+    pr->blocks->release(pr->d_G[1]);
+    pr->blocks->release(pr->d_Ga);
+    pr->blocks->release(pr->d_Gtc);
+    pr->blocks->release(pr->d_Gtcs);
+    pr->blocks->release(pr->d_Vz);
+    pr->blocks->release(pr->d_Utc);
+    pr->blocks->release(pr->d_Utcs);
+    pr->blocks->release(pr->d_tables);
     delete pr;
     return FL_OK;
 }
@@ -2196,10 +2292,10 @@ int fl_forward_evidence(fl_problem* pr, int nsave, double* ev_out) {
     const size_t bytes = sizeof(double) * (size_t)nsave * (kEvFixed + M);
     if (bytes > pr->ev_bytes) {
         CU(cudaStreamSynchronize(ctx->stream));
-        cudaFree(pr->d_ev);
+        pr->blocks->release(pr->d_ev);
         pr->d_ev = nullptr;
         pr->ev_bytes = 0;
-        CU(cudaMalloc(&pr->d_ev, bytes));
+        CU(block_alloc(pr->blocks, &pr->d_ev, bytes));
         pr->ev_bytes = bytes;
     }
     EvidenceArgs a{pr->d_tw[1], static_cast<const double*>(pr->d_ss[1]), d_save, nsave, M, nt,
@@ -2369,10 +2465,10 @@ static int phase_gradient_host(fl_problem* pr, const double* u0, int nbatch,
     const size_t need = up256(16 * nm) + 2 * up256(8 * np) + up256(8 * (size_t)nbatch) + up256(nt);
     if (need > pr->stage_bytes) {
         CU(cudaStreamSynchronize(ctx->stream));
-        cudaFree(pr->d_stage);
+        pr->blocks->release(pr->d_stage);
         pr->d_stage = nullptr;
         pr->stage_bytes = 0;
-        CU(cudaMalloc(&pr->d_stage, need));
+        CU(block_alloc(pr->blocks, &pr->d_stage, need));
         pr->stage_bytes = need;
     }
     char* sp = pr->d_stage;

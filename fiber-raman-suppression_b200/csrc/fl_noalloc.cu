@@ -38,7 +38,7 @@ size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
 // Offsets of every region inside the scratch array for nt points.
 struct Layout {
-    size_t desc, state, active, dturns, heff, ss, tw, u0b, u1b, kf[7], scr0, scr1, esv, end;
+    size_t desc, state, active, dturns, heff, heff32, ss, tw, tw32, u0b, u1b, kf[7], scr0, scr1, esv, end;
     explicit Layout(int nt) {
         size_t p = 0;
         auto take = [&](size_t bytes) {
@@ -51,8 +51,10 @@ struct Layout {
         active = take(sizeof(int));
         dturns = take(8 * (size_t)nt);
         heff = take(16 * (size_t)nt);
+        heff32 = take(8 * (size_t)nt);
         ss = take(8 * (size_t)nt);
         tw = take(16 * (size_t)nt);
+        tw32 = take(8 * (size_t)nt);
         u0b = take(16 * (size_t)nt);
         u1b = take(16 * (size_t)nt);
         for (int i = 0; i < 7; i++) kf[i] = take(8 * (size_t)nt);
@@ -74,10 +76,13 @@ __global__ void noalloc_prepare(SlotDesc desc, unsigned char* base, Layout lay, 
         reinterpret_cast<double*>(base + lay.dturns)[i] = D[i] / (2.0 * M_PI);
         const double sg = (i & 1) ? -1.0 : 1.0;  // fftshift folded into the response
         reinterpret_cast<double2*>(base + lay.heff)[i] = make_double2(hR[2 * i] * sg, hR[2 * i + 1] * sg);
+        reinterpret_cast<float2*>(base + lay.heff32)[i] =
+            make_float2((float)(hR[2 * i] * sg), (float)(hR[2 * i + 1] * sg));
         reinterpret_cast<double*>(base + lay.ss)[i] = selfsteep[i];
         double s, c;
         sincospi(-2.0 * (double)i / (double)nt, &s, &c);
         reinterpret_cast<double2*>(base + lay.tw)[i] = make_double2(c, s);
+        reinterpret_cast<float2*>(base + lay.tw32)[i] = make_float2((float)c, (float)s);
     }
     if (i == 0) {
         *reinterpret_cast<SlotDesc*>(base + lay.desc) = desc;
@@ -150,8 +155,10 @@ extern "C" int fl_forward_noalloc(int device, int nt, const double* d_D, double 
 
     SlotDesc d{};
     d.Dturns = reinterpret_cast<const double*>(base + lay.dturns);
+    d.Heff[0] = base + lay.heff32;
     d.Heff[1] = base + lay.heff;
     d.ss[1] = base + lay.ss;
+    d.tw[0] = base + lay.tw32;
     d.tw[1] = base + lay.tw;
     d.gamma = gamma;
     d.one_m_fR = one_m_fR;

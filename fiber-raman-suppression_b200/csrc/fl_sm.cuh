@@ -23,9 +23,10 @@
 // complex conjugates of each other and combine into the single real
 // correlation of Y; h∗I and h̃⋆Y share one complex transform pair.
 //
-// Precision (FP32 mode, RF = float): states, phase arguments, transforms,
-// stage sums, error norm and reductions in FP64; the forward's stage vectors
-// and the dense interpolant are stored in RF (see SmSolver).  The adjoint
+// Precision (FP32 mode, RF = float): states, phase arguments, transforms of
+// the field, stage sums, error norm and reductions in FP64; the forward's
+// stage vectors and the dense interpolant are stored in RF, and on the grids
+// up to 2^11 its Raman convolution runs in RF (see SmSolver).  The adjoint
 // integration (the gradient accumulation along z) is FP64 throughout, stage
 // vectors included: an FP32 adjoint amplifies its round-off through the
 // modulation-instability gain of the anomalous-dispersion fiber and misses
@@ -206,8 +207,14 @@ template <typename RMAX, int LOGN, int C>
 struct SmShared {
     static constexpr size_t RED = XPlan<RMAX, RMAX, LOGN, C>::BYTES;
     static constexpr size_t TAB = RED + 64 * sizeof(double);
+    static constexpr size_t TAB32 = TAB + sizeof(cx<RMAX>) * XTables<RMAX, LOGN, C>::SIZE;
+    // FP64 arithmetic with E = 4 or 8: the tables of the forward's FP32
+    // transforms (SmSolver)
+    static constexpr bool BOTH =
+        sizeof(RMAX) == 8 && XShape<LOGN, C>::E >= 4 && XShape<LOGN, C>::SMALL;
+    using X32 = XTables<float, LOGN, C, x_loge(LOGN), true>;
     static constexpr size_t SLOT =
-        (TAB + sizeof(cx<RMAX>) * XTables<RMAX, LOGN, C>::SIZE + 15) & ~size_t(15);
+        (TAB32 + (BOTH ? sizeof(cx<float>) * X32::SIZE : 0) + 15) & ~size_t(15);
     // a cluster's CTAs hold tensor memory until their siblings finish: at
     // most one such CTA fits an SM, so that no two clusters wait for each
     // other's columns
@@ -222,7 +229,11 @@ __device__ __forceinline__ cx<R>* smem_tables(unsigned char* smraw) {
 // Fill the transform tables and wait for the group.
 template <typename R, int LOGN, int C>
 __device__ __forceinline__ void load_tables(const SlotDesc& d, unsigned char* smraw, int rank) {
+    using SH = SmShared<R, LOGN, C>;
     x_fill<R, LOGN, C>(smem_tables<R, LOGN, C>(smraw), (const cx<R>*)d.tw[sizeof(R) == 8], rank);
+    if constexpr (SH::BOTH)
+        x_fill<float, LOGN, C, x_loge(LOGN), true>(reinterpret_cast<cx<float>*>(smraw + SH::TAB32),
+                                                   (const cx<float>*)d.tw[0], rank);
     XForm<R, R, LOGN, C>::sync();
 }
 
@@ -475,6 +486,13 @@ struct SmSolver {
     using TMS = TmScratch<R, LOGN, CL>;
     static constexpr int VPC = TMS::VPC, CH = TMS::CH;
     static constexpr bool REGS = E == 2;  // slots in registers (2^6)
+    // The forward's Raman convolution in FP32: on the grids of 4 or 8 values
+    // per thread its two transforms are a third of an evaluation's FP64
+    // latency (one solve at Nt = 2^10: 3.2 -> 2.7 ms).  On the larger ones
+    // two more transform bodies cost more instruction fetch than they save
+    // arithmetic (forward body at 2^13 105 KB; one solve at 2^14 9.4 -> 12.1
+    // ms, 592 gradients at 2^13 unchanged).
+    static constexpr bool CONV32 = sizeof(K) < sizeof(R) && SmShared<R, LOGN, CL>::BOTH;
     static constexpr bool PHC = REGS || TM::template phasors<R>();  // phasors kept in a slot
     static constexpr int PHF = sizeof(R) == 8 || REGS ? 2 : 1;       // ... this one
 
@@ -558,6 +576,12 @@ struct SmSolver {
     //            f4: η -F⁻¹->
     __device__ __forceinline__ void transforms(const bool adj, C (&v)[E]) const {
         const R g = (R)d.gamma, ofr = (R)d.one_m_fR, invn = R(1) / R(N);
+        if constexpr (CONV32) {
+            if (!adj) {
+                forward32(v, g, ofr, invn);
+                return;
+            }
+        }
         const int nfft = adj ? 5 : 4;
 #pragma unroll 1
         for (int f = 0; f < nfft; f++) {
@@ -638,6 +662,39 @@ struct SmSolver {
             xf.transform(v, to_a, presync);
             if (inv) conj_all(v);
         }
+    }
+
+    // The forward with its Raman convolution (f1, f2) in FP32
+    __device__ __forceinline__ void forward32(C (&v)[E], const R g, const R ofr, const R invn) const {
+        using F = cx<float>;
+        const F* __restrict__ H = (const F*)d.Heff[0];
+        XForm<float, R, LOGN, CL> xc(
+            xf.sm, reinterpret_cast<const F*>(xf.sm + SmShared<R, LOGN, CL>::TAB32), xf.rank);
+        xf.transform(v, false, false);
+        put_all(0, v);
+        F w[E];
+#pragma unroll
+        for (int s = 0; s < E; s++) w[s] = mk((float)(g * abs2(v[s])), 0.f);
+        xc.flip = xf.flip;
+        xc.transform(w, true, false);
+#pragma unroll
+        for (int s = 0; s < E; s++) w[s] = conjc(cmul(w[s], H[bin(s)]));
+        xc.transform(w, false, false);  // real: its conjugate is not needed
+        xf.flip = xc.flip;
+#pragma unroll
+        for (int c = 0; c < CH; c++) {
+            C u[VPC];
+            get(0, c, u);
+#pragma unroll
+            for (int j = 0; j < VPC; j++) {
+                const int s = c * VPC + j;
+                // (which product the compiler fuses would depend on the instance)
+                const R fac = fma((R)w[s].re, invn, ofr * (g * abs2(u[j])));
+                v[s] = conjc(scale(u[j], fac));
+            }
+        }
+        xf.transform(v, true, false);
+        conj_all(v);
     }
 
     // ---- stage helpers ---------------------------------------------------

@@ -211,8 +211,9 @@ struct XPlan {
 // Twiddle tables in shared memory, filled once per kernel from the full
 // table W_N^k.  E >= 16: first-pass columns (FP32: two-level products
 // W^e = hi[e >> 6] lo[e & 63]; FP64: W_N^x, powers by products), second pass
-// (FP32: W_{N/16}^{lr}; FP64: W_{N/16}^l), W_32^i.
-template <typename R, int LOGN, int C, int LE = x_loge(LOGN)>
+// (FP32: W_{N/16}^{lr}; FP64: W_{N/16}^l), W_32^i.  LEAN: the FP32 transforms
+// of an FP64 solve, whose tables come on top.
+template <typename R, int LOGN, int C, int LE = x_loge(LOGN), bool LEAN = false>
 struct XTables {
     using S = XShape<LOGN, C, LE>;
     static constexpr bool F32 = sizeof(R) == 4;
@@ -223,12 +224,12 @@ struct XTables {
     static constexpr int N2 = S::SMALL ? 0 : (F32 ? R2 * S::L : S::L);
     static constexpr int N3 = !S::SMALL && S::L == 32 && S::E == 16 ? 16 : 0;
     // E <= 8: W_{E ns}^{m r}, m < ns, of each radix-E pass (ns = its stride)
-    // after the first pass, r = 1..E-1 (FP64 with E = 8: r = 1, the others by
+    // after the first pass, r = 1..E-1 (FP64 with E = 8 and LEAN: r = 1, the others by
     // products); a pass's table starts at (ns - FIRST) NR / (E - 1)
     static constexpr int RE = S::E < 4 ? 4 : S::E;
     static constexpr int LRE = RE == 4 ? 2 : 3;
     static constexpr int FIRST = LOGN % LRE ? 1 << (LOGN % LRE) : RE;
-    static constexpr int NR = !F32 && RE == 8 ? 1 : RE - 1;
+    static constexpr int NR = LEAN || (!F32 && RE == 8) ? 1 : RE - 1;
     static constexpr int SIZE = S::SMALL ? (S::N - FIRST) / (RE - 1) * NR : N1 + N2 + N3;
 };
 
@@ -261,10 +262,10 @@ __device__ __forceinline__ int x_owner(int x, int& half) {
     }
 }
 
-template <typename R, int LOGN, int C, int LE = x_loge(LOGN)>
+template <typename R, int LOGN, int C, int LE = x_loge(LOGN), bool LEAN = false>
 __device__ __forceinline__ void x_fill(cx<R>* dst, const cx<R>* __restrict__ full, int rank) {
     using S = XShape<LOGN, C, LE>;
-    using X = XTables<R, LOGN, C, LE>;
+    using X = XTables<R, LOGN, C, LE, LEAN>;
     if constexpr (S::SMALL) {
         for (int ns = X::FIRST; ns < S::N; ns *= X::RE)
             for (int i = threadIdx.x; i < X::NR * ns; i += S::TC)
@@ -285,14 +286,18 @@ __device__ __forceinline__ void x_fill(cx<R>* dst, const cx<R>* __restrict__ ful
     }
 }
 
-// One group's transform engine in precision R.
+// One group's transform engine in precision R.  An FP32 engine beside an FP64
+// one (RMAX) uses the same bytes for the same region, column buffer and flip
+// side, so transforms of both precisions may follow one another.
 template <typename R, typename RMAX, int LOGN, int C, int LE = x_loge(LOGN)>
 struct XForm {
     using S = XShape<LOGN, C, LE>;
     using P = XPlan<R, RMAX, LOGN, C, LE>;
-    using X = XTables<R, LOGN, C, LE>;
+    using X = XTables<R, LOGN, C, LE, (sizeof(R) < sizeof(RMAX))>;
     using V = cx<R>;
-    static constexpr int N = S::N, E = S::E, T = S::T, TC = S::TC, TT = S::TT, L = S::L, RS = S::RS;
+    static constexpr int N = S::N, E = S::E, T = S::T, TC = S::TC, TT = S::TT, L = S::L;
+    // region stride in elements, the larger precision's in bytes
+    static constexpr int RS = S::RS * (int)(P::ONEM / P::ONE);
 
     unsigned char* sm;        // the buffers
     const cx<R>* tab;         // XTables in shared memory
@@ -353,7 +358,7 @@ struct XForm {
     __device__ __forceinline__ void regions_to_columns(V (&v)[E]) const {
         const int q0 = g / L, l = g % L;
         if constexpr (C > 1) {
-            const uint32_t base = x_smem(sm + P::ONE);
+            const uint32_t base = x_smem(sm + P::ONEM);
 #pragma unroll
             for (int j = 0; j < E; j++) {
                 int half;
@@ -363,12 +368,12 @@ struct XForm {
                      v[j]);
             }
             sync();
-            const V* a = reinterpret_cast<const V*>(sm + P::ONE);
+            const V* a = reinterpret_cast<const V*>(sm + P::ONEM);
 #pragma unroll
             for (int s = 0; s < E; s++) v[s] = a[s * TC + threadIdx.x];
         } else {
             constexpr int PARTS = P::SPLIT ? 2 : 1;
-            constexpr int AB = P::TWO ? S::BUF : 0;  // the column buffer
+            constexpr int AB = P::TWO ? S::RS : 0;  // the column buffer: the regions' second halves
             V w[E];
 #pragma unroll
             for (int part = 0; part < PARTS; part++) {
@@ -481,7 +486,7 @@ struct XForm {
     // values, 2.3 ms with 256 threads of 4.
     static __device__ __forceinline__ int pad4(int i) { return i + (i >> (sizeof(R) == 8 ? 3 : 4)); }
     __device__ __forceinline__ V* flip_buffer() const {
-        V* b = reinterpret_cast<V*>(sm) + (flip ? S::BUF : 0);
+        V* b = reinterpret_cast<V*>(sm + (flip ? P::ONEM : 0));
         flip ^= 1;
         return b;
     }

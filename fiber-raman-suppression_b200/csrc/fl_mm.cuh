@@ -50,6 +50,11 @@ __host__ __device__ __forceinline__ bool mm_rhs_phase(int ph) {
     return ph == PH_FWD_INIT || ph == PH_FWD || ph == PH_REC || ph == PH_ADJ_INIT ||
            ph == PH_ADJ || ph == PH_EVAL_FWD || ph == PH_EVAL_ADJ;
 }
+// An adjoint step's last evaluation lies where the one before it did (c = 1,
+// the same attempt): u_t and the convolved products S' are still there.
+__host__ __device__ __forceinline__ bool mm_same_field(const MmState& st) {
+    return st.phase == PH_ADJ && st.stage == 6;
+}
 // the pending evaluation of this slot runs in precision R
 template <typename R>
 __device__ __forceinline__ bool mm_takes(const MmDesc& d, const MmState& st) {
@@ -361,7 +366,7 @@ __device__ __forceinline__ void mm_prologue(MmGroup<R, LOGN, LOGE, CL>& grp, con
         grp.to_time(v);
 #pragma unroll
         for (int s = 0; s < E; s++) out[off + grp.own(s)] = v[s];
-        if (!adj || d.adj_mixed) return;  // (mixed: the FP32 kernel takes the forward field)
+        if (!adj || d.adj_mixed || mm_same_field(st)) return;  // (mixed: the FP32 kernel takes the forward field)
     }
 
     // ---- adjoint: the forward field at ezload, F(e^{iDz} ũ(z))
@@ -418,7 +423,8 @@ __global__ void __launch_bounds__(MmTasks<MIX, LOGN, LOGE, CL>::T, MmTasks<MIX, 
         [&](const MmState& st) {
             if (!mm_rhs_phase(st.phase)) return 0;
             const bool adj = mm_adjoint_phase(st.phase);
-            if (field) return adj && d.adj_mixed && unit < 2 * d.M ? 4 : 0;
+            if (field)
+                return adj && d.adj_mixed && unit < 2 * d.M && !mm_same_field(st) ? 4 : 0;
             return adj || d.fp64 ? 8 : 4;
         },
         [&](auto& grp, const MmState& st) { mm_prologue(grp, d, st, field ? unit - d.M : unit, field); });
@@ -532,7 +538,7 @@ __global__ void __launch_bounds__(MmTasks<MIX, LOGN, LOGE, CL>::T, MmTasks<MIX, 
             const bool adj = mm_adjoint_phase(st.phase);
             const int ntp = (d.NP + 1) / 2;
             const bool ytask = unit >= ntp;
-            if (ytask && !adj) return 0;
+            if (ytask ? !adj : mm_same_field(st)) return 0;
             if (2 * (ytask ? unit - ntp : unit) >= (d.rank > 0 ? d.rank : d.NP)) return 0;
             return d.fp64 || ytask || (adj && !d.adj_mixed) ? 8 : 4;
         },

@@ -40,14 +40,6 @@ int mm_cluster_ctas(int logn) { return logn == 15 ? 4 : 1; }
 
 bool mm_supported_modes(int M) { return M >= 2 && M <= 10; }
 
-int mm_round_kernels(const MmRound& a) {
-    const bool mixed = mm_adj_mixed(a.M, a.N, a.fp64);
-    int n = 4 + (a.control ? 1 : 0);  // prologue, pairs, forward contraction, epilogue
-    if (mixed && a.lowrank_some) n++;
-    if (a.adjoint) n += 1 + (!mixed || a.fullrank_some ? 1 : 0);
-    return n;
-}
-
 __global__ void __launch_bounds__(kMmCtl)
     mm_control_kernel(const MmDesc* __restrict__ descs, MmState* states,
                       const int* __restrict__ active, int consume, int* __restrict__ ndone) {
@@ -110,6 +102,23 @@ __global__ void __launch_bounds__(kTcRows, 2)
     const MmState st = states[slot];
     if (!mm_takes<double>(d, st) || !mm_adjoint_phase(st.phase)) return;
     mm_contract_adj_tc<M>(d, blockIdx.x, tc_smem);
+}
+
+// Both in one launch: each CTA takes its slot's contraction (mm_one_contraction).
+template <int M>
+__global__ void __launch_bounds__(kTcRows, 2)
+    mm_contract_both_tc_kernel(const MmDesc* __restrict__ descs, const MmState* states,
+                               const int* __restrict__ active) {
+    extern __shared__ __align__(16) unsigned char tc_smem[];
+    mm_chain_start();
+    const int slot = active[blockIdx.y];
+    const MmDesc& d = descs[slot];
+    mm_chain_wait();
+    if (d.M != M || !d.adj_mixed) return;
+    const MmState st = states[slot];
+    if (!mm_rhs_phase(st.phase)) return;
+    if (mm_adjoint_phase(st.phase)) mm_contract_adj_tc<M>(d, blockIdx.x, tc_smem);
+    else mm_contract_fwd_tc<M>(d, blockIdx.x, gridDim.x, tc_smem);
 }
 
 // The adjoint's Im X contraction of FP32-forward batches on the tensor
@@ -195,6 +204,29 @@ cudaError_t contract_tc(const MmRound& a) {
                            static_cast<const MmState*>(a.state), a.active);
 }
 
+// Forward and adjoint contraction of a mixed batch in one launch from 9 modes
+// on, where both hold half an SM's shared memory.  Apart, each costs the other's
+// rounds a launch of empty CTAs (64 x 10 modes at 2^14: 75 us of a forward
+// round of 1.05 ms, 120 us of an adjoint one of 2.7 ms; the gradient 484 ->
+// 469 ms).  With fewer modes the forward contraction alone fits three to six
+// CTAs per SM, and in the chain of a small launch the empty kernel costs
+// nothing measurable (6 modes, one slot: 21.7 ms either way).
+bool mm_one_contraction(const MmRound& a) {
+    return a.adjoint && a.tensor_cores && a.M >= 9 && mm_adj_mixed(a.M, a.N, a.fp64);
+}
+
+template <int M>
+cudaError_t contract_both_tc(const MmRound& a) {
+    const size_t smem = TcShape<M>::SMEM > TcSymShape<M>::SMEM_LAUNCH ? TcShape<M>::SMEM
+                                                                      : TcSymShape<M>::SMEM_LAUNCH;
+    cudaError_t e = cudaFuncSetAttribute(mm_contract_both_tc_kernel<M>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    return mm_chain_launch(mm_contract_both_tc_kernel<M>, dim3(a.N / kTcRows, a.nactive), kTcRows,
+                           smem, a.stream, 1, true, static_cast<const MmDesc*>(a.desc),
+                           static_cast<const MmState*>(a.state), a.active);
+}
+
 template <typename R, int M>
 cudaError_t contract_m(const MmRound& a, int which) {
     // which = 3: the low-rank form's Z reduction (FP32 batches with M >= 6;
@@ -207,11 +239,15 @@ cudaError_t contract_m(const MmRound& a, int which) {
     }
     // FP32 forward with M >= 6 modes: tensor cores (3xTF32)
     if constexpr (sizeof(R) == 4 && M >= 6) {
+        if constexpr (M >= 9) {
+            if (which == 0 && mm_one_contraction(a)) return contract_both_tc<M>(a);
+        }
         if (which == 0 && a.tensor_cores && a.N % kTcRows == 0) return contract_tc<M>(a);
     }
     // mixed-precision adjoint (mm_adj_mixed): the assembly's forward-field
     // contractions and the Im X contraction on the tensor cores (3xTF32)
     if constexpr (sizeof(R) == 8 && M >= 6) {
+        if (which == 2 && mm_one_contraction(a)) return cudaSuccess;
         if (which == 2 && mm_adj_mixed(M, a.N, a.fp64)) return contract_adj_tc<M>(a);
         if (which == 1 && mm_adj_mixed(M, a.N, a.fp64))
             return a.fullrank_some ? imx_tc<M>(a) : cudaSuccess;
@@ -252,6 +288,15 @@ cudaError_t mm_launch_contract(const MmRound& a, int which) {
 cudaError_t mm_launch_control(const MmRound& a, int consume) {
     return mm_chain_launch(mm_control_kernel, dim3(a.nactive), kMmCtl, 0, a.stream, 1, consume != 0,
                            static_cast<const MmDesc*>(a.desc), a.state, a.active, consume, a.ndone);
+}
+
+int mm_round_kernels(const MmRound& a) {
+    const bool mixed = mm_adj_mixed(a.M, a.N, a.fp64);
+    int n = 4 + (a.control ? 1 : 0);  // prologue, pairs, forward contraction, epilogue
+    if (mixed && a.lowrank_some) n++;
+    if (a.adjoint) n += 1 + (!mixed || a.fullrank_some ? 1 : 0);
+    if (mm_one_contraction(a)) n--;
+    return n;
 }
 
 }  // namespace fl

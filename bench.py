@@ -66,7 +66,7 @@ def cpu_model() -> str:
 
 
 def config(B, world, extra=None,
-           precision="FP32 bulk; FP64 phase/state/error norm/reductions; FP64 adjoint"):
+           precision="FP32 forward stages and interpolant; FP64 arithmetic; FP64 adjoint"):
     c = {"workload": f"single-mode inverse-design batch: Nt=2^13 over 10 ps, SMF-28, L=0.5 m, "
                      f"0.1 W/80 MHz 185 fs sech², phase N(0,0.5²), Raman band < -13 THz, "
                      f"fwd+adjoint, 32 z-checkpoints / 64 dense-output steps",

@@ -53,7 +53,9 @@ extern "C" {
                                 index left its buffer's bounds; the slot stopped before
                                 the access */
 
-/* FP32 bulk, FP64 phase/norm/reductions/state.  The single-mode adjoint runs
+/* FP32 bulk, FP64 phase/norm/reductions/state; single-mode solves keep only
+ * the stage vectors, the dense interpolant and (to Nt = 2^11) the Raman
+ * convolution in FP32 and compute in FP64.  The single-mode adjoint runs
  * in FP64; the multimode adjoint (M >= 6, Nt a multiple of 128) keeps λ and
  * its transforms in FP64 and takes the forward field's transform, pair
  * products and the per-point contractions at FP32 accuracy (3xTF32 tensor

@@ -621,7 +621,7 @@ def run_ours(args):
                 "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak,
                              "unit": "GB/s", "frac": achieved / peak, "traffic": traffic,
                              "peak_source": peak_kind,
-                             "kernel": "sm_advance_kernel<float,13,4>",
+                             "kernel": "sm_advance_kernel<float,double,13,1>",
                              "alg_bytes_per_launch": alg_bytes},
                 "cpu_baseline": cpu, "gpu_launches": int(launches), "clocks": clocks,
                 "plain_one_at_a_time": plain, "batched": batched_lat,

@@ -208,7 +208,7 @@ __global__ void __launch_bounds__(XShape<LOGN, 1>::T, 1)
                     st2(d.esv, b, mk(dt * er, dt * ei));
                     const double m0 = x0.re * x0.re + x0.im * x0.im;
                     const double m1 = u1.re * u1.re + u1.im * u1.im;
-                    d.skv[b] = at + sqrt_nb(fmax(m0, m1)) * rt;
+                    d.skv[b] = at + sqrt(fmax(m0, m1)) * rt;
                 }
             }
             if (st == 6) pnew = pps;

@@ -75,19 +75,22 @@ constexpr double kEps = 2.220446049250313e-16;
 // Square root and reciprocal without the library's branches (sixteen of
 // each per step sit on one warp's critical path, and a call in the slow path
 // keeps the compiler from interleaving them): the hardware's approximation
-// (about 2^-20) and two Newton steps each, error at most an ulp or two.
-// Subnormal arguments of the root count as zero.
+// (about 2^-20) and two Newton steps each.  The root's first step is coupled
+// (Goldschmidt's iteration: g -> sqrt(m), h -> 1 / (2 sqrt(m))), its second
+// adds the residual m - g g, so one rounding is left.
+// Both hold to an ulp where argument and result are normal numbers (measured
+// 0.50).  Outside: sqrt_nb of zero and of subnormal m is 0, rcp_nb above 2^1022 is
+// 0; infinity, and for rcp_nb zero and subnormal w, give no finite value, which
+// error_norm catches.
 __device__ __forceinline__ double sqrt_nb(double m) {
     double r;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(m));
     double g = m * r, h = 0.5 * r;
-#pragma unroll
-    for (int i = 0; i < 2; i++) {
-        const double e = fma(-g, h, 0.5);
-        g = fma(g, e, g);
-        h = fma(h, e, h);
-    }
-    return m < 2.3e-308 ? 0.0 : g;
+    const double e = fma(-g, h, 0.5);
+    g = fma(g, e, g);
+    h = fma(h, e, h);
+    g = fma(fma(-g, g, m), h, g);
+    return fabs(m) < 2.2250738585072014e-308 ? 0.0 : g;
 }
 __device__ __forceinline__ double rcp_nb(double w) {
     double r;
@@ -875,6 +878,23 @@ struct SmSolver {
                 const double ei = e6[i].im + dt * bt * (double)v[i].im;
                 acc += (er * er + ei * ei) * (w * w);
             }
+        }
+        return acc < INFINITY ? acc : error_norm_any(in, k);
+    }
+    // the same where a weight, a modulus or a square leaves the range above
+    // (tolerances below 1e-154, say): the library's root and quotient
+    __device__ __noinline__ double error_norm_any(const StageRun& in, const CK* k) const {
+        double acc = 0.0;
+#pragma unroll 1
+        for (int s = 0; s < E; s++) {
+            const int b = own(s);
+            const cx<double> e6 = ld2(d.esv, b), un = ld2(in.x, b), u1 = ld2(in.xnew, b);
+            const CK v = k[b];
+            const double m0 = un.re * un.re + un.im * un.im, m1 = u1.re * u1.re + u1.im * u1.im;
+            const double w = in.at + sqrt(fmax(m0, m1)) * in.rt;
+            const double er = (e6.re + in.dt * kT5bt[6] * (double)v.re) / w;
+            const double ei = (e6.im + in.dt * kT5bt[6] * (double)v.im) / w;
+            acc += er * er + ei * ei;
         }
         return acc;
     }

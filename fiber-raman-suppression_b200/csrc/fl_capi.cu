@@ -24,96 +24,16 @@
 #include <nvtx3/nvToolsExt.h>
 
 #include "../../include/fiberlab_gpu.h"
+#include "fl_blocks.h"
 #include "fl_launch.h"
 #include "fl_mm_launch.h"
 
 using namespace fl;
 
-// Device blocks of a context's problems and workspaces.  Mapping and unmapping
-// device memory is what a short call on a fresh problem used to wait for: of
-// 5.4 ms for a propagation at Nt = 2^12 with five save positions, 0.8 ms in
-// cudaMalloc and 0.8 ms in cudaFree, beside 3.5 ms of kernels.  Released
-// blocks are kept for the next object: at most kKeep bytes, given back with
-// the context, and before an allocation fails.  A block is reused only after
-// the context's stream has run dry, and by objects of the same context.
-struct BlockCache {
-    static constexpr size_t kKeep = size_t(256) << 20;
-    struct Block {
-        void* p;
-        size_t bytes;
-    };
-    std::mutex mu;
-    bool open = true;                // the context is alive
-    cudaStream_t stream = nullptr;   // its stream
-    std::vector<Block> live, spare;  // spare: oldest first
-    size_t kept = 0;
-
-    cudaError_t alloc(void** out, size_t bytes) {
-        std::lock_guard<std::mutex> lk(mu);
-        *out = nullptr;
-        bytes = (std::max<size_t>(bytes, 1) + 511) & ~size_t(511);
-        // the smallest spare block that wastes no more than half of itself
-        size_t best = spare.size();
-        for (size_t i = 0; i < spare.size(); i++)
-            if (spare[i].bytes >= bytes && spare[i].bytes <= 2 * bytes &&
-                (best == spare.size() || spare[i].bytes < spare[best].bytes))
-                best = i;
-        Block b{nullptr, bytes};
-        if (best < spare.size()) {
-            b = spare[best];
-            spare.erase(spare.begin() + best);
-            kept -= b.bytes;
-        } else {
-            cudaError_t e = cudaMalloc(&b.p, bytes);
-            if (e == cudaErrorMemoryAllocation && !spare.empty()) {
-                cudaGetLastError();
-                trim(0);
-                e = cudaMalloc(&b.p, bytes);
-            }
-            if (e != cudaSuccess) return e;
-        }
-        live.push_back(b);
-        *out = b.p;
-        return cudaSuccess;
-    }
-    void release(void* p) {
-        if (!p) return;
-        std::lock_guard<std::mutex> lk(mu);
-        for (size_t i = 0; i < live.size(); i++) {
-            if (live[i].p != p) continue;
-            const Block b = live[i];
-            live.erase(live.begin() + i);
-            if (!open || b.bytes > kKeep / 2 || cudaStreamSynchronize(stream) != cudaSuccess) {
-                cudaFree(p);
-                return;
-            }
-            spare.push_back(b);
-            kept += b.bytes;
-            trim(kKeep);
-            return;
-        }
-    }
-    void close() {
-        std::lock_guard<std::mutex> lk(mu);
-        open = false;
-        trim(0);
-    }
-
-private:
-    void trim(size_t limit) {
-        size_t n = 0;
-        while (kept > limit && n < spare.size()) {
-            kept -= spare[n].bytes;
-            cudaFree(spare[n++].p);
-        }
-        spare.erase(spare.begin(), spare.begin() + n);
-    }
-};
-
 struct fl_ctx {
     int device = 0;
     // shared with the objects that hold blocks (they may outlive the context)
-    std::shared_ptr<BlockCache> blocks = std::make_shared<BlockCache>();
+    std::shared_ptr<BlockCache> blocks;
     cudaStream_t stream = nullptr;  // the stream every call of this context runs on
     cudaStream_t own = nullptr;     // the context's private stream (the default for stream)
     std::string err;
@@ -149,10 +69,11 @@ int set_err(fl_ctx* c, int code, const char* fmt, ...) {
     return code;
 }
 
-// a cache that keeps nothing
-std::shared_ptr<BlockCache> closed_blocks() {
+// a cache that keeps nothing (objects on a stream of their own)
+std::shared_ptr<BlockCache> closed_blocks(const fl_ctx* ctx) {
     auto c = std::make_shared<BlockCache>();
     c->close();
+    c->set_lender(ctx->blocks);
     return c;
 }
 template <class T>
@@ -351,7 +272,7 @@ int work_create(fl_problem* pr, int B, int nsave, int mode, Work** out,
     cudaStream_t strm = opt ? stream : ctx->stream;
     auto w = std::make_unique<Work>();
     w->ctx = ctx;
-    w->blocks = opt ? closed_blocks() : ctx->blocks;
+    w->blocks = opt ? closed_blocks(ctx) : ctx->blocks;
     w->B = B;
     w->nt = pr->nt;
     w->rsize = (int)rf;
@@ -654,7 +575,7 @@ int mm_work_create(fl_problem* pr, int B, int nsave, int mode, int per_mode, MmW
     const size_t rf = pr->precision == FL_PRECISION_FP64 ? 8 : 4;
     auto w = std::make_unique<MmWork>();
     w->ctx = ctx;
-    w->blocks = opt ? closed_blocks() : ctx->blocks;
+    w->blocks = opt ? closed_blocks(ctx) : ctx->blocks;
     w->B = B;
     w->nt = pr->nt;
     w->m = pr->m;
@@ -1294,7 +1215,8 @@ struct SrvChunk {
     cudaEvent_t ev = nullptr;
     bool inflight = false;
     std::vector<SrvRequest*> slot;     // nullptr: free
-    unsigned char* d_masks = nullptr;  // per-slot band masks (B * Nt)
+    std::shared_ptr<BlockCache> blocks;  // of the masks
+    unsigned char* d_masks = nullptr;    // per-slot band masks (B * Nt)
     size_t bytes = 0;
     std::vector<SlotState> hs;
     std::vector<MmState> hms;
@@ -1303,7 +1225,7 @@ struct SrvChunk {
         if (graph) cudaGraphExecDestroy(graph);
         delete w;
         delete mw;
-        cudaFree(d_masks);
+        if (blocks) blocks->release(d_masks);
         if (ev) cudaEventDestroy(ev);
         if (stream) cudaStreamDestroy(stream);
     }
@@ -1394,7 +1316,8 @@ int srv_new_chunk(fl_server* sv, SrvBucket* b) {
     int rc = c->mm ? mm_work_create(b->tables, c->B, 0, MODE_FORWARD, 0, &c->mw, &o, c->stream)
                    : work_create(b->tables, c->B, 0, MODE_FORWARD, &c->w, &o, c->stream);
     if (rc) return rc;
-    CU(cudaMalloc(&c->d_masks, (size_t)c->B * b->nt));
+    c->blocks = closed_blocks(ctx);
+    CU(block_alloc(c->blocks, &c->d_masks, (size_t)c->B * b->nt));
     // every slot starts free (finished)
     if (c->mm) {
         std::vector<MmState> st(c->B);
@@ -1814,7 +1737,9 @@ int fl_ctx_create(int device, const fl_ctx_opts* opts, fl_ctx** out) {
         delete ctx;
         return FL_ECUDA;
     }
-    ctx->blocks->stream = ctx->stream = ctx->own;
+    ctx->stream = ctx->own;
+    ctx->blocks = std::make_shared<BlockCache>(ctx->opts.hbm_budget_bytes);
+    ctx->blocks->set_stream(ctx->own);
     for (auto& e : ctx->ev)
         if (cudaEventCreate(&e) != cudaSuccess) {
             fl_ctx_destroy(ctx);
@@ -1840,8 +1765,8 @@ int fl_ctx_set_stream(fl_ctx* ctx, void* stream) {
     // work already queued on the previous stream completes before the switch,
     // so the context's device buffers are never used by two streams at once
     CU(cudaStreamSynchronize(ctx->stream));
-    std::lock_guard<std::mutex> lk(ctx->blocks->mu);
-    ctx->blocks->stream = ctx->stream = stream ? static_cast<cudaStream_t>(stream) : ctx->own;
+    ctx->stream = stream ? static_cast<cudaStream_t>(stream) : ctx->own;
+    ctx->blocks->set_stream(ctx->stream);
     return FL_OK;
 }
 
@@ -2025,7 +1950,7 @@ int fl_forward_gain(fl_problem* pr, const fl_gain* gain, double pump_power, cons
                          al(8 * (size_t)nsave) + al(F * (size_t)nsave) + al(8 * (size_t)nsave) +
                          al(sizeof(GainDesc)) + al(sizeof(GainOut));
     char* pool = nullptr;
-    CU(cudaMalloc(&pool, bytes));
+    CU(block_alloc(pr->blocks, &pool, bytes));
     char* p = pool;
     auto take = [&](size_t n) { char* q = p; p += al(n); return q; };
     GainDesc hd;
@@ -2075,7 +2000,7 @@ int fl_forward_gain(fl_problem* pr, const fl_gain* gain, double pump_power, cons
     GainDesc* d_desc = (GainDesc*)take(sizeof(GainDesc));
     GainOut* d_out = (GainOut*)take(sizeof(GainOut));
     if ((size_t)(p - pool) > bytes) {
-        cudaFree(pool);
+        pr->blocks->release(pool);
         return set_err(ctx, FL_ECUDA, "internal: gain workspace overflow (%zu > %zu)",
                        (size_t)(p - pool), bytes);
     }
@@ -2100,7 +2025,7 @@ int fl_forward_gain(fl_problem* pr, const fl_gain* gain, double pump_power, cons
         e = cudaMemcpyAsync(out_pump, hd.pump_save, 8 * (size_t)nsave, cudaMemcpyDeviceToHost,
                             ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-    cudaFree(pool);
+    pr->blocks->release(pool);
     if (e != cudaSuccess) return set_err(ctx, FL_ECUDA, "gain propagation: %s", cudaGetErrorString(e));
     if (stats) {
         memset(stats, 0, sizeof *stats);

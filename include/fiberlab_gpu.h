@@ -68,7 +68,11 @@ typedef struct fl_problem fl_problem;
 typedef struct fl_server fl_server;
 
 typedef struct {
-    size_t hbm_budget_bytes;   /* 0: no limit beyond cudaMalloc */
+    size_t hbm_budget_bytes;   /* 0: no limit beyond cudaMalloc.  A workspace above it is
+                                  refused (FL_OOM_ADMISSION).  A context keeps the device
+                                  blocks of destroyed problems for later ones, up to 256 MiB
+                                  and, with a budget, to what its blocks in use leave of it;
+                                  they are freed before an allocation of the context fails */
     int checkpoints;           /* z-checkpoint slots K for the adjoint (power of 2, default 32) */
     int segment_steps;         /* dense-output steps kept (default 64).  A solve of at most
                                   segment_steps accepted steps keeps every step's interpolant

@@ -360,36 +360,6 @@ int work_create(fl_problem* pr, int B, int nsave, int mode, Work** out,
     return FL_OK;
 }
 
-// CTAs per slot for a launch of this many slots: the size whose waves take
-// the least time.  A C-CTA solve takes a fraction of a one-CTA solve (column
-// rel), and the clusters in flight are bounded by the SMs of a GPC: 74 of two
-// CTAs, 32 of four, 14 of eight on 148 SMs.  Measured per gradient batch
-// (ms, 0.3 m; 1 / 2 / 4 / 8 CTAs): Nt = 2^13, 8 slots 8.9 / 5.9 / 4.7 / 4.5,
-// 24 slots 9.0 / 6.0 / 4.8 / 8.7, 60 slots 9.6 / 6.5 / 9.5 / 17.7, 148 slots
-// 11.6 / 13.7 / 23 / 44; 2^12, 8 slots 4.9 / 4.2 / 4.0, 36 slots 5.4 / 4.6 /
-// 7.9; 2^14, 8 slots 23.8 / - / 9.1 / 8.1, 40 slots 26.6 / - / 18.5 / 24.1.
-int sm_cluster(const fl_ctx* ctx, int logn, int slots) {
-    static const struct {
-        int c, per148;
-        double rel[3];  // 2^12, 2^13, 2^14
-    } size[] = {{1, 148, {1.0, 1.0, 1.0}},
-                {2, 74, {0.86, 0.66, 1.0}},
-                {4, 32, {0.82, 0.54, 0.38}},
-                {8, 14, {1.0, 0.50, 0.34}}};
-    int best = 1;
-    double least = 1e300;
-    for (const auto& z : size) {
-        if (z.c > 1 && !sm_cluster_built(logn, z.c)) continue;
-        const int cap = std::max(1, z.per148 * ctx->sm_count / 148);
-        const double t = ((slots + cap - 1) / cap) * (z.c == 1 ? 1.0 : z.rel[logn - 12]);
-        if (t < least) {
-            least = t;
-            best = z.c;
-        }
-    }
-    return best;
-}
-
 int launch_slots(fl_ctx* ctx, fl_problem* pr, Work* w, int nactive, int max_evals) {
     const int logn = ilog2i(pr->nt);
     const int fp64 = pr->precision == FL_PRECISION_FP64;
@@ -398,7 +368,7 @@ int launch_slots(fl_ctx* ctx, fl_problem* pr, Work* w, int nactive, int max_eval
         return set_err(ctx, FL_EUNSUPPORTED, "Nt = 2^%d is not built for %s", logn,
                        fp64 ? "FP64" : "FP32");
     LaunchArgs a{w->d_desc, w->d_state, w->d_active, nactive, max_evals, ctx->stream};
-    a.cluster = sm_cluster(ctx, logn, nactive);
+    a.cluster = sm_cluster(ctx->sm_count, logn, nactive);
     CU(fn(a));
     ctx->launches++;
     return FL_OK;
@@ -1540,7 +1510,7 @@ int srv_launch(fl_server* sv, SrvBucket* b, SrvChunk* c) {
                            cudaMemcpyHostToDevice, c->stream));
         LaunchArgs a{c->w->d_desc, c->w->d_state, c->w->d_active, (int)act.size(),
                      sv->opts.evals_per_launch, c->stream};
-        a.cluster = sm_cluster(ctx, logn, all);
+        a.cluster = sm_cluster(ctx->sm_count, logn, all);
         CU(fn(a));
         sv->launches++;
     }

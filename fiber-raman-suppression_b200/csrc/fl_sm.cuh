@@ -1415,7 +1415,7 @@ __device__ __forceinline__ double init_after_f1(const Sol& S, const double* x0, 
 // so the FFT code exists once per precision in the kernel.
 // 128 registers per thread up to 2^12: 512 threads per SM
 constexpr int sm_min_ctas(int logn) {
-    return logn <= 7 ? 16 : logn <= 10 ? 1 << (11 - logn) : logn == 11 ? 2 : 1;
+    return logn <= 6 ? 8 : logn <= 7 ? 16 : logn <= 10 ? 1 << (11 - logn) : logn == 11 ? 2 : 1;
 }
 template <typename RF, typename RA, int LOGN, int CL>
 __global__ void __launch_bounds__(XShape<LOGN, CL>::TC, sm_min_ctas(LOGN))

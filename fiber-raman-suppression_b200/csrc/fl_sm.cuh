@@ -270,9 +270,10 @@ struct TmLayout {
     static constexpr int COLS = NEED <= 32 ? 32 : NEED <= 64 ? 64 : NEED <= 128 ? 128
                               : NEED <= 256 ? 256 : 512;
     // one CTA per problem: the grids whose registers admit no more CTAs per
-    // SM than the columns do (2^8: 8 of 64, 2^10: 4 of 128 columns, 2^11 and
-    // 2^12: 2 of 256, 2^13: 1), so an allocation never waits; clusters:
-    // always (one CTA per SM, SmShared)
+    // SM than the columns do (sm_min_ctas: 2^7 and 2^8 eight of 64 columns,
+    // 2^9 four of 64, 2^10 two of 128, 2^11 two of 256, 2^12 one of 256, 2^13
+    // one of 512), so an allocation waits for no CTA of its own kernel;
+    // clusters: always (one CTA per SM, SmShared)
     static constexpr bool ENABLED = NEED <= 512 && E >= 4 && (C > 1 || LOGN <= 13);
     static_assert(C == 1 || ENABLED, "clusters keep their scratch in tensor memory");
     template <typename R>
@@ -1413,12 +1414,19 @@ __device__ __forceinline__ double init_after_f1(const Sol& S, const double* x0, 
 // The state machine.  Each loop iteration performs at most one RHS
 // evaluation (forward in RF, adjoint in RA) plus the bookkeeping around it,
 // so the FFT code exists once per precision in the kernel.
-// 128 registers per thread up to 2^12: 512 threads per SM
-constexpr int sm_min_ctas(int logn) {
-    return logn <= 6 ? 8 : logn <= 7 ? 16 : logn <= 10 ? 1 << (11 - logn) : logn == 11 ? 2 : 1;
+// CTAs per SM the registers must admit: 128 per thread at 2^8..2^11 (512
+// threads per SM), up to 255 on the other grids of less than 512 threads.
+// FP64 stage vectors (wide) need more than 128 at 2^8 and 2^11, where the cap
+// spilled 700 to 1100 bytes per adjoint evaluation: 592 gradients 1.61 ->
+// 1.32 ms at 2^8 and 6.90 -> 5.81 at 2^11, one 1.26 -> 1.02 and 3.42 -> 2.20.
+// At 2^7 the tensor memory admits eight (TmLayout), so a cap for sixteen
+// bought nothing: 592 gradients 1.35 -> 1.07 ms without, one 1.09 -> 0.90.
+constexpr int sm_min_ctas(int logn, bool wide) {
+    return logn <= 7 ? 8 : logn == 8 && wide ? 4 : logn <= 10 ? 1 << (11 - logn)
+         : logn == 11 && !wide ? 2 : 1;
 }
 template <typename RF, typename RA, int LOGN, int CL>
-__global__ void __launch_bounds__(XShape<LOGN, CL>::TC, sm_min_ctas(LOGN))
+__global__ void __launch_bounds__(XShape<LOGN, CL>::TC, sm_min_ctas(LOGN, sizeof(RF) == 8))
     sm_advance_kernel(const SlotDesc* __restrict__ descs, SlotState* __restrict__ states,
                       const int* __restrict__ active, int max_evals) {
     using SolF = SmSolver<RA, RF, LOGN, CL>;
@@ -1426,6 +1434,9 @@ __global__ void __launch_bounds__(XShape<LOGN, CL>::TC, sm_min_ctas(LOGN))
     using CF = cx<RF>;
     using CA = cx<RA>;
     constexpr int N = SolF::N, E = SolF::E, T = SolF::XF::T;
+    static_assert(!TmLayout<LOGN, CL>::ENABLED || CL > 1 ||
+                      TmLayout<LOGN, CL>::COLS * sm_min_ctas(LOGN, sizeof(RF) == 8) <= 512,
+                  "a CTA that the registers admit finds its columns");
     extern __shared__ __align__(16) unsigned char smraw[];
     double* red = reinterpret_cast<double*>(smraw + SmShared<RA, LOGN, CL>::RED);
 

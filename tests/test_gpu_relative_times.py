@@ -29,3 +29,9 @@ def _evaluation_us(nt, precision="fp32", batch=1, L=0.1):
 @pytest.mark.parametrize("batch", [1, 148])
 def test_smallest_grid_against_the_next(gpu_ctx, precision, batch):
     assert _evaluation_us(64, precision, batch) < 1.15 * _evaluation_us(128, precision, batch)
+
+
+# FP64 stage vectors (more registers) against FP32 ones under the cap of 128
+@pytest.mark.parametrize("nt,batch", [(256, 592), (2048, 1), (2048, 148)])
+def test_double_precision_against_single(gpu_ctx, nt, batch):
+    assert _evaluation_us(nt, "fp64", batch) < 1.1 * _evaluation_us(nt, "fp32", batch)

@@ -80,8 +80,8 @@ constexpr double kEps = 2.220446049250313e-16;
 // adds the residual m - g g, so one rounding is left.
 // Both hold to an ulp where argument and result are normal numbers (measured
 // 0.50).  Outside: sqrt_nb of zero and of subnormal m is 0, rcp_nb above 2^1022 is
-// 0; infinity, and for rcp_nb zero and subnormal w, give no finite value, which
-// error_norm catches.
+// 0; infinity, and for rcp_nb zero and subnormal w, give no finite value, upon
+// which the attempt takes error_norm_any.
 __device__ __forceinline__ double sqrt_nb(double m) {
     double r;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(m));
@@ -880,23 +880,6 @@ struct SmSolver {
                 acc += (er * er + ei * ei) * (w * w);
             }
         }
-        return acc < INFINITY ? acc : error_norm_any(in, k);
-    }
-    // the same where a weight, a modulus or a square leaves the range above
-    // (tolerances below 1e-154, say): the library's root and quotient
-    __device__ __noinline__ double error_norm_any(const StageRun& in, const CK* k) const {
-        double acc = 0.0;
-#pragma unroll 1
-        for (int s = 0; s < E; s++) {
-            const int b = own(s);
-            const cx<double> e6 = ld2(d.esv, b), un = ld2(in.x, b), u1 = ld2(in.xnew, b);
-            const CK v = k[b];
-            const double m0 = un.re * un.re + un.im * un.im, m1 = u1.re * u1.re + u1.im * u1.im;
-            const double w = in.at + sqrt(fmax(m0, m1)) * in.rt;
-            const double er = (e6.re + in.dt * kT5bt[6] * (double)v.re) / w;
-            const double ei = (e6.im + in.dt * kT5bt[6] * (double)v.im) / w;
-            acc += er * er + ei * ei;
-        }
         return acc;
     }
 
@@ -1072,6 +1055,29 @@ struct SmSolver {
         return acc;
     }
 };
+
+// SmSolver::error_norm (K: its stage vectors, k7 the last) where a weight, a
+// modulus or a square leaves the range of the fast routines (tolerances below
+// 1e-154, say): the library's root and quotient.  Called where the fast sum is
+// not finite, out of the evaluations (a call in them costs registers there:
+// FP64 gradients at 2^9 and 2^10 1 to 4 %).
+template <typename K, class XF>
+__device__ __noinline__ double error_norm_any(const XF& xf, const SlotDesc& d, const StageRun& in) {
+    const cx<K>* k7 = (const cx<K>*)in.stage_vec(6);
+    double acc = 0.0;
+#pragma unroll 1
+    for (int s = 0; s < XF::E; s++) {
+        const int b = xf.own(s);
+        const cx<double> e6 = ld2(d.esv, b), un = ld2(in.x, b), u1 = ld2(in.xnew, b);
+        const cx<K> v = k7[b];
+        const double m0 = un.re * un.re + un.im * un.im, m1 = u1.re * u1.re + u1.im * u1.im;
+        const double w = in.at + sqrt(fmax(m0, m1)) * in.rt;
+        const double er = (e6.re + in.dt * kT5bt[6] * (double)v.re) / w;
+        const double ei = (e6.im + in.dt * kT5bt[6] * (double)v.im) / w;
+        acc += er * er + ei * ei;
+    }
+    return acc;
+}
 
 // PI controller: returns q and q11 (OrdinaryDiffEqCore stepsize_controller!)
 __device__ __forceinline__ double pi_q(double EEst, double qold, double& q11) {
@@ -1770,7 +1776,8 @@ __global__ void __launch_bounds__(XShape<LOGN, CL>::TC, sm_min_ctas(LOGN, sizeof
                 if (n + 1 >= sb.hi) st.phase = st.a_nf == 0 ? PH_ADJ_INIT : PH_ADJ;
                 continue;
             }
-            const double EEst = sqrt(sum(acc) / (double)N);
+            double EEst = sqrt(sum(acc) / (double)N);
+            if (!isfinite(EEst)) EEst = sqrt(sum(error_norm_any<RF>(SF.xf, d, in)) / (double)N);
             if (!isfinite(EEst)) {
                 st.status = ST_NONFINITE;
                 st.phase = PH_DONE;
@@ -1896,7 +1903,8 @@ __global__ void __launch_bounds__(XShape<LOGN, CL>::TC, sm_min_ctas(LOGN, sizeof
             st.stage = 0;
             const double z = st.cz, dt = st.cdt;
             const double zlo = d.steplog[2 * sub_segment(d, st).lo];
-            const double EEst = sqrt(sum(acc) / (double)N);
+            double EEst = sqrt(sum(acc) / (double)N);
+            if (!isfinite(EEst)) EEst = sqrt(sum(error_norm_any<RA>(SF.xf, d, in)) / (double)N);
             if (!isfinite(EEst)) {
                 st.status = ST_NONFINITE;
                 st.phase = PH_DONE;

@@ -79,9 +79,9 @@ constexpr double kEps = 2.220446049250313e-16;
 // (Goldschmidt's iteration: g -> sqrt(m), h -> 1 / (2 sqrt(m))), its second
 // adds the residual m - g g, so one rounding is left.
 // Both hold to an ulp where argument and result are normal numbers (measured
-// 0.50).  Outside: sqrt_nb of zero and of subnormal m is 0, rcp_nb above 2^1022 is
-// 0; infinity, and for rcp_nb zero and subnormal w, give no finite value, upon
-// which the attempt takes error_norm_any.
+// 0.50).  Outside: sqrt_nb of zero and of subnormal m is 0, rcp_nb above 2^1022
+// is 0; infinity, and for rcp_nb zero and subnormal w, give no finite value (a
+// field whose square overflows has no finite derivative either).
 __device__ __forceinline__ double sqrt_nb(double m) {
     double r;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(m));
@@ -875,9 +875,10 @@ struct SmSolver {
                 const double m0 = un[i].re * un[i].re + un[i].im * un[i].im;
                 const double m1 = u1[i].re * u1[i].re + u1[i].im * u1[i].im;
                 const double w = rcp_nb(in.at + sqrt_nb(fmax(m0, m1)) * in.rt);
-                const double er = e6[i].re + dt * bt * (double)v[i].re;
-                const double ei = e6[i].im + dt * bt * (double)v[i].im;
-                acc += (er * er + ei * ei) * (w * w);
+                // (w * w would leave the range where the tolerances are below 1e-154)
+                const double er = (e6[i].re + dt * bt * (double)v[i].re) * w;
+                const double ei = (e6[i].im + dt * bt * (double)v[i].im) * w;
+                acc += er * er + ei * ei;
             }
         }
         return acc;
@@ -1055,29 +1056,6 @@ struct SmSolver {
         return acc;
     }
 };
-
-// SmSolver::error_norm (K: its stage vectors, k7 the last) where a weight, a
-// modulus or a square leaves the range of the fast routines (tolerances below
-// 1e-154, say): the library's root and quotient.  Called where the fast sum is
-// not finite, out of the evaluations (a call in them costs registers there:
-// FP64 gradients at 2^9 and 2^10 1 to 4 %).
-template <typename K, class XF>
-__device__ __noinline__ double error_norm_any(const XF& xf, const SlotDesc& d, const StageRun& in) {
-    const cx<K>* k7 = (const cx<K>*)in.stage_vec(6);
-    double acc = 0.0;
-#pragma unroll 1
-    for (int s = 0; s < XF::E; s++) {
-        const int b = xf.own(s);
-        const cx<double> e6 = ld2(d.esv, b), un = ld2(in.x, b), u1 = ld2(in.xnew, b);
-        const cx<K> v = k7[b];
-        const double m0 = un.re * un.re + un.im * un.im, m1 = u1.re * u1.re + u1.im * u1.im;
-        const double w = in.at + sqrt(fmax(m0, m1)) * in.rt;
-        const double er = (e6.re + in.dt * kT5bt[6] * (double)v.re) / w;
-        const double ei = (e6.im + in.dt * kT5bt[6] * (double)v.im) / w;
-        acc += er * er + ei * ei;
-    }
-    return acc;
-}
 
 // PI controller: returns q and q11 (OrdinaryDiffEqCore stepsize_controller!)
 __device__ __forceinline__ double pi_q(double EEst, double qold, double& q11) {
@@ -1776,8 +1754,7 @@ __global__ void __launch_bounds__(XShape<LOGN, CL>::TC, sm_min_ctas(LOGN, sizeof
                 if (n + 1 >= sb.hi) st.phase = st.a_nf == 0 ? PH_ADJ_INIT : PH_ADJ;
                 continue;
             }
-            double EEst = sqrt(sum(acc) / (double)N);
-            if (!isfinite(EEst)) EEst = sqrt(sum(error_norm_any<RF>(SF.xf, d, in)) / (double)N);
+            const double EEst = sqrt(sum(acc) / (double)N);
             if (!isfinite(EEst)) {
                 st.status = ST_NONFINITE;
                 st.phase = PH_DONE;
@@ -1903,8 +1880,7 @@ __global__ void __launch_bounds__(XShape<LOGN, CL>::TC, sm_min_ctas(LOGN, sizeof
             st.stage = 0;
             const double z = st.cz, dt = st.cdt;
             const double zlo = d.steplog[2 * sub_segment(d, st).lo];
-            double EEst = sqrt(sum(acc) / (double)N);
-            if (!isfinite(EEst)) EEst = sqrt(sum(error_norm_any<RA>(SF.xf, d, in)) / (double)N);
+            const double EEst = sqrt(sum(acc) / (double)N);
             if (!isfinite(EEst)) {
                 st.status = ST_NONFINITE;
                 st.phase = PH_DONE;

@@ -262,8 +262,12 @@ struct TmLayout {
     static constexpr int WARPS = T / 32;
     static constexpr int PER_Q = (WARPS + 3) / 4;      // warps sharing a lane quarter
     // FP64 fields (4 words per value); the third holds the evaluation's
-    // phasors where the columns of the CTAs that fit an SM allow it.
-    static constexpr int FIELDS = C > 1 || LOGN <= 11 ? 3 : 2;
+    // phasors where the columns of the CTAs that fit an SM allow it.  At 2^14
+    // one FP64 field on one CTA is the whole tensor memory: it takes slot 0
+    // (u_t, λ_t and, around the transforms, the phasors), slot 1 stays in
+    // global memory.  148 gradients there, 0.1 m: 16.9 ms with all of them in
+    // global memory (38 MB a field over the SMs), 12.9 so.
+    static constexpr int FIELDS = C > 1 || LOGN <= 11 ? 3 : LOGN <= 13 ? 2 : 1;
     static constexpr int COLS_WARP = FIELDS * 4 * E;
     static constexpr int NEED = COLS_WARP * PER_Q;
     // allocation: a power of two >= 32 columns
@@ -272,12 +276,12 @@ struct TmLayout {
     // one CTA per problem: the grids whose registers admit no more CTAs per
     // SM than the columns do (sm_min_ctas: 2^7 and 2^8 eight of 64 columns,
     // 2^9 four of 64, 2^10 two of 128, 2^11 two of 256, 2^12 one of 256, 2^13
-    // one of 512), so an allocation waits for no CTA of its own kernel;
+    // and 2^14 one of 512), so an allocation waits for no CTA of its own kernel;
     // clusters: always (one CTA per SM, SmShared)
-    static constexpr bool ENABLED = NEED <= 512 && E >= 4 && (C > 1 || LOGN <= 13);
+    static constexpr bool ENABLED = NEED <= 512 && E >= 4;
     static_assert(C == 1 || ENABLED, "clusters keep their scratch in tensor memory");
     template <typename R>
-    static constexpr bool phasors() { return ENABLED && (FIELDS == 3 || sizeof(R) == 4); }
+    static constexpr bool phasors() { return ENABLED && (FIELDS == 3 || (FIELDS == 2 && sizeof(R) == 4)); }
 };
 
 __device__ __forceinline__ void tm_st16(uint32_t a, const uint32_t (&r)[16]) {
@@ -524,7 +528,7 @@ struct SmSolver {
         if constexpr (REGS) {
 #pragma unroll
             for (int j = 0; j < VPC; j++) slot_[f][j] = v[j];
-        } else if (tmem()) {
+        } else if (f < TM::FIELDS && tmem()) {
             TMS(tm).put_chunk(f, c, v);
         } else {
             C* s = f ? scr1 : scr0;
@@ -536,7 +540,7 @@ struct SmSolver {
         if constexpr (REGS) {
 #pragma unroll
             for (int j = 0; j < VPC; j++) v[j] = slot_[f][j];
-        } else if (tmem()) {
+        } else if (f < TM::FIELDS && tmem()) {
             TMS(tm).get(f, c, v);
         } else {
             const C* s = f ? scr1 : scr0;
@@ -643,7 +647,7 @@ struct SmSolver {
 #pragma unroll
                 for (int c = 0; c < CH; c++) {
                     C l[VPC], u[VPC];
-                    if (tmem()) {
+                    if (TM::FIELDS > 1 && tmem()) {
                         TMS(tm).get2(c, l, u);
                     } else {
                         get(0, c, l);

@@ -1910,13 +1910,14 @@ int fl_forward_gain(fl_problem* pr, const fl_gain* gain, double pump_power, cons
     }
     if (!(nrm > 0)) return set_err(ctx, FL_EINVAL, "input spectrum must be nonzero");
     if (cudaSetDevice(ctx->device) != cudaSuccess) return set_err(ctx, FL_ENODEV, "cudaSetDevice");
-    // one device area: launch, two states, seven FP32 stages, the stage
-    // field and its gain term, two scratch fields, error partial and weights, output, gain tables, descriptor, result
+    // one device area: launch, two states, seven FP32 stages, a stage's gain
+    // term, two scratch fields, error partial and weights, output, gain
+    // tables, descriptor, result
     // (the size is the sum of the regions taken below, each rounded up to the
     // 256-byte alignment that take() gives it)
     const size_t F = 16 * (size_t)nt, H = 8 * (size_t)nt;
     auto al = [](size_t n) { return (n + 255) & ~size_t(255); };
-    const size_t bytes = 4 * al(F) + 9 * al(H) + 2 * al(F) + al(F) + al(H) + al(4 * H) +
+    const size_t bytes = 4 * al(F) + 8 * al(H) + 2 * al(F) + al(F) + al(H) + al(4 * H) +
                          al(8 * (size_t)nsave) + al(F * (size_t)nsave) + al(8 * (size_t)nsave) +
                          al(sizeof(GainDesc)) + al(sizeof(GainOut));
     char* pool = nullptr;
@@ -1943,7 +1944,6 @@ int fl_forward_gain(fl_problem* pr, const fl_gain* gain, double pump_power, cons
     d.u[1] = (double*)take(F);
     d.uL_out = (double*)take(F);
     for (int i = 0; i < 7; i++) d.kf[i] = take(H);
-    d.ka[0] = take(H);  // the stage field and its derivative
     d.ka[1] = take(H);  // the stage's gain term
     d.scr[0] = take(F);
     d.scr[1] = take(F);

@@ -6,12 +6,11 @@
 // 150-166), and the solver :204-239 (Tsit5 over the state [P; ũ]).
 //
 // One CTA integrates one problem to z = L in one launch.  The nonlinear term
-// is the single-mode stepper's forward right-hand side (its transforms, with
-// the field handed over through the shared transform buffer).  The gain of a
-// stage is computed from the stage input before that call: two block sums
+// is the single-mode stepper's forward right-hand side (its transforms).  The
+// gain of a stage is computed from the stage input before them: two block sums
 // give the rate-equation terms W12 and W21 of the stage's spectrum (|ũ|² =
 // |e^{iDz}ũ|²), the inversion n2 follows, and each thread keeps g_b ũ_b / 2
-// of its own bins in scratch and adds it to the returned derivative.  The
+// of its own bins in scratch and adds it to the derivative.  The
 // pump power and its seven stage derivatives are block-uniform FP64 scalars;
 // the RMS error norm runs over the Nt + 1 components of the state, as the
 // reference's does over [P; ũ].  FP32 right-hand side, FP64 state, stage
@@ -20,6 +19,110 @@
 #include "fl_sm.cuh"
 
 namespace fl {
+
+// One evaluation at z, the field in registers from the stage sum to the stored
+// derivative k[to]: the field is u + dt Σ_{j<n} a_j k_j (FP64 accumulation;
+// a_j the coefficients of stage n, or 1 for the probe), the pump power there
+// pp; stage 6 also leaves the new state in un, the partial error and the
+// weights.  Returns dP/dz.
+// Out of line: one body for the launch, the probe and the stages.  All loads
+// of a chunk of points are in flight for one stage vector after the other
+// (Nt = 2^12, 0.2 m, one solve: 2.07 ms with the stages inside the points and
+// the field handed over through global memory, 1.37 so; 2^13 2.96 and 2.09).
+template <int LOGN>
+__device__ __noinline__ double gain_eval(const GainDesc& g, unsigned char* smraw, double* red,
+                                         int& flip, int n, int to, bool probe, double z, double dt,
+                                         double pp, const double* u, double* un) {
+    using Sol = SmSolver<float, float, LOGN, 1>;
+    using CF = cx<float>;
+    constexpr int N = Sol::N, E = Sol::E, T = Sol::XF::T, SC = E < 8 ? E : 8;
+    const SlotDesc& d = g.s;
+    const Sol S(d, smraw, 0);
+    auto sum = [&](double v) { return x_reduce<T, 1, false>(v, red, flip, 0); };
+    CF v[E];
+#pragma unroll
+    for (int s0 = 0; s0 < E; s0 += SC) {
+        double ar[SC], ai[SC], er[SC], ei[SC];
+#pragma unroll
+        for (int c = 0; c < SC; c++) ar[c] = ai[c] = er[c] = ei[c] = 0.0;
+#pragma unroll 1
+        for (int j = 0; j < n; j++) {
+            const CF* kj = static_cast<const CF*>(d.kf[j]);
+            const double a = probe ? 1.0 : kT5a[n][j];
+            CF x[SC];
+#pragma unroll
+            for (int c = 0; c < SC; c++) x[c] = kj[S.own(s0 + c)];
+#pragma unroll
+            for (int c = 0; c < SC; c++) {
+                ar[c] += a * (double)x[c].re;
+                ai[c] += a * (double)x[c].im;
+            }
+            if (n == 6) {
+                const double bt = kT5bt[j];
+#pragma unroll
+                for (int c = 0; c < SC; c++) {
+                    er[c] += bt * (double)x[c].re;
+                    ei[c] += bt * (double)x[c].im;
+                }
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < SC; c++) {
+            const int b = S.own(s0 + c);
+            const cx<double> x0 = ld2(u, b);
+            const cx<double> u1 = mk(x0.re + dt * ar[c], x0.im + dt * ai[c]);
+            v[s0 + c] = down<float>(u1);
+            if (n == 6) {
+                st2(un, b, u1);
+                st2(d.esv, b, mk(dt * er[c], dt * ei[c]));
+                const double m0 = x0.re * x0.re + x0.im * x0.im;
+                const double m1 = u1.re * u1.re + u1.im * u1.im;
+                d.skv[b] = d.abstol + sqrt(fmax(m0, m1)) * d.reltol;
+            }
+        }
+    }
+    // g(ω)ũ/2, kept for the way out
+    CF* gb = static_cast<CF*>(d.ka[1]);
+    double gP = -1.0;
+    if (g.kind == 0) {
+#pragma unroll
+        for (int s = 0; s < E; s++) gb[S.own(s)] = scale(v[s], (float)(0.5 * g.g_const));
+    } else {
+        double w12 = 0.0, w21 = 0.0;
+#pragma unroll
+        for (int s = 0; s < E; s++) {
+            const int b = S.bin(s);
+            const double e = abs2(up(v[s]));
+            w12 += g.wa[b] * e;
+            w21 += g.we[b] * e;
+        }
+        w12 = sum(w12);
+        w21 = sum(w21);
+        const double r12 = g.r12c * pp, r21 = g.r21c * pp;
+        const double n2 = (r12 + w12) / (r12 + r21 + w12 + w21 + g.inv_tau), n1 = 1.0 - n2;
+#pragma unroll
+        for (int s = 0; s < E; s++) {
+            const int b = S.bin(s);
+            gb[S.own(s)] = scale(v[s], (float)(0.5 * (g.sE[b] * n2 - g.sA[b] * n1)));
+        }
+        gP = g.gpe * n2 - g.gpa * n1;
+    }
+#pragma unroll
+    for (int s = 0; s < E; s++) v[s] = cmul(v[s], phasor<float>(d.Dturns[S.bin(s)], z));
+    // (the run before may still be reading the first exchange buffer)
+    if constexpr (Sol::XF::S::SMALL) Sol::XF::sync();
+    S.transforms(false, v);
+    CF* out = static_cast<CF*>(d.kf[to]);
+    const float invn = 1.0f / N;
+#pragma unroll
+    for (int s = 0; s < E; s++) {
+        const int f = S.bin(s), b = S.own(s);
+        const CF y = cmulc(v[s], phasor<float>(d.Dturns[f], z));  // e^{-iDz} x
+        const float sc = S.ss[f] * invn;
+        out[b] = mk(-y.im * sc, y.re * sc) + gb[b];
+    }
+    return gP * pp;
+}
 
 template <int LOGN>
 __global__ void __launch_bounds__(XShape<LOGN, 1>::T, 1)
@@ -32,60 +135,17 @@ __global__ void __launch_bounds__(XShape<LOGN, 1>::T, 1)
     const GainDesc& g = *gdp;
     const SlotDesc& d = g.s;
     load_tables<float, LOGN, 1>(d, smraw, 0);
-    Sol S(d, smraw, 0);
+    const Sol S(d, smraw, 0);
     int flip = 0;
     auto sum = [&](double v) { return x_reduce<T, 1, false>(v, red, flip, 0); };
-    // the stage field, then its derivative (the thread's own bins)
-    struct {
-        CF* p;
-        const Sol& S;
-        __device__ CF& operator[](int s) const { return p[S.own(s)]; }
-    } const io{static_cast<CF*>(d.ka[0]), S};
-    CF* gb = static_cast<CF*>(d.ka[1]);  // g_b ũ_b / 2 of the current stage
     CF* k[7];
 #pragma unroll
     for (int i = 0; i < 7; i++) k[i] = static_cast<CF*>(d.kf[i]);
     double* u = d.u[0];
     double* un = d.u[1];
     const double L = d.L, dtmin = kEps * L, at = d.abstol, rt = d.reltol;
-
-    // g(ω)ũ/2 of the stage in io into gb (own bins); returns g_P
-    auto gain_of_stage = [&](double pp) -> double {
-        if (g.kind == 0) {
-#pragma unroll
-            for (int s = 0; s < E; s++) gb[S.own(s)] = scale(io[s], (float)(0.5 * g.g_const));
-            return -1.0;
-        }
-        double w12 = 0.0, w21 = 0.0;
-#pragma unroll
-        for (int s = 0; s < E; s++) {
-            const int b = S.bin(s);
-            const double e = abs2(up(io[s]));
-            w12 += g.wa[b] * e;
-            w21 += g.we[b] * e;
-        }
-        w12 = sum(w12);
-        w21 = sum(w21);
-        const double r12 = g.r12c * pp, r21 = g.r21c * pp;
-        const double n2 = (r12 + w12) / (r12 + r21 + w12 + w21 + g.inv_tau), n1 = 1.0 - n2;
-#pragma unroll
-        for (int s = 0; s < E; s++) {
-            const int b = S.bin(s);
-            gb[S.own(s)] = scale(io[s], (float)(0.5 * (g.sE[b] * n2 - g.sA[b] * n1)));
-        }
-        return g.gpe * n2 - g.gpa * n1;
-    };
-    // derivative of the stage (field in io, pump pp) at z: io <- dũ, returns dP
-    auto deriv = [&](double z, double pp) -> double {
-        const double gP = gain_of_stage(pp);
-        StageRun in{};
-        in.k1 = io.p;
-        in.out = io.p;
-        in.z = z;
-        rhs_fwd_call<float, float, LOGN, 1>(&d, smraw, 0, &in);
-#pragma unroll
-        for (int s = 0; s < E; s++) io[s] = io[s] + gb[S.own(s)];
-        return gP * pp;
+    auto eval = [&](int n, int to, bool probe, double z, double dt, double pp) -> double {
+        return gain_eval<LOGN>(g, smraw, red, flip, n, to, probe, z, dt, pp, u, un);
     };
 
     // ---- launch and f0
@@ -93,7 +153,6 @@ __global__ void __launch_bounds__(XShape<LOGN, 1>::T, 1)
     for (int s = 0; s < E; s++) {
         const cx<double> x = ld2(d.u0, S.bin(s));
         st2(u, S.own(s), x);
-        io[s] = down<float>(x);
     }
     double pp = g.pump0;
     // save positions at z = 0: the launch (the lab frame equals the interaction frame there)
@@ -108,10 +167,8 @@ __global__ void __launch_bounds__(XShape<LOGN, 1>::T, 1)
     long nf = 0, naccept = 0, nreject = 0;
     int status = ST_OK;
     double kp[7];
-    kp[0] = deriv(0.0, pp);
+    kp[0] = eval(0, 0, false, 0.0, 0.0, pp);
     nf++;
-#pragma unroll
-    for (int s = 0; s < E; s++) k[0][S.own(s)] = io[s];
 
     // ---- initial step (OrdinaryDiffEqCore ode_determine_initdt), P one more
     // component of the norms; weights from the launch
@@ -121,7 +178,7 @@ __global__ void __launch_bounds__(XShape<LOGN, 1>::T, 1)
     for (int s = 0; s < E; s++) {
         const cx<double> x = ld2(u, S.own(s));
         const double ax = sqrt(x.re * x.re + x.im * x.im), sk = at + ax * rt;
-        const double af = sqrt(abs2(up(io[s])));
+        const double af = sqrt(abs2(up(k[0][S.own(s)])));
         s0 += (ax / sk) * (ax / sk);
         s1 += (af / sk) * (af / sk);
     }
@@ -136,14 +193,7 @@ __global__ void __launch_bounds__(XShape<LOGN, 1>::T, 1)
         if (dt0 < 10.0 * kEps) {
             dt = fmax(1e-6, dtmin);
         } else {
-#pragma unroll
-            for (int s = 0; s < E; s++) {
-                const int b = S.own(s);
-                const cx<double> x = ld2(u, b);
-                const CF f0 = k[0][b];
-                io[s] = mk((float)(x.re + dt0 * (double)f0.re), (float)(x.im + dt0 * (double)f0.im));
-            }
-            const double kp1 = deriv(dt0, pp + dt0 * kp[0]);
+            const double kp1 = eval(1, 1, true, dt0, dt0, pp + dt0 * kp[0]);
             nf++;
             double s2 = 0.0, nd = 0.0;
 #pragma unroll
@@ -151,9 +201,9 @@ __global__ void __launch_bounds__(XShape<LOGN, 1>::T, 1)
                 const int b = S.own(s);
                 const cx<double> x = ld2(u, b);
                 const double sk = at + sqrt(x.re * x.re + x.im * x.im) * rt;
-                const CF f0 = k[0][b];
-                const double dr = (double)io[s].re - (double)f0.re;
-                const double di = (double)io[s].im - (double)f0.im;
+                const CF f0 = k[0][b], f1 = k[1][b];
+                const double dr = (double)f1.re - (double)f0.re;
+                const double di = (double)f1.im - (double)f0.im;
                 s2 += (dr * dr + di * di) / (sk * sk);
                 nd += (dr != 0.0 || di != 0.0) ? 1.0 : 0.0;
             }
@@ -187,35 +237,9 @@ __global__ void __launch_bounds__(XShape<LOGN, 1>::T, 1)
             double acc = 0.0;
             for (int j = 0; j < st; j++) acc += kT5a[st][j] * kp[j];
             const double pps = pp + dt * acc;
-            // stage input (FP64 accumulation) and, for stage 7, the new state,
-            // the partial error and the weights
-#pragma unroll 4
-            for (int s = 0; s < E; s++) {
-                const int b = S.own(s);
-                double ar = 0.0, ai = 0.0, er = 0.0, ei = 0.0;
-                for (int j = 0; j < st; j++) {
-                    const CF x = k[j][b];
-                    ar += kT5a[st][j] * (double)x.re;
-                    ai += kT5a[st][j] * (double)x.im;
-                    er += kT5bt[j] * (double)x.re;
-                    ei += kT5bt[j] * (double)x.im;
-                }
-                const cx<double> x0 = ld2(u, b);
-                const cx<double> u1 = mk(x0.re + dt * ar, x0.im + dt * ai);
-                io[s] = down<float>(u1);
-                if (st == 6) {
-                    st2(un, b, u1);
-                    st2(d.esv, b, mk(dt * er, dt * ei));
-                    const double m0 = x0.re * x0.re + x0.im * x0.im;
-                    const double m1 = u1.re * u1.re + u1.im * u1.im;
-                    d.skv[b] = at + sqrt(fmax(m0, m1)) * rt;
-                }
-            }
             if (st == 6) pnew = pps;
-            kp[st] = deriv(z + kT5c[st] * dt, pps);
+            kp[st] = eval(st, st, false, z + kT5c[st] * dt, dt, pps);
             nf++;
-#pragma unroll
-            for (int s = 0; s < E; s++) k[st][S.own(s)] = io[s];
         }
         // error dt Σ b̃_j k_j over the Nt + 1 components
         double acc = 0.0;
@@ -223,8 +247,9 @@ __global__ void __launch_bounds__(XShape<LOGN, 1>::T, 1)
         for (int s = 0; s < E; s++) {
             const int b = S.own(s);
             const cx<double> e6 = ld2(d.esv, b);
-            const double er = e6.re + dt * kT5bt[6] * (double)io[s].re;
-            const double ei = e6.im + dt * kT5bt[6] * (double)io[s].im;
+            const CF k6 = k[6][b];
+            const double er = e6.re + dt * kT5bt[6] * (double)k6.re;
+            const double ei = e6.im + dt * kT5bt[6] * (double)k6.im;
             const double w = d.skv[b];
             acc += (er * er + ei * ei) / (w * w);
         }
@@ -290,7 +315,7 @@ __global__ void __launch_bounds__(XShape<LOGN, 1>::T, 1)
         for (int s = 0; s < E; s++) {
             const int b = S.own(s);
             st2(u, b, ld2(un, b));
-            k[0][b] = io[s];
+            k[0][b] = k[6][b];
         }
         pp = pnew;
         kp[0] = kp[6];

@@ -156,7 +156,7 @@ struct MmGroup {
 // an FP32 batch (FP64 batches have no FP32 task).
 //
 // All kernels of a round form one chain of programmatic dependent launches:
-// each lets its successor start at once (mm_chain_start) and waits for its
+// each lets its successor start at once (mm_chain_start; see MmTasks::run) and waits for its
 // predecessor (mm_chain_wait) before it touches what the chain writes; every
 // thread waits, so a kernel's end implies the end of all before it.  Before
 // the wait only what the chain never writes is read: the active list, the
@@ -172,6 +172,7 @@ struct MmGroup {
 // saves the empty CTAs: 64 x 10 modes at 2^14, 560 -> 503 ms together with
 // the pair sequences read twice (mm_pairs).
 // ---------------------------------------------------------------------------
+constexpr unsigned kSms = 148;
 __device__ __forceinline__ void mm_chain_start() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
@@ -204,8 +205,14 @@ struct MmTasks {
               reinterpret_cast<double*>(smraw + RED));
         GF gf(smraw, reinterpret_cast<cx<float>*>(smraw + TABF),
               reinterpret_cast<double*>(smraw + RED));
-        const bool early = gridDim.x * gridDim.y <= 148;
-        mm_chain_start();
+        const bool early = gridDim.x * gridDim.y <= kSms;
+        // From 2^14 on a CTA fills an SM.  A successor that waits there from
+        // the start, and its own successors behind it, crowd the kernels
+        // between them onto fewer SMs, which costs more than the launches
+        // they hide: they start at this kernel's end (10 modes, FP64, one
+        // forward at 2^14 9.51 -> 8.88 ms, gradient 18.2 -> 17.5; 6 modes 6.45
+        // -> 6.36; below, 6 modes at 2^13 in FP32 2.45 so and 2.53 without).
+        if constexpr (LOGN < 14) mm_chain_start();
         if (early) {
             gd.fill(d);
             if constexpr (MIX) gf.fill(d);

@@ -681,7 +681,6 @@ MmRound mm_round_args(fl_problem* pr, MmWork* w, int nactive) {
     a.lowrank_some = pr->rank > 0;  // one problem per batch
     a.fullrank_some = pr->rank == 0;
     a.control = 1;
-    a.tensor_cores = 1;
     a.ndone = nullptr;
     a.stream = pr->ctx->stream;
     return a;
@@ -1465,7 +1464,6 @@ int srv_launch(fl_server* sv, SrvBucket* b, SrvChunk* c) {
         a.N = b->nt;
         a.fp64 = b->precision == FL_PRECISION_FP64;
         a.control = 1;
-        a.tensor_cores = 1;
         a.ndone = nullptr;
         a.stream = c->stream;
         MmRoundFn round = mm_round_launcher(logn);

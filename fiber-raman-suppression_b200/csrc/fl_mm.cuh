@@ -100,6 +100,9 @@ __device__ __forceinline__ void stcr(void* p, size_t i, cx<double> v, bool fp64)
 // field in frequency and, after to_time, element own(s) of a field in time:
 // time fields lie in the order the transforms leave them in, which every
 // kernel between two transforms shares (their work is pointwise in time).
+// 2^12 on 512 threads of 8 values (radix 8), where the single-mode stepper
+// takes 256 of 16: one gradient of 6 modes 1.95 ms for 2.60, 32 of 6 modes
+// 5.70 for 5.78, 32 of 10 modes 10.2 for 10.1 and in FP64 24.2 for 25.7.
 __host__ __device__ constexpr int mm_loge(int logn) { return logn == 12 ? 3 : x_loge(logn); }
 template <typename R, int LOGN, int LOGE, int C>
 struct MmGroup {
@@ -156,12 +159,12 @@ struct MmGroup {
 // an FP32 batch (FP64 batches have no FP32 task).
 //
 // All kernels of a round form one chain of programmatic dependent launches:
-// each lets its successor start at once (mm_chain_start; see MmTasks::run) and waits for its
-// predecessor (mm_chain_wait) before it touches what the chain writes; every
-// thread waits, so a kernel's end implies the end of all before it.  Before
-// the wait only what the chain never writes is read: the active list, the
-// descriptors, the twiddle tables.  State pointers are not __restrict__ (an
-// invariant load could move above the wait).
+// each lets its successor start at once (mm_chain_start; from 2^14 on at its
+// end, see MmTasks::run) and waits for its predecessor (mm_chain_wait) before
+// it touches what the chain writes; every thread waits, so a kernel's end
+// implies the end of all before it.  Before the wait only what the chain never
+// writes is read: the active list, the descriptors, the twiddle tables.  State
+// pointers are not __restrict__ (an invariant load could move above the wait).
 //
 // What bounds a round of one slot is the chain itself: six to eight kernels
 // of 3..32 CTAs, each a launch, its descriptor and table loads, and one pass

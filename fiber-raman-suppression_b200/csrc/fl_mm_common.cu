@@ -210,9 +210,9 @@ cudaError_t contract_tc(const MmRound& a) {
 // round of 1.05 ms, 120 us of an adjoint one of 2.7 ms; the gradient 484 ->
 // 469 ms).  With fewer modes the forward contraction alone fits three to six
 // CTAs per SM, and in the chain of a small launch the empty kernel costs
-// nothing measurable (6 modes, one slot: 21.7 ms either way).
+// nothing measurable (6 modes, one slot).
 bool mm_one_contraction(const MmRound& a) {
-    return a.adjoint && a.tensor_cores && a.M >= 9 && mm_adj_mixed(a.M, a.N, a.fp64);
+    return a.adjoint && a.M >= 9 && mm_adj_mixed(a.M, a.N, a.fp64);
 }
 
 template <int M>
@@ -242,13 +242,15 @@ cudaError_t contract_m(const MmRound& a, int which) {
         if constexpr (M >= 9) {
             if (which == 0 && mm_one_contraction(a)) return contract_both_tc<M>(a);
         }
-        if (which == 0 && a.tensor_cores && a.N % kTcRows == 0) return contract_tc<M>(a);
+        if (which == 0 && a.N % kTcRows == 0) return contract_tc<M>(a);
     }
     // mixed-precision adjoint (mm_adj_mixed): the assembly's forward-field
     // contractions and the Im X contraction on the tensor cores (3xTF32)
     if constexpr (sizeof(R) == 8 && M >= 6) {
-        if (which == 2 && mm_one_contraction(a)) return cudaSuccess;
-        if (which == 2 && mm_adj_mixed(M, a.N, a.fp64)) return contract_adj_tc<M>(a);
+        if (which == 2 && mm_adj_mixed(M, a.N, a.fp64)) {
+            if constexpr (M >= 9) return cudaSuccess;  // in mm_one_contraction's kernel
+            else return contract_adj_tc<M>(a);
+        }
         if (which == 1 && mm_adj_mixed(M, a.N, a.fp64))
             return a.fullrank_some ? imx_tc<M>(a) : cudaSuccess;
     }

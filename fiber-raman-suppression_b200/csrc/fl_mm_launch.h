@@ -16,7 +16,6 @@ struct MmRound {
     int M, NP, N;          // modes, pairs, points (same for every slot of the batch)
     int fp64;              // forward precision of the batch
     int control;           // run the control kernel after the evaluation
-    int tensor_cores;      // FP32 forward contraction on tcgen05 when M >= 6
     // slots with and without a low-rank form (rank > 0) may be in the batch:
     // the Z kernel serves the first, the Im X kernel the second; a kind known
     // to be absent is not launched

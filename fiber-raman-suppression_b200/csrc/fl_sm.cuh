@@ -354,7 +354,7 @@ struct TmScratch {
     static constexpr int E = L::E;
     static constexpr int WPV = (int)(2 * sizeof(R) / 4);  // words per complex value
     // values per chunk: the loads of a chunk have to fit the registers
-    // (FP64 with 512 threads: half as many)
+    // (FP64 with fewer than 16 values per thread: half as many)
     static constexpr int VPC = E < 4 ? E : sizeof(R) == 8 && E < 16 ? 2 : 4;
     static constexpr int CH = E / VPC;                    // chunks per field
     static constexpr int W = VPC * WPV < 8 ? 8 : VPC * WPV;  // words per chunk
@@ -889,7 +889,8 @@ struct SmSolver {
     }
 
     // The same with the thread's values unrolled, in registers from the input
-    // to the stored derivative, for 16 warps per SM.  There the warps hide
+    // to the stored derivative, for CTAs of 8 warps and more (2^12 to 2^14 on
+    // one CTA, 2^13 on two).  There the warps hide
     // one another's latencies and instruction fetches, and the loads in
     // flight per thread decide: at Nt = 2^13 on one CTA the rolled loops
     // above took 27.6 ms per gradient, this form 22.5.
@@ -1263,7 +1264,7 @@ __device__ __forceinline__ int last_sub(const Desc& d, const State& st, int seg)
 
 // Dense interpolant of an accepted step into sg (5 fields): c0 = ũ_n,
 // c_p = Σ_i r_ip k_i (Tsit5's free 4th-order interpolant); all stage loads
-// of a chunk of points in flight together, as in stage_input.
+// of a chunk of points in flight together, as in SmSolver::input.
 template <typename RF, class Sol>
 __device__ __forceinline__ void store_interp(const Sol& S, const double* u, int kperm,
                                              cx<RF>* sg) {
@@ -1480,7 +1481,7 @@ __global__ void __launch_bounds__(XShape<LOGN, CL>::TC, sm_min_ctas(LOGN, sizeof
                 int pk = -1;
                 if (peak) {
                     band = maxv(emax);
-                    // lowest index as the largest key N - b (block_max folds from 0)
+                    // lowest index as the largest key N - b (the maximum folds from 0)
                     double key = 0.0;
 #pragma unroll 4
                     for (int s = 0; s < E; s++) {
